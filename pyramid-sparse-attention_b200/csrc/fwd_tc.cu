@@ -37,15 +37,17 @@
 // TMEM (512 columns), head_dim 128: S0/P0 [0,128), S1/P1 [128,256), O of even tiles [256,384), O of odd tiles [384,512);
 // head_dim 64: three score buffers [0,384), O of even tiles [384,448), O of odd tiles [448,512).
 //
-// bf16 without the causal rule runs the FIXED-REFERENCE variant of the same kernel: the exponent that the probabilities of
-// a query row are taken relative to is the maximum of the row's FIRST tile (the group that owns that tile leaves it in
-// shared memory for the other one) and is never raised.  A bf16 probability has the exponent range of fp32, so later scores
-// may exceed the reference by dozens of octaves without losing a bit; the sum stays in fp32.  That removes the maximum
-// pass from every tile but the first and the rescaling of the accumulator, so both groups add into ONE accumulator
-// ([384, 384 + head_dim)), a third score buffer fits at head_dim 128 as well, and the row's end needs only the two sums.
-// A row whose sum of probabilities exceeds 2^90 (or is NaN) sets a guard word; the exact kernel is launched right behind
-// on the same stream and returns at once unless that word is set, in which case it redoes the call.  fp16 probabilities
-// (range 2^-24 .. 2^15) and the causal variants always take the exact kernel.
+// Every call runs the FIXED-REFERENCE variant of the same kernel first: the exponent that the probabilities of a query row
+// are taken relative to is the maximum of the row's FIRST tile (the group that owns that tile leaves it in shared memory
+// for the other one) and is never raised.  A bf16 probability has the exponent range of fp32, so later scores may exceed the
+// reference by dozens of octaves without losing a bit; an fp16 one ends at 2^16, so there the first maximum is put at 2^-6
+// and later scores may exceed it by 21 octaves.  The sum stays in fp32.  That removes the maximum pass from every tile but
+// the first and the rescaling of the accumulator, so both groups add into ONE accumulator ([384, 384 + head_dim)), a third
+// score buffer fits at head_dim 128 as well, and the row's end needs only the two sums.  With the causal rule a row sees a
+// key of its first tile or none at all: only the diagonal block hides keys; at level 1 it shows every row at least one, and
+// at the other levels it fills half a tile at most, with any other block of the row packed beside it.
+// A row whose sum of probabilities exceeds 2^90 (fp16: 2^15), or is NaN, sets a guard word; the exact kernel is launched
+// right behind on the same stream and returns at once unless that word is set, in which case it redoes the call.
 //
 // Every wait is bounded - mbarrier waits, the issuer's polling loop and the warp-group rendezvous (mbarriers, never
 // bar.sync, inside the role loops); on expiry the CTA records PSA_ERR_TIMEOUT in the status word, lets copies in
@@ -98,11 +100,9 @@ struct TcParams {
   const int* only_if;   // run only if this word is non-zero (the exact kernel as the fixed-reference variant's fallback)
 };
 
-// FIXED (bf16, head_dim 128, no causal rule): the reference exponent of a query row is the maximum of its FIRST tile and
-// is never raised - bf16 probabilities have the exponent range of fp32, so later scores may exceed it by dozens of
-// octaves without harm (a guard word reports rows that came near the range; the exact kernel then redoes the call).
-// No maximum pass after the first tile, no rescaling of the accumulator, hence ONE accumulator for both softmax groups
-// and room for a third score buffer.
+// FIXED: the reference exponent of a query row is the maximum of its FIRST tile and is never raised (see the head of the
+// file).  No maximum pass after the first tile, no rescaling of the accumulator, hence ONE accumulator for both softmax
+// groups and room for a third score buffer.
 template <int D, bool FIXED = false> struct Cfg {
   static constexpr int SLABS = D / 64;
   static constexpr int NK = D == 64 ? 4 : 3;   // K-tile ring
@@ -194,7 +194,6 @@ constexpr uint32_t kItemQuirk = 1u << 14, kItemPad = 1u << 15;
 template <int D, int FMT, bool IMG, bool CAUSAL, bool FIXED>
 __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_constant__ TmapPack maps, const TcParams p) {
   using C = Cfg<D, FIXED>;
-  static_assert(!FIXED || (FMT == 1 && !CAUSAL), "the fixed reference needs bf16 probabilities and a first tile that every row sees");
   if (p.only_if && *p.only_if == 0) return;
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
@@ -707,6 +706,10 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
     bool ok = true;
     int g0 = 0, q_rows = 0, pv_rows = 0;
     float* sMref = sXch + 1024;                   // fixed reference: [row & 3][128], behind the exchange area
+    // fp16 probabilities end at 2^16, and below 2^-14 they lose bits: the first tile's maximum is put at 2^-6, so later scores
+    // may lie 21 octaves above it, and a probability 2^-11 below the largest one is still off by 2^-8 of itself at most
+    constexpr float kRefLift = FMT == 1 ? 0.f : 6.f;
+    constexpr float kSumMax = FMT == 1 ? 1.2379400e27f : 32768.f;          // 2^90, 2^15
     for (int rit = 0; ok; ++rit) {
       const int rslot = rit & 3;
       ok = tc::mbar_wait(&ctl->row_ready[rslot], (rit >> 2) & 1, abort_flag);
@@ -826,7 +829,7 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
           if (FIXED) {
             if (j == 0) {
               // the group that owns the row's first tile sets the reference for both groups
-              m_run = mx == -INFINITY ? 0.f : mx;
+              m_run = mx == -INFINITY ? 0.f : mx + kRefLift;
               sMref[ref_slot * 128 + r] = m_run;
               __syncwarp();
               if (lane == 0) tc::mbar_arrive(&ctl->mref_full[ref_slot]);
@@ -970,11 +973,12 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
         const float w_me = FIXED ? 1.f : (m_run == -INFINITY ? 0.f : ex2(m_run - m_all));
         const float w_ot = FIXED ? 1.f : (m_o == -INFINITY ? 0.f : ex2(m_o - m_all));
         const float l_all = l_run * w_me + l_o * w_ot;
-        // legacy kernel: no visible key -> 0, lse -inf (fixed reference: every row sees its first tile, so "no key" = sum 0)
+        // legacy kernel: no visible key -> 0, lse -inf (fixed reference: a row that sees any key sees one of its first tile,
+        // so "no key" = sum 0)
         const bool dead = p.legacy && (FIXED ? l_all == 0.f : m_all == -INFINITY);
         const float inv = dead ? 0.f : 1.0f / l_all;              // otherwise an empty row is 0/0 like the reference
         const float w = w_me * inv, wo = w_ot * inv;
-        if (FIXED && p.guard && !(l_all < 1.2e27f) && qrow < p.seq_q) *p.guard = 1;   // 2^90: near the end of the exponent range (or NaN)
+        if (FIXED && p.guard && !(l_all < kSumMax) && qrow < p.seq_q) *p.guard = 1;   // near the end of the exponent range (or NaN)
         if (p.lse && g == 0 && qrow < p.seq_q)
           p.lse[(int64_t)bh * p.seq_q + qrow] = dead ? -INFINITY : (m_all + log2f(l_all)) * 0.6931471805599453f;
         const bool other_has = !FIXED && n_tiles - my_tiles > 0;
@@ -1175,16 +1179,16 @@ static int launch_tc(const FwdArgs& a, cudaStream_t st, int* guard = nullptr, co
   return PSA_OK;
 }
 
-// bf16 without the causal rule: the fixed-reference kernel, then the exact one, which returns at once unless the first one
-// raised its guard word (a row whose probabilities came near the end of the exponent range) - no host round trip.
-template <int D, bool IMG>
+// The fixed-reference kernel, then the exact one, which returns at once unless the first one raised its guard word (a row
+// whose probabilities came near the end of the exponent range) - no host round trip.
+template <int D, int FMT, bool IMG, bool CAUSAL>
 static int launch_fixed_then_exact(const FwdArgs& a, cudaStream_t st) {
   int* guard = nullptr;
   int rc = next_row_counter(&guard, st);      // a zeroed device word of this launch
   if (rc != PSA_OK) return rc;
-  rc = launch_tc<D, 1, IMG, false, true>(a, st, guard, nullptr);
+  rc = launch_tc<D, FMT, IMG, CAUSAL, true>(a, st, guard, nullptr);
   if (rc != PSA_OK) return rc;
-  return launch_tc<D, 1, IMG, false, false>(a, st, nullptr, guard);
+  return launch_tc<D, FMT, IMG, CAUSAL, false>(a, st, nullptr, guard);
 }
 
 int fwd_tc_launch(const FwdArgs& a, cudaStream_t st) {
@@ -1194,15 +1198,15 @@ int fwd_tc_launch(const FwdArgs& a, cudaStream_t st) {
     PSA_REQUIRE(a.bn >= 64, PSA_ERR_UNSUPPORTED, "tile images need block_n >= 64 (blocks of at least 8 pooled rows)");
     PSA_REQUIRE((((uintptr_t)a.kimg | (uintptr_t)a.vimg) & 15) == 0, PSA_ERR_ARG, "tile images must be 16-byte aligned");
     if (a.causal) {   // only the legacy forward asks for it; a variant of its own keeps the common kernel lean
-      if (a.D == 64) return fmt ? launch_tc<64, 1, true, true>(a, st) : launch_tc<64, 0, true, true>(a, st);
-      return fmt ? launch_tc<128, 1, true, true>(a, st) : launch_tc<128, 0, true, true>(a, st);
+      if (a.D == 64) return fmt ? launch_fixed_then_exact<64, 1, true, true>(a, st) : launch_fixed_then_exact<64, 0, true, true>(a, st);
+      return fmt ? launch_fixed_then_exact<128, 1, true, true>(a, st) : launch_fixed_then_exact<128, 0, true, true>(a, st);
     }
-    if (a.D == 64) return fmt ? launch_fixed_then_exact<64, true>(a, st) : launch_tc<64, 0, true>(a, st);
-    return fmt ? launch_fixed_then_exact<128, true>(a, st) : launch_tc<128, 0, true>(a, st);
+    if (a.D == 64) return fmt ? launch_fixed_then_exact<64, 1, true, false>(a, st) : launch_fixed_then_exact<64, 0, true, false>(a, st);
+    return fmt ? launch_fixed_then_exact<128, 1, true, false>(a, st) : launch_fixed_then_exact<128, 0, true, false>(a, st);
   }
   PSA_REQUIRE(!a.causal, PSA_ERR_UNSUPPORTED, "the causal rule needs the tile-image path");
-  if (a.D == 64) return fmt ? launch_fixed_then_exact<64, false>(a, st) : launch_tc<64, 0, false>(a, st);
-  return fmt ? launch_fixed_then_exact<128, false>(a, st) : launch_tc<128, 0, false>(a, st);
+  if (a.D == 64) return fmt ? launch_fixed_then_exact<64, 1, false, false>(a, st) : launch_fixed_then_exact<64, 0, false, false>(a, st);
+  return fmt ? launch_fixed_then_exact<128, 1, false, false>(a, st) : launch_fixed_then_exact<128, 0, false, false>(a, st);
 }
 
 }  // namespace psa

@@ -550,3 +550,32 @@ def test_scores_far_above_a_rows_first_tile(P, D, images, key_gain):
     assert float((got - ref).abs().max()) <= ATOL_OUT and cosine(got, ref) >= COS_OUT
     # head 0 is the value row of the one key, head 1 an ordinary average
     assert float((got[0, 0] - v[0, 0, 900].float()).abs().max()) <= ATOL_OUT
+
+
+@pytest.mark.parametrize("causal", [False, True], ids=["full", "causal"])
+@pytest.mark.parametrize("dt,octaves", [("bf16", 60), ("bf16", 200), ("fp16", 15), ("fp16", 40)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_legacy_rows_far_above_their_first_tile(P, D, dt, octaves, causal):
+    """The same for the old mask format (whose first tile is simply the first block), causal or not, and for fp16, whose
+    probabilities end 21 octaves above the first tile's maximum; the log-sum-exp rows are checked as well.  Query block 0
+    holds its diagonal at level 8 only: its first seven causal rows see no key at all."""
+    S, lead = 640, 350
+    g = torch.Generator().manual_seed(78)
+    q, k = 0.1 * torch.randn(1, 2, S, D, generator=g), 0.1 * torch.randn(1, 2, S, D, generator=g)
+    v = torch.randn(1, 2, S, D, generator=g)
+    q[..., 0] = 40.0
+    k[0, 0, lead, 0] = octaves * 0.6931 * D ** 0.5 / 40.0     # head 0: one key of block 2 far above everything else
+    q, k, v = (x.to(C.DT[dt]) for x in (q, k, v))
+    mask = torch.ones(1, 2, S // 128, S // 128, dtype=torch.int32)
+    mask[:, :, 0, 0] = 8
+    mask[:, 1, 3, 1:3] = 4
+    o, lse, _ = P.ops.legacy_forward(q.to(DEV), k.to(DEV), v.to(DEV), mask.to(DEV), causal, need_lse=True)
+    assert int(o._psa_status.item()) == 0
+    ref, ref_lse = O.legacy_forward(q, k, v, mask, causal)
+    o, lse, ref_lse = o.float().cpu(), lse.cpu(), ref_lse.float()
+    assert torch.isfinite(o).all()
+    assert float((o - ref.float()).abs().max()) <= ATOL_OUT and cosine(o, ref) >= COS_OUT
+    dead = (torch.arange(S) < (7 if causal else 0)).expand(1, 2, S)
+    assert torch.equal(torch.isinf(lse), dead) and float(o[dead].abs().sum()) == 0.0
+    # scores of one key are exact to an fp32 rounding of a sum of D products; the sum behind the logarithm to 2^-8
+    assert float((lse - ref_lse)[~dead].abs().max()) <= 2e-2
