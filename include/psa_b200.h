@@ -128,13 +128,13 @@ int psa_ksim(const void* k, int32_t* out, int64_t bh, int64_t seq, int head_dim,
  * and more than 256 launches of this family in flight at once on one device would share counters (a captured graph pins
  * its slot for every replay: do not replay such graphs while more than 255 other launches overlap them).  This holds
  * for every psa_fwd* / psa_legacy_fwd_images* entry point.
- * Every call is TWO launches of the tcgen05 kernel.  The first takes the probabilities of a query row
+ * A bf16 call is TWO launches of the tcgen05 kernel (an fp16 one is the second of them alone).  The first takes the probabilities of a query row
  * relative to the maximum of the row's first tile instead of a running maximum (same result: the factor cancels against
- * the row sum; bf16 probabilities and the fp32 sum have the exponent range for it, fp16 ones for scores up to 21 octaves
- * above that maximum), which saves the maximum pass and the rescaling; a row whose sum leaves the safe range sets a guard word (another slot of the counter ring).  The
+ * the row sum; bf16 probabilities and the fp32 sum have the exponent range for it), which saves the maximum pass and
+ * the rescaling; a row whose sum leaves the safe range sets a guard word (another slot of the counter ring).  The
  * second launch is the running-maximum kernel: it reads the guard word, returns at once if it is zero and recomputes
- * the call otherwise.  Both are ordered on `stream`; nothing is read back by the host.  A call therefore takes THREE words
- * of the ring (two row counters and the guard word): about 85 calls may be in flight on one device before words are
+ * the call otherwise.  Both are ordered on `stream`; nothing is read back by the host.  A bf16 call therefore takes THREE
+ * words of the ring (two row counters and the guard word): about 85 such calls may be in flight on one device before words are
  * shared. */
 int psa_fwd(const void* q, const void* k, const void* v, const void* k2, const void* k4, const void* k8,
             const void* v2, const void* v4, const void* v8, const int32_t* mask, void* out, int64_t bh,

@@ -37,17 +37,18 @@
 // TMEM (512 columns), head_dim 128: S0/P0 [0,128), S1/P1 [128,256), O of even tiles [256,384), O of odd tiles [384,512);
 // head_dim 64: three score buffers [0,384), O of even tiles [384,448), O of odd tiles [448,512).
 //
-// Every call runs the FIXED-REFERENCE variant of the same kernel first: the exponent that the probabilities of a query row
+// bf16 calls run the FIXED-REFERENCE variant of the same kernel first: the exponent that the probabilities of a query row
 // are taken relative to is the maximum of the row's FIRST tile (the group that owns that tile leaves it in shared memory
 // for the other one) and is never raised.  A bf16 probability has the exponent range of fp32, so later scores may exceed the
-// reference by dozens of octaves without losing a bit; an fp16 one ends at 2^16, so there the first maximum is put at 2^-6
-// and later scores may exceed it by 21 octaves.  The sum stays in fp32.  That removes the maximum pass from every tile but
+// reference by dozens of octaves without losing a bit.  (Not so fp16, which takes the exact kernel: a probability below 2^-14
+// is subnormal, and with one reference for both groups more of them are - error against 64 bits up to 4 % larger.)  The sum
+// stays in fp32.  That removes the maximum pass from every tile but
 // the first and the rescaling of the accumulator, so both groups add into ONE accumulator ([384, 384 + head_dim)), a third
 // score buffer fits at head_dim 128 as well, and the row's end needs only the two sums.  With the causal rule a row sees a
 // key of its first tile or none at all: only the diagonal block hides keys; at level 1 it shows every row at least one, and
 // at the other levels it fills half a tile at most, with any other block of the row packed beside it.
-// A row whose sum of probabilities exceeds 2^90 (fp16: 2^15), or is NaN, sets a guard word; the exact kernel is launched
-// right behind on the same stream and returns at once unless that word is set, in which case it redoes the call.
+// A row whose sum of probabilities exceeds 2^90, or is NaN, sets a guard word; the exact kernel is launched right behind on the
+// same stream and returns at once unless that word is set, in which case it redoes the call.
 //
 // Every wait is bounded - mbarrier waits, the issuer's polling loop and the warp-group rendezvous (mbarriers, never
 // bar.sync, inside the role loops); on expiry the CTA records PSA_ERR_TIMEOUT in the status word, lets copies in
@@ -706,10 +707,7 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
     bool ok = true;
     int g0 = 0, q_rows = 0, pv_rows = 0;
     float* sMref = sXch + 1024;                   // fixed reference: [row & 3][128], behind the exchange area
-    // fp16 probabilities end at 2^16, and below 2^-14 they lose bits: the first tile's maximum is put at 2^-6, so later scores
-    // may lie 21 octaves above it, and a probability 2^-11 below the largest one is still off by 2^-8 of itself at most
-    constexpr float kRefLift = FMT == 1 ? 0.f : 6.f;
-    constexpr float kSumMax = FMT == 1 ? 1.2379400e27f : 32768.f;          // 2^90, 2^15
+    constexpr float kSumMax = 1.2379400e27f;      // 2^90
     for (int rit = 0; ok; ++rit) {
       const int rslot = rit & 3;
       ok = tc::mbar_wait(&ctl->row_ready[rslot], (rit >> 2) & 1, abort_flag);
@@ -829,7 +827,7 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
           if (FIXED) {
             if (j == 0) {
               // the group that owns the row's first tile sets the reference for both groups
-              m_run = mx == -INFINITY ? 0.f : mx + kRefLift;
+              m_run = mx == -INFINITY ? 0.f : mx;
               sMref[ref_slot * 128 + r] = m_run;
               __syncwarp();
               if (lane == 0) tc::mbar_arrive(&ctl->mref_full[ref_slot]);
@@ -1183,6 +1181,7 @@ static int launch_tc(const FwdArgs& a, cudaStream_t st, int* guard = nullptr, co
 // whose probabilities came near the end of the exponent range) - no host round trip.
 template <int D, int FMT, bool IMG, bool CAUSAL>
 static int launch_fixed_then_exact(const FwdArgs& a, cudaStream_t st) {
+  static_assert(FMT == 1, "bf16 only");
   int* guard = nullptr;
   int rc = next_row_counter(&guard, st);      // a zeroed device word of this launch
   if (rc != PSA_OK) return rc;
@@ -1198,15 +1197,15 @@ int fwd_tc_launch(const FwdArgs& a, cudaStream_t st) {
     PSA_REQUIRE(a.bn >= 64, PSA_ERR_UNSUPPORTED, "tile images need block_n >= 64 (blocks of at least 8 pooled rows)");
     PSA_REQUIRE((((uintptr_t)a.kimg | (uintptr_t)a.vimg) & 15) == 0, PSA_ERR_ARG, "tile images must be 16-byte aligned");
     if (a.causal) {   // only the legacy forward asks for it; a variant of its own keeps the common kernel lean
-      if (a.D == 64) return fmt ? launch_fixed_then_exact<64, 1, true, true>(a, st) : launch_fixed_then_exact<64, 0, true, true>(a, st);
-      return fmt ? launch_fixed_then_exact<128, 1, true, true>(a, st) : launch_fixed_then_exact<128, 0, true, true>(a, st);
+      if (a.D == 64) return fmt ? launch_fixed_then_exact<64, 1, true, true>(a, st) : launch_tc<64, 0, true, true>(a, st);
+      return fmt ? launch_fixed_then_exact<128, 1, true, true>(a, st) : launch_tc<128, 0, true, true>(a, st);
     }
-    if (a.D == 64) return fmt ? launch_fixed_then_exact<64, 1, true, false>(a, st) : launch_fixed_then_exact<64, 0, true, false>(a, st);
-    return fmt ? launch_fixed_then_exact<128, 1, true, false>(a, st) : launch_fixed_then_exact<128, 0, true, false>(a, st);
+    if (a.D == 64) return fmt ? launch_fixed_then_exact<64, 1, true, false>(a, st) : launch_tc<64, 0, true, false>(a, st);
+    return fmt ? launch_fixed_then_exact<128, 1, true, false>(a, st) : launch_tc<128, 0, true, false>(a, st);
   }
   PSA_REQUIRE(!a.causal, PSA_ERR_UNSUPPORTED, "the causal rule needs the tile-image path");
-  if (a.D == 64) return fmt ? launch_fixed_then_exact<64, 1, false, false>(a, st) : launch_fixed_then_exact<64, 0, false, false>(a, st);
-  return fmt ? launch_fixed_then_exact<128, 1, false, false>(a, st) : launch_fixed_then_exact<128, 0, false, false>(a, st);
+  if (a.D == 64) return fmt ? launch_fixed_then_exact<64, 1, false, false>(a, st) : launch_tc<64, 0, false, false>(a, st);
+  return fmt ? launch_fixed_then_exact<128, 1, false, false>(a, st) : launch_tc<128, 0, false, false>(a, st);
 }
 
 }  // namespace psa

@@ -556,8 +556,8 @@ def test_scores_far_above_a_rows_first_tile(P, D, images, key_gain):
 @pytest.mark.parametrize("dt,octaves", [("bf16", 60), ("bf16", 200), ("fp16", 15), ("fp16", 40)])
 @pytest.mark.parametrize("D", [64, 128])
 def test_legacy_rows_far_above_their_first_tile(P, D, dt, octaves, causal):
-    """The same for the old mask format (whose first tile is simply the first block), causal or not, and for fp16, whose
-    probabilities end 21 octaves above the first tile's maximum; the log-sum-exp rows are checked as well.  Query block 0
+    """The same for the old mask format (whose first tile is simply the first block), causal or not, and for fp16 (whose
+    probabilities end 16 octaves above a reference); the log-sum-exp rows are checked as well.  Query block 0
     holds its diagonal at level 8 only: its first seven causal rows see no key at all."""
     S, lead = 640, 350
     g = torch.Generator().manual_seed(78)
