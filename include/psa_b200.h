@@ -237,6 +237,16 @@ int psa_block_scores_perm_rope(const void* q, const void* k, const int32_t* perm
                                size_t scratch_bytes, int64_t bh, int64_t seq, int head_dim, int block_m, int block_n, int dtype,
                                void* stream);
 
+/* Up to three (n) strided 16-bit operands of one shape [batch][heads][seq][head_dim], head_dim contiguous, copied to
+ * contiguous head-major tensors in ONE launch:
+ *   dst[i][b][h][t][:] = row perm[t] (t if perm is NULL) of head h of src[i], rotated first where rotate[i] != 0.
+ * strides: {batch, head, token} of each operand in elements, multiples of 8.  The rotation is the one of the entry points
+ * above (modify_diffusers.py:260-281, :363-369), the order that of rearranger.py:69-132; the copies are what the attention
+ * calls without row tables or rotating loads read (old mask format, block_n 32, no reordering).  Not in place. */
+int psa_gather_views(const void* const* src, const int64_t* strides, const int32_t* rotate, void* const* dst, int n,
+                     const int32_t* perm, const float* rope_a, const float* rope_b, int64_t rope_first, int64_t batch, int heads,
+                     int64_t seq, int head_dim, int dtype, void* stream);
+
 /* Antidiagonal block-importance estimate of the causal (vision-language) call site.  Replaces estimate_block_importance
  * with select_mode "inverse", softmax, kdb 1 - and its Triton kernels flat_group_gemm_fuse_reshape /
  * softmax_fuse_block_sum - qwen2.5-vl-example/src/attention/PSA_casual/utils/block_importance.py:282-562,

@@ -83,8 +83,103 @@ __global__ void __launch_bounds__(256) gather_heads_rope_kernel(const uint4* __r
   }
 }
 
+// Up to three strided operands [batch][heads][seq][D] copied head-major and contiguous in one launch, each read through
+// the row table and, where asked, rotated on the way (RopeTables in fwd.h).
+struct ViewSet {
+  const uint4* src[3];
+  int64_t batch_stride[3], head_stride[3], token_stride[3];   // in 16-byte words
+  uint4* dst[3];
+  int rotate[3];
+};
+
+// HBM-bound: every row is read and written once.  A thread moves the same 16-byte word of kUnroll rows, with all loads
+// issued before the first store: the address of a row hangs on its table entry, so one row at a time leaves a warp with a
+// single load in flight behind another one.  Rows are 128 or 256 contiguous bytes, whatever the order of the tokens.
+// 12 heads x 32760 tokens x 128, q, k, v from token-major views, ordered, q and k rotated: 134 us (4.5 TB/s of rows; the
+// rotary tables come on top, from L2).  The framework's element-wise operations took 2.5 ms for the same copies.
+template <int CPR, bool ROPE>
+__global__ void __launch_bounds__(256) gather_views_kernel(const ViewSet v, const int32_t* __restrict__ perm, int64_t seq, int heads,
+                                                           int bh_count, const RopeTables rope) {
+  constexpr int kUnroll = 4, kRows = 256 / CPR;
+  const int z = blockIdx.z, c = threadIdx.x % CPR;
+  // blocks walk the heads fastest where the rows of a token lie together (token-major), so that one DRAM page and one row of
+  // the rotary tables serve all heads; head by head otherwise
+  const unsigned stretches = gridDim.x / (unsigned)bh_count;
+  const bool heads_fastest = v.head_stride[z] < v.token_stride[z];
+  const int bh = (int)(heads_fastest ? blockIdx.x % (unsigned)bh_count : blockIdx.x / stretches);
+  const int64_t stretch = heads_fastest ? blockIdx.x / (unsigned)bh_count : blockIdx.x % stretches;
+  const int64_t b = bh / heads, h = bh % heads;
+  const uint4* src = v.src[z] + b * v.batch_stride[z] + h * v.head_stride[z] + c;
+  uint4* dst = v.dst[z] + (int64_t)bh * seq * CPR + c;
+  const int64_t t0 = stretch * (kRows * kUnroll) + threadIdx.x / CPR;
+  int64_t row[kUnroll];
+  uint4 x[kUnroll];
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u) {
+    const int64_t t = t0 + u * kRows;
+    row[u] = t < seq ? (perm ? (int64_t)perm[t] : t) : -1;
+  }
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u)
+    if (row[u] >= 0) x[u] = __ldg(src + row[u] * v.token_stride[z]);
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u) {
+    if (row[u] < 0) continue;
+    if (ROPE && v.rotate[z] && row[u] >= rope.first) {
+      const int64_t off = ((row[u] - rope.first) * CPR + c) * 8;
+      x[u] = rotate_word(x[u], rope.a + off, rope.b + off, rope.bf16 != 0);
+    }
+    dst[(t0 + u * kRows) * CPR] = x[u];
+  }
+}
+
 }  // namespace
 }  // namespace psa
+
+extern "C" int psa_gather_views(const void* const* src, const int64_t* strides, const int32_t* rotate, void* const* dst, int n,
+                                const int32_t* perm, const float* rope_a, const float* rope_b, int64_t rope_first, int64_t batch,
+                                int heads, int64_t seq, int head_dim, int dtype, void* stream) {
+  using namespace psa;
+  PSA_REQUIRE(src && strides && rotate && dst && n >= 1 && n <= 3, PSA_ERR_ARG, "psa_gather_views: 1 to 3 operands");
+  PSA_REQUIRE(dtype == PSA_F16 || dtype == PSA_BF16, PSA_ERR_UNSUPPORTED, "psa_gather_views: f16/bf16 only");
+  PSA_REQUIRE(head_dim == 64 || head_dim == 128, PSA_ERR_ARG, "psa_gather_views: head_dim=%d unsupported (64/128)", head_dim);
+  PSA_REQUIRE(batch > 0 && heads > 0 && batch * heads < 65536 && seq > 0 && seq < ((int64_t)1 << 31), PSA_ERR_ARG,
+              "psa_gather_views: bad shape");
+  PSA_REQUIRE((rope_a != nullptr) == (rope_b != nullptr) && (!rope_a || (rope_first >= 0 && rope_first <= seq)), PSA_ERR_ARG,
+              "psa_gather_views: bad rotary tables");
+  PSA_REQUIRE((((uintptr_t)rope_a | (uintptr_t)rope_b) & 15) == 0, PSA_ERR_ARG, "psa_gather_views: tables must be 16-byte aligned");
+  ViewSet v = {};
+  for (int i = 0; i < n; ++i) {
+    PSA_REQUIRE(src[i] && dst[i] && src[i] != dst[i], PSA_ERR_ARG, "psa_gather_views: operand %d", i);
+    PSA_REQUIRE((((uintptr_t)src[i] | (uintptr_t)dst[i]) & 15) == 0, PSA_ERR_ARG, "psa_gather_views: operand %d is not 16-byte aligned", i);
+    PSA_REQUIRE(!rotate[i] || rope_a, PSA_ERR_ARG, "psa_gather_views: operand %d is to be rotated without tables", i);
+    for (int d = 0; d < 3; ++d)
+      PSA_REQUIRE(strides[3 * i + d] >= 0 && strides[3 * i + d] % 8 == 0, PSA_ERR_ARG,
+                  "psa_gather_views: strides of operand %d must be multiples of 8 elements", i);
+    v.src[i] = (const uint4*)src[i];
+    v.dst[i] = (uint4*)dst[i];
+    v.batch_stride[i] = strides[3 * i] / 8;
+    v.head_stride[i] = strides[3 * i + 1] / 8;
+    v.token_stride[i] = strides[3 * i + 2] / 8;
+    v.rotate[i] = rotate[i] != 0;
+  }
+  const RopeTables rope = {rope_a, rope_b, rope_first, dtype == PSA_BF16};
+  const int rows_per_block = 256 / (head_dim / 8) * 4;
+  const int64_t blocks = cdiv64(seq, rows_per_block) * batch * heads;
+  PSA_REQUIRE(blocks < ((int64_t)1 << 31), PSA_ERR_ARG, "psa_gather_views: too many rows");
+  const dim3 grid((unsigned)blocks, 1, (unsigned)n);
+  const int bh = (int)(batch * heads);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (head_dim == 64) {
+    if (rope_a) gather_views_kernel<8, true><<<grid, 256, 0, st>>>(v, perm, seq, heads, bh, rope);
+    else gather_views_kernel<8, false><<<grid, 256, 0, st>>>(v, perm, seq, heads, bh, rope);
+  } else {
+    if (rope_a) gather_views_kernel<16, true><<<grid, 256, 0, st>>>(v, perm, seq, heads, bh, rope);
+    else gather_views_kernel<16, false><<<grid, 256, 0, st>>>(v, perm, seq, heads, bh, rope);
+  }
+  PSA_CHECK_LAUNCH("psa_gather_views");
+  return PSA_OK;
+}
 
 extern "C" int psa_gather_rows(const void* src, const int32_t* perm, void* dst, int64_t bh, int64_t seq, int head_dim,
                                int elem_bytes, void* stream) {

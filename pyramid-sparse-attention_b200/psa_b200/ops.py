@@ -200,6 +200,39 @@ def rotate_rows(x: torch.Tensor, rope: RotaryTables) -> torch.Tensor:
     return torch.cat([head, out.to(x.dtype)], dim=2)
 
 
+def views_supported(q, k, v, rope: Optional[RotaryTables] = None) -> bool:
+    """Whether gather_views takes these operands: 16-bit CUDA tensors of one shape, no gradient wanted, tables that fit."""
+    if any(t.dim() != 4 or t.shape != q.shape or t.dtype != q.dtype or t.device != q.device for t in (k, v)):
+        return False
+    if not q.is_cuda or q.dtype not in (torch.float16, torch.bfloat16) or q.dim() != 4 or q.shape[-1] not in (64, 128):
+        return False
+    if q.numel() == 0 or q.shape[0] * q.shape[1] >= 65536 or (torch.is_grad_enabled() and any(t.requires_grad for t in (q, k, v))):
+        return False
+    return rope is None or (rope.a.device == rope.b.device == q.device and tuple(rope.a.shape) == (q.shape[2] - rope.first, q.shape[3])
+                            and 0 <= rope.first <= q.shape[2] and (rope.a.data_ptr() | rope.b.data_ptr()) % 16 == 0)
+
+
+def gather_views(q, k, v, perm: Optional[torch.Tensor] = None, rope: Optional[RotaryTables] = None):
+    """Contiguous copies of q, k, v [B, H, S, D] (any batch, head and token strides) in one launch: rows in the order of
+    perm (None: as stored), q and k rotated by rope (None: as they are)."""
+    _need_cuda(q, k, v)
+    B, H, S, D = q.shape
+    perm = None if perm is None else _perm32(perm, S)
+    if rope is not None and rope.first == S:
+        rope = None                               # no token is rotated; the tables have no rows
+    # rows the kernel cannot address word by word are laid out first
+    views = [x if x.stride(3) == 1 and all(s % 8 == 0 for s in x.stride()[:3]) and x.data_ptr() % 16 == 0
+             else x.clone(memory_format=torch.contiguous_format) for x in (q, k, v)]
+    with torch.cuda.device(q.device):
+        outs = [torch.empty((B, H, S, D), dtype=q.dtype, device=q.device) for _ in range(3)]
+        rc = lib.psa_gather_views((C.c_void_p * 3)(*[x.data_ptr() for x in views]),
+                                  (C.c_int64 * 9)(*[s for x in views for s in x.stride()[:3]]), (C.c_int32 * 3)(*([int(rope is not None)] * 2), 0),
+                                  (C.c_void_p * 3)(*[o.data_ptr() for o in outs]), 3, _ptr(perm), _ptr(rope and rope.a), _ptr(rope and rope.b),
+                                  rope.first if rope is not None else 0, B, H, S, D, _dt(q), _stream(q))
+    check(rc, "psa_gather_views")
+    return outs
+
+
 def gather_heads(x: torch.Tensor, perm: Optional[torch.Tensor] = None, rope: Optional[RotaryTables] = None) -> torch.Tensor:
     """[S, H, D] -> [1, H, S, D] with out[0, h, t] = x[perm[t], h] (perm None: a plain transpose copy), rotated on the
     way if rope is given."""
@@ -635,15 +668,22 @@ def legacy_forward_reordered(q, k, v, mask, perm: torch.Tensor, sm_scale: Option
     sm_scale = D ** -0.5 if sm_scale is None else sm_scale
     if not _legacy_tc_ok(q, sm_scale):
         raise ValueError("the reordered legacy forward needs f16/bf16 tensors, at most 1467 blocks of 128 tokens and a positive scale")
+    return legacy_forward_gathered(gather_rows(q, perm), pyramid_kv_images(k, v, 128, perm=perm), mask, perm, sm_scale)
+
+
+def legacy_forward_gathered(q_r, imgs: KVImages, mask, perm: torch.Tensor, sm_scale: Optional[float] = None) -> torch.Tensor:
+    """The second half of legacy_forward_reordered: q_r = q[..., perm, :], imgs the tile images of the reordered k, v."""
+    _need_cuda(q_r, mask, perm)
+    mask = _mask32(mask)
+    B, H, S, D = q_r.shape
+    sm_scale = D ** -0.5 if sm_scale is None else sm_scale
     perm = _perm32(perm, S)
-    imgs = pyramid_kv_images(k, v, 128, perm=perm)
-    q_r = gather_rows(q, perm)
-    with torch.cuda.device(q.device):
-        o = torch.empty_like(q)
-        scratch = torch.empty(lib.psa_legacy_index_bytes(B * H, S) // 4, dtype=torch.int32, device=q.device)
-        status = status_word(q.device)
+    with torch.cuda.device(q_r.device):
+        o = torch.empty_like(q_r)
+        scratch = torch.empty(lib.psa_legacy_index_bytes(B * H, S) // 4, dtype=torch.int32, device=q_r.device)
+        status = status_word(q_r.device)
         rc = lib.psa_legacy_fwd_images_perm(_ptr(q_r), _ptr(imgs.kimg), _ptr(imgs.vimg), _ptr(mask), _ptr(scratch), _ptr(o), _ptr(perm),
-                                            B * H, S, D, mask.shape[-1], float(sm_scale), _dt(q), _ptr(status), _stream(q))
+                                            B * H, S, D, mask.shape[-1], float(sm_scale), _dt(q_r), _ptr(status), _stream(q_r))
     check(rc, "psa_legacy_fwd_images_perm")
     o._psa_status = status
     return o

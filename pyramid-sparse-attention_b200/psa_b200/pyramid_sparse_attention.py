@@ -161,11 +161,24 @@ class PyramidSparseAttention(nn.Module):
 
     _v_requires_grad = False      # set per call by forward()
 
-    def _forward_old_format_in_place(self, q, k, v, compute_stats):
+    def _one_copy(self, q, k, v, rotary) -> bool:
+        """Whether rotation, order and layout of q, k, v can be one copy each (ops.gather_views)."""
+        g = self.gilbert_rearranger
+        return (ops.views_supported(q, k, v, rotary)
+                and (not self.use_rearrange or q.shape[2] == g.total_elements + g.text_length))
+
+    def _forward_old_format_in_place(self, q, k, v, compute_stats, rope=None):
         c = self.config
         perm = self.gilbert_rearranger.source_rows(q.device)
-        mask, _, _ = compute_block_mask(q, k, c, text_length=c.text_length, perm=perm)
-        out = ops.legacy_forward_reordered(q, k, v, mask, perm)
+        if ops.views_supported(q, k, v, rope) and (rope is not None or not all(x.is_contiguous() for x in (q, k, v))):
+            # rotation, order and the change from the caller's strides are one copy of each operand: the kernels behind it
+            # read contiguous rows.  (Head-major tensors that need no rotation are read through the row table instead.)
+            q, k, v = ops.gather_views(q, k, v, perm, rope)
+            mask, _, _ = compute_block_mask(q, k, c, text_length=c.text_length)
+            out = ops.legacy_forward_gathered(q, ops.pyramid_kv_images(k, v, 128), mask, perm)
+        else:
+            mask, _, _ = compute_block_mask(q, k, c, text_length=c.text_length, perm=perm)
+            out = ops.legacy_forward_reordered(q, k, v, mask, perm)
         dens = ops.density(mask, False) if compute_stats else None
         return out, dens
 
@@ -187,15 +200,16 @@ class PyramidSparseAttention(nn.Module):
         the kernels rotate the rows as they read them, on every other route they are rotated here first."""
         is_warmup = self.get_current_time() < self.config.warmup_steps
         if rotary is not None:
-            # the in-place routes (token-major views or head-major tensors) rotate inside their loads
-            if is_warmup or not self._rows_in_place(q, k):
+            # the in-place routes (token-major views or head-major tensors) rotate inside their loads, the others inside the
+            # copy that lays their operands out
+            if is_warmup or not (self._rows_in_place(q, k) or self._one_copy(q, k, v, rotary)):
                 q, k = ops.rotate_rows(q, rotary), ops.rotate_rows(k, rotary)
                 rotary = None
         compute_stats = self.config.verbose or self.logger is not None
         dens = None
         self._v_requires_grad = v.requires_grad
         if not is_warmup and self._rows_in_place_old_format(q, k):
-            out, dens = self._forward_old_format_in_place(q, k, v, compute_stats)
+            out, dens = self._forward_old_format_in_place(q, k, v, compute_stats, rope=rotary)
             self.sparsity_counter += 1
             if self.logger is not None:
                 self.logger.log_sparsity(layer_idx=layer_idx, density=dens, sequence_length=q.shape[2],
@@ -217,7 +231,11 @@ class PyramidSparseAttention(nn.Module):
                 self.logger.log_sparsity(layer_idx=layer_idx, density=dens, sequence_length=q.shape[2],
                                          batch_size=q.shape[0], num_heads=q.shape[1], is_warmup=False)
             return out
-        if self.use_rearrange:
+        if rotary is not None:
+            # routes without rotating loads (block_n 32, no reordering): rotation, order and layout in one copy each
+            perm = self.gilbert_rearranger.source_rows(q.device) if self.use_rearrange else None
+            q_r, k_r, v_r = ops.gather_views(q, k, v, perm, rotary)
+        elif self.use_rearrange:
             q_r, k_r, v_r = self.gilbert_rearranger.rearrange(q, k, v)
         else:
             q_r, k_r, v_r = q, k, v
