@@ -77,6 +77,8 @@ inline RowSource local_rows(const void* base) {
 __device__ __forceinline__ const uint4* row_word(const RowSource& s, int64_t bh, int64_t seq, int64_t tok, int row16, int c) {
   if (s.perm) tok = s.perm[tok];
   if (s.n_peers == 0) return reinterpret_cast<const uint4*>(s.base) + (bh * seq + tok) * row16 + c;
+  if (s.n_peers == 1)       // one token-major buffer: no owner to look for (a 64-bit division per row)
+    return reinterpret_cast<const uint4*>(s.peer[0]) + (tok * s.heads_total + s.head0 + bh) * row16 + c;
   const int64_t owner = tok / s.tokens_per_rank, local = tok - owner * s.tokens_per_rank;
   return reinterpret_cast<const uint4*>(s.peer[owner]) + (local * s.heads_total + s.head0 + bh) * row16 + c;
 }

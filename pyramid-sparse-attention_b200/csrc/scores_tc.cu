@@ -24,22 +24,46 @@ constexpr int kSlabBytes = 128 * 128;
 constexpr int kThreads = 192;
 constexpr int kStages = 2;
 
-template <typename T, bool ROPE>
-__global__ void __launch_bounds__(256) gather_samples_kernel(const RowSource x, const int32_t* __restrict__ idx,
-                                                             T* __restrict__ out, int64_t seq, int D, int block, int keep,
-                                                             int n_valid, int n_out, const RopeTables rope) {
-  const int cpr = D * (int)sizeof(T) / 16;
-  const int64_t bh = blockIdx.y;
-  uint4* dst = reinterpret_cast<uint4*>(out + bh * (int64_t)n_out * D);
-  const int64_t total = (int64_t)n_out * cpr;
-  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (int64_t)gridDim.x * blockDim.x) {
-    int i = (int)(w / cpr);
-    const int c = (int)(w % cpr);
-    const int ic = i < n_valid ? i : n_valid - 1;
-    int64_t tok = (int64_t)(ic / keep) * block + idx[bh * keep + (ic % keep)];
-    tok = tok < seq ? tok : seq - 1;
-    dst[(int64_t)i * cpr + c] = load_row_word<ROPE>(x, rope, bh, seq, tok, cpr, c);
+// One operand of the sample gather: rows of x picked by idx (keep per block of `block` tokens), n_out rows per head, those
+// past n_valid repeating the last one.
+struct SampleSet {
+  RowSource x;
+  const int32_t* idx;
+  uint4* out;
+  int64_t seq;
+  int block, keep, n_valid, n_out;
+};
+
+// Queries (blockIdx.z 0) and keys (1) in one launch.  HBM-bound: a quarter of the rows is read, and written once.  A thread
+// moves the same 16-byte word of four rows, all loads before the first store, with 32-bit row arithmetic.  Blocks walk the
+// heads fastest when the rows of a token lie together (token-major tensors): one DRAM page and one row of the rotary tables
+// then serve all heads.  40 heads x 75600 tokens x 128: 395 -> 113 us (6.9 TB/s) against one row per thread and 64-bit
+// divisions; 12 x 32760: 50 -> 14 us; 40 x 32760 rotated from token-major tensors: 187 -> 93 us.
+template <int CPR, bool ROPE>
+__global__ void __launch_bounds__(256) gather_samples_kernel(const SampleSet q, const SampleSet k, int bh_count, int heads_fastest,
+                                                             const RopeTables rope) {
+  constexpr int kUnroll = 4, kRows = 256 / CPR;
+  const SampleSet& s = blockIdx.z ? k : q;
+  const int n_blocks = (s.n_out + kRows * kUnroll - 1) / (kRows * kUnroll);
+  const int unit = (int)blockIdx.x;
+  if (unit >= n_blocks * bh_count) return;
+  const int bh = heads_fastest ? unit % bh_count : unit / n_blocks, blk = heads_fastest ? unit / bh_count : unit % n_blocks;
+  const int c = threadIdx.x % CPR, i0 = blk * (kRows * kUnroll) + (int)threadIdx.x / CPR;
+  const int32_t* idx = s.idx + (int64_t)bh * s.keep;
+  uint4* dst = s.out + ((int64_t)bh * s.n_out) * CPR + c;
+  int64_t tok[kUnroll];
+  uint4 w[kUnroll];
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u) {
+    const int i = min(i0 + u * kRows, s.n_valid - 1);
+    const int64_t t = (int64_t)(i / s.keep) * s.block + idx[i % s.keep];
+    tok[u] = t < s.seq ? t : s.seq - 1;
   }
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u) w[u] = load_row_word<ROPE>(s.x, rope, bh, s.seq, tok[u], CPR, c);
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u)
+    if (i0 + u * kRows < s.n_out) dst[(int64_t)(i0 + u * kRows) * CPR] = w[u];
 }
 
 struct Ctrl {
@@ -297,15 +321,19 @@ int launch_scores_cellmax_tc(const RowSource& q, const RowSource& k, const int32
   void* qs = extra;
   void* ks = (char*)extra + qb;
   {
-    const int cpr = d.D * 2 / 16;
-    dim3 gq((unsigned)std::min<int64_t>(cdiv64((int64_t)d.nq_s * cpr, 256), 148 * 8), (unsigned)bh);
-    dim3 gk((unsigned)std::min<int64_t>(cdiv64((int64_t)d.nk_cols * cpr, 256), 148 * 8), (unsigned)bh);
-    if (rope.a) {
-      gather_samples_kernel<uint16_t, true><<<gq, 256, 0, st>>>(q, idx_q, (uint16_t*)qs, d.seq_q, d.D, d.bm, d.kq, d.nq_s, d.nq_s, rope);
-      gather_samples_kernel<uint16_t, true><<<gk, 256, 0, st>>>(k, idx_k, (uint16_t*)ks, d.seq_k, d.D, d.bn, d.kk, d.nk_s, d.nk_cols, rope);
+    const SampleSet sq = {q, idx_q, (uint4*)qs, d.seq_q, d.bm, d.kq, d.nq_s, d.nq_s};
+    const SampleSet sk = {k, idx_k, (uint4*)ks, d.seq_k, d.bn, d.kk, d.nk_s, d.nk_cols};
+    const int rows_per_block = 256 / (d.D / 8) * 4;
+    const int64_t units = cdiv64(std::max(d.nq_s, d.nk_cols), rows_per_block) * bh;
+    PSA_REQUIRE(units < ((int64_t)1 << 31), PSA_ERR_ARG, "psa_block_scores: too many sampled rows");
+    const dim3 grid((unsigned)units, 1, 2);
+    const int heads_fastest = q.n_peers > 0;
+    if (d.D == 64) {
+      if (rope.a) gather_samples_kernel<8, true><<<grid, 256, 0, st>>>(sq, sk, (int)bh, heads_fastest, rope);
+      else gather_samples_kernel<8, false><<<grid, 256, 0, st>>>(sq, sk, (int)bh, heads_fastest, rope);
     } else {
-      gather_samples_kernel<uint16_t, false><<<gq, 256, 0, st>>>(q, idx_q, (uint16_t*)qs, d.seq_q, d.D, d.bm, d.kq, d.nq_s, d.nq_s, rope);
-      gather_samples_kernel<uint16_t, false><<<gk, 256, 0, st>>>(k, idx_k, (uint16_t*)ks, d.seq_k, d.D, d.bn, d.kk, d.nk_s, d.nk_cols, rope);
+      if (rope.a) gather_samples_kernel<16, true><<<grid, 256, 0, st>>>(sq, sk, (int)bh, heads_fastest, rope);
+      else gather_samples_kernel<16, false><<<grid, 256, 0, st>>>(sq, sk, (int)bh, heads_fastest, rope);
     }
     PSA_CHECK_LAUNCH("psa_block_scores(gather)");
   }
