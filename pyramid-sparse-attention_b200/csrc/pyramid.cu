@@ -122,25 +122,40 @@ __device__ __forceinline__ void img_store(unsigned char* base, int64_t bh, int64
   *reinterpret_cast<uint4*>(p) = val;
 }
 
-template <typename T, bool ROPE>
-__global__ void __launch_bounds__(256) pyramid_img_kernel(const RowSource k, const RowSource v, unsigned char* __restrict__ kimg,
-                                                          unsigned char* __restrict__ vimg, ImgLevels L, int64_t bh, int64_t S, int64_t n8,
-                                                          int cpr, const RopeTables rope) {
-  const RowSource& x = blockIdx.y ? v : k;
+struct KVSource { RowSource s[2]; };      // indexed in parameter space (a selected copy would live in local memory)
+
+// A block of 256 threads builds 256 / CPR token groups of one head at a time.  Units (head, stretch of groups) are walked
+// with the heads fastest when the rows of a token lie together (token-major tensors), so that one DRAM page and one row of the
+// rotary tables serve all heads while they are in L2; head by head otherwise.  40 heads x 32760 tokens x 128, token-major,
+// ordered and rotated: 945 -> 408 us against head by head with a 64-bit division per row and the operand's description
+// copied to local memory; 12 x 32760 head-major: 111 -> 87 us (6.6 TB/s).
+template <typename T, int CPR, bool ROPE>
+__global__ void __launch_bounds__(256) pyramid_img_kernel(const __grid_constant__ KVSource kv, unsigned char* __restrict__ kimg,
+                                                          unsigned char* __restrict__ vimg, ImgLevels L, int bh, int64_t S, int64_t n8,
+                                                          int heads_fastest, const RopeTables rope) {
+  constexpr int kGroups = 256 / CPR, slabs = CPR / 8;
+  const RowSource& x = kv.s[blockIdx.y];
   unsigned char* img = blockIdx.y ? vimg : kimg;
-  const int slabs = cpr / 8;
-  const int64_t total = bh * n8 * cpr;
-  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(w % cpr);
-    const int64_t g = w / cpr;
-    const int64_t head = g / n8;
-    const int64_t j = g % n8;
+  const int64_t stretches = (n8 + kGroups - 1) / kGroups, units = stretches * bh;
+  const int c = threadIdx.x % CPR;
+  for (int64_t unit = blockIdx.x; unit < units; unit += gridDim.x) {
+    int64_t head, stretch;
+    if (units < ((int64_t)1 << 31)) {      // 32-bit division
+      const unsigned u = (unsigned)unit, d = heads_fastest ? (unsigned)bh : (unsigned)stretches, hi = u / d, lo = u - hi * d;
+      head = heads_fastest ? lo : hi;
+      stretch = heads_fastest ? hi : lo;
+    } else {
+      head = heads_fastest ? unit % bh : unit / stretches;
+      stretch = heads_fastest ? unit / bh : unit % stretches;
+    }
+    const int64_t j = stretch * kGroups + threadIdx.x / CPR;
+    if (j >= n8) continue;
     uint4 r[8];
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
       int64_t tok = j * 8 + t;
       tok = tok < S ? tok : S - 1;
-      r[t] = (ROPE && blockIdx.y == 0) ? load_row_word<true>(x, rope, head, S, tok, cpr, c) : *row_word(x, head, S, tok, cpr, c);
+      r[t] = (ROPE && blockIdx.y == 0) ? load_row_word<true>(x, rope, head, S, tok, CPR, c) : *row_word(x, head, S, tok, CPR, c);
     }
     uint4 a[4], b[2], d;
 #pragma unroll
@@ -173,17 +188,22 @@ static int launch_pyramid_images(const RowSource& k, const RowSource& v, void* k
   const int64_t s_pad = cdiv64(seq, block_n) * block_n;
   const int64_t n8 = s_pad / 8;
   const int cpr = head_dim * 2 / 16;
-  int64_t blocks = cdiv64(bh * n8 * cpr, 256);
+  int64_t blocks = cdiv64(n8, 256 / cpr) * bh;
   const int64_t cap = max_blocks > 0 ? max_blocks : 148 * 16;
   if (blocks > cap) blocks = cap;
-  dim3 grid((unsigned)blocks, 2);
-  if (dtype == PSA_F16) {
-    if (rope.a) pyramid_img_kernel<__half, true><<<grid, 256, 0, st>>>(k, v, (unsigned char*)kimg, (unsigned char*)vimg, L, bh, seq, n8, cpr, rope);
-    else pyramid_img_kernel<__half, false><<<grid, 256, 0, st>>>(k, v, (unsigned char*)kimg, (unsigned char*)vimg, L, bh, seq, n8, cpr, rope);
-  } else {
-    if (rope.a) pyramid_img_kernel<__nv_bfloat16, true><<<grid, 256, 0, st>>>(k, v, (unsigned char*)kimg, (unsigned char*)vimg, L, bh, seq, n8, cpr, rope);
-    else pyramid_img_kernel<__nv_bfloat16, false><<<grid, 256, 0, st>>>(k, v, (unsigned char*)kimg, (unsigned char*)vimg, L, bh, seq, n8, cpr, rope);
-  }
+  const dim3 grid((unsigned)blocks, 2);
+  const int heads_fastest = k.n_peers > 0;
+  const KVSource kv = {{k, v}};
+#define PSA_IMG(TT, CPR, ROPE)                                                                                                      \
+  pyramid_img_kernel<TT, CPR, ROPE><<<grid, 256, 0, st>>>(kv, (unsigned char*)kimg, (unsigned char*)vimg, L, (int)bh, seq, n8, heads_fastest, rope)
+#define PSA_IMG_T(TT)                                                            \
+  do {                                                                           \
+    if (cpr == 8) { if (rope.a) PSA_IMG(TT, 8, true); else PSA_IMG(TT, 8, false); }   \
+    else { if (rope.a) PSA_IMG(TT, 16, true); else PSA_IMG(TT, 16, false); }         \
+  } while (0)
+  if (dtype == PSA_F16) PSA_IMG_T(__half); else PSA_IMG_T(__nv_bfloat16);
+#undef PSA_IMG_T
+#undef PSA_IMG
   PSA_CHECK_LAUNCH("psa_pyramid_kv_images");
   return PSA_OK;
 }
