@@ -10,6 +10,7 @@
 //
 // This file holds the scalar fp32 stage A (any dtype; exact fp32 dot products) and stage B.  The tcgen05
 // stage A for f16/bf16 lives in scores_tc.cu.
+#include <algorithm>
 #include <mutex>
 
 #include "psa_common.cuh"
@@ -106,8 +107,11 @@ template <typename T, int VEC>
 struct alignas(VEC * sizeof(T)) CellPack { T e[VEC]; };
 
 // VEC neighbouring cells per thread and load; the launcher picks the widest VEC (<= 8 bytes) that divides n_d.
+// HBM-bound (R is read once).  The block has as many threads as there are packs to load (up to 512, in equal shares beyond):
+// with 256 for every size, half of them idled at 32k tokens (128 packs) and a second pass ran at an eighth at 75k (296).  12 x 32760 tokens: 44 -> 28 us, 40 x 32760 (blocks of 128): 125 -> 48 us,
+// 40 x 75600: 600 -> 520 us.
 template <typename T, int VEC>
-__global__ void __launch_bounds__(256) scores_pool_normalise(const T* __restrict__ R, const float* __restrict__ rowmax,
+__global__ void __launch_bounds__(512) scores_pool_normalise(const T* __restrict__ R, const float* __restrict__ rowmax,
                                                             T* __restrict__ po, ScoreDims d) {
   extern __shared__ float sm_po[];
   __shared__ float red[8];
@@ -119,7 +123,6 @@ __global__ void __launch_bounds__(256) scores_pool_normalise(const T* __restrict
   // exp2 is monotone, so the pooled maximum of exp2(x - m_t) is exp2 of the maximum of (x - m_t): one exp2 per cell.
   // A thread owns VEC neighbouring cells and walks the block's sampled rows.
   using Pack = CellPack<T, VEC>;
-  float part = 0.f;
   for (int c = threadIdx.x * VEC; c < d.n_d; c += blockDim.x * VEC) {
     float best[VEC];
 #pragma unroll
@@ -144,20 +147,31 @@ __global__ void __launch_bounds__(256) scores_pool_normalise(const T* __restrict
       for (int v = 0; v < VEC; ++v) best[v] = fmaxf(best[v], Elem<T>::to_f(raw.e[v]) - m);
     }
 #pragma unroll
-    for (int v = 0; v < VEC; ++v) {
-      const float b = Elem<T>::round(exp2f(best[v]));
-      sm_po[c + v] = b;
-      part += b;
-    }
+    for (int v = 0; v < VEC; ++v) sm_po[c + v] = Elem<T>::round(exp2f(best[v]));
   }
-  for (int off = 16; off; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = part;
+  __syncthreads();
+  // The row sum is taken in one order whatever the block size: 256 strided partial sums, folded warp by warp.
+  for (int vt = threadIdx.x; vt < 256; vt += blockDim.x) {
+    float part = 0.f;
+    for (int c = vt * VEC; c < d.n_d; c += 256 * VEC)
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) part += sm_po[c + v];
+    for (int off = 16; off; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
+    if ((vt & 31) == 0) red[vt >> 5] = part;
+  }
   __syncthreads();
   float sum = 0.f;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) sum += red[w];
+  for (int w = 0; w < 8; ++w) sum += red[w];
   sum = Elem<T>::round(sum);
   T* dst = po + ((int64_t)bh * d.Mq + r) * d.Nk;
   for (int c = threadIdx.x; c < d.Nk; c += blockDim.x) dst[c] = Elem<T>::from_f(sm_po[c] / sum);
+}
+
+// Block size of the pooling kernel for a row of `packs` loads: whole warps, at least 64 threads (the row maxima are loaded
+// by one thread each), the row in equal passes of at most 512.
+static unsigned pool_threads(int packs) {
+  const int passes = (packs + 511) / 512, per_pass = (packs + passes - 1) / passes;
+  return (unsigned)std::max(64, (per_pass + 31) / 32 * 32);
 }
 
 template <typename T>
@@ -183,9 +197,9 @@ static int launch_scores(const RowSource& q, const RowSource& k, const int32_t* 
   dim3 gridb((unsigned)d.Mq, (unsigned)bh);
   // n_d is a multiple of 64 / (block_n / 4), i.e. of 2 at least; R itself is 256-byte aligned
   constexpr int kWide = 8 / (int)sizeof(T);
-  if (d.n_d % kWide == 0) scores_pool_normalise<T, kWide><<<gridb, 256, d.n_d * sizeof(float), st>>>(R, rowmax, (T*)po, d);
-  else if (d.n_d % 2 == 0) scores_pool_normalise<T, 2><<<gridb, 256, d.n_d * sizeof(float), st>>>(R, rowmax, (T*)po, d);
-  else scores_pool_normalise<T, 1><<<gridb, 256, d.n_d * sizeof(float), st>>>(R, rowmax, (T*)po, d);
+  if (d.n_d % kWide == 0) scores_pool_normalise<T, kWide><<<gridb, pool_threads(d.n_d / kWide), d.n_d * sizeof(float), st>>>(R, rowmax, (T*)po, d);
+  else if (d.n_d % 2 == 0) scores_pool_normalise<T, 2><<<gridb, pool_threads(d.n_d / 2), d.n_d * sizeof(float), st>>>(R, rowmax, (T*)po, d);
+  else scores_pool_normalise<T, 1><<<gridb, pool_threads(d.n_d), d.n_d * sizeof(float), st>>>(R, rowmax, (T*)po, d);
   PSA_CHECK_LAUNCH("psa_block_scores(stage B)");
   return PSA_OK;
 }
@@ -465,13 +479,13 @@ extern "C" int psa_block_scores_samples(const void* qs, const void* ks, void* po
   if (rc != PSA_OK) return rc;
   dim3 gridb((unsigned)d.Mq, (unsigned)bh);
   if (dtype == PSA_F16) {
-    if (d.n_d % 4 == 0) scores_pool_normalise<__half, 4><<<gridb, 256, d.n_d * sizeof(float), st>>>((const __half*)R, rowmax, (__half*)po, d);
-    else scores_pool_normalise<__half, 2><<<gridb, 256, d.n_d * sizeof(float), st>>>((const __half*)R, rowmax, (__half*)po, d);
+    if (d.n_d % 4 == 0) scores_pool_normalise<__half, 4><<<gridb, pool_threads(d.n_d / 4), d.n_d * sizeof(float), st>>>((const __half*)R, rowmax, (__half*)po, d);
+    else scores_pool_normalise<__half, 2><<<gridb, pool_threads(d.n_d / 2), d.n_d * sizeof(float), st>>>((const __half*)R, rowmax, (__half*)po, d);
   } else {
     if (d.n_d % 4 == 0)
-      scores_pool_normalise<__nv_bfloat16, 4><<<gridb, 256, d.n_d * sizeof(float), st>>>((const __nv_bfloat16*)R, rowmax, (__nv_bfloat16*)po, d);
+      scores_pool_normalise<__nv_bfloat16, 4><<<gridb, pool_threads(d.n_d / 4), d.n_d * sizeof(float), st>>>((const __nv_bfloat16*)R, rowmax, (__nv_bfloat16*)po, d);
     else
-      scores_pool_normalise<__nv_bfloat16, 2><<<gridb, 256, d.n_d * sizeof(float), st>>>((const __nv_bfloat16*)R, rowmax, (__nv_bfloat16*)po, d);
+      scores_pool_normalise<__nv_bfloat16, 2><<<gridb, pool_threads(d.n_d / 2), d.n_d * sizeof(float), st>>>((const __nv_bfloat16*)R, rowmax, (__nv_bfloat16*)po, d);
   }
   PSA_CHECK_LAUNCH("psa_block_scores_samples(stage B)");
   return PSA_OK;
