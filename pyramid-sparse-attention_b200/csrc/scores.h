@@ -33,4 +33,16 @@ int launch_scores_cellmax_tc(const RowSource& q, const RowSource& k, const int32
 int launch_scores_cellmax_tc_samples(const void* qs, const void* ks, void* R, float* rowmax, const ScoreDims& d, int64_t bh,
                                      int dtype, cudaStream_t st);
 
+// rowmax[0, n) = -inf, before row maxima meet through atomic_max_float
+int launch_fill_neg_inf(float* x, int64_t n, cudaStream_t st);
+
+#ifdef __CUDACC__
+// max of floats through integer atomics; *addr must start at -inf
+__device__ __forceinline__ void atomic_max_float(float* addr, float v) {
+  v += 0.0f;   // -0 -> +0
+  if (v >= 0.f) atomicMax(reinterpret_cast<int*>(addr), __float_as_int(v));
+  else atomicMin(reinterpret_cast<unsigned int*>(addr), __float_as_uint(v));
+}
+#endif
+
 }  // namespace psa

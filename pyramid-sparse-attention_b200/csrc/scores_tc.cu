@@ -80,13 +80,6 @@ struct Params {
   float qk_scale;
 };
 
-// max of floats through integer atomics; *addr must start at -inf
-__device__ __forceinline__ void atomic_max_float(float* addr, float v) {
-  v += 0.0f;   // -0 -> +0
-  if (v >= 0.f) atomicMax(reinterpret_cast<int*>(addr), __float_as_int(v));
-  else atomicMin(reinterpret_cast<unsigned int*>(addr), __float_as_uint(v));
-}
-
 __global__ void fill_neg_inf(float* x, int64_t n) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) x[i] = -INFINITY;
 }
@@ -291,8 +284,8 @@ int launch_cellmax(const void* qs, const void* ks, void* R, float* rowmax, const
   }
   p.ksplit = ksplit;
   if (ksplit > 1) {
-    const int64_t n = bh * (int64_t)d.nq_s;
-    fill_neg_inf<<<(unsigned)std::min<int64_t>((n + 255) / 256, 1024), 256, 0, st>>>(rowmax, n);
+    rc = launch_fill_neg_inf(rowmax, bh * (int64_t)d.nq_s, st);
+    if (rc != PSA_OK) return rc;
   }
   dim3 grid((d.nq_s + 127) / 128, (unsigned)bh, (unsigned)ksplit);
   scores_cellmax_tc_kernel<D, FMT><<<grid, kThreads, smem, st>>>(tq, tk, p);
@@ -301,6 +294,12 @@ int launch_cellmax(const void* qs, const void* ks, void* R, float* rowmax, const
 }
 
 }  // namespace
+
+int launch_fill_neg_inf(float* x, int64_t n, cudaStream_t st) {
+  fill_neg_inf<<<(unsigned)std::min<int64_t>((n + 255) / 256, 1024), 256, 0, st>>>(x, n);
+  PSA_CHECK_LAUNCH("psa_block_scores(row maxima)");
+  return PSA_OK;
+}
 
 bool scores_tc_supported(const ScoreDims& d) {
   return (d.D == 64 || d.D == 128) && (d.kk == 8 || d.kk == 16 || d.kk == 32) && d.kq >= 1 && (d.n_d % 2 == 0);
