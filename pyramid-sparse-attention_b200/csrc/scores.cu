@@ -112,12 +112,14 @@ __global__ void __launch_bounds__(256) scores_cellmax_simt(const T* __restrict__
 template <typename T, int VEC>
 struct alignas(VEC * sizeof(T)) CellPack { T e[VEC]; };
 
-// VEC neighbouring cells per thread and load; the launcher picks the widest VEC (<= 8 bytes) that divides n_d.
+// VEC neighbouring cells per thread and load; the launcher picks the widest VEC (<= 16 bytes) that divides n_d.
 // HBM-bound (R is read once).  The block has as many threads as there are packs to load (up to 512, in equal shares beyond):
 // with 256 for every size, half of them idled at 32k tokens (128 packs) and a second pass ran at an eighth at 75k (296).  12 x 32760 tokens: 44 -> 28 us, 40 x 32760 (blocks of 128): 125 -> 48 us,
-// 40 x 75600: 600 -> 520 us.
-template <typename T, int VEC>
-__global__ void __launch_bounds__(512) scores_pool_normalise(const T* __restrict__ R, const float* __restrict__ rowmax,
+// 40 x 75600: 600 -> 316 us.  (512, 2): without the second bound the compiler keeps to 40 registers, too few for eight
+// 16-byte loads in flight, and the last figure is 520 us.
+// SUM: the cells one partial sum takes at a time (the widest VEC <= 8 bytes; the order of the row sum does not follow VEC).
+template <typename T, int VEC, int SUM = VEC>
+__global__ void __launch_bounds__(512, 2) scores_pool_normalise(const T* __restrict__ R, const float* __restrict__ rowmax,
                                                             T* __restrict__ po, ScoreDims d) {
   extern __shared__ float sm_po[];
   __shared__ float red[8];
@@ -159,9 +161,9 @@ __global__ void __launch_bounds__(512) scores_pool_normalise(const T* __restrict
   // The row sum is taken in one order whatever the block size: 256 strided partial sums, folded warp by warp.
   for (int vt = threadIdx.x; vt < 256; vt += blockDim.x) {
     float part = 0.f;
-    for (int c = vt * VEC; c < d.n_d; c += 256 * VEC)
+    for (int c = vt * SUM; c < d.n_d; c += 256 * SUM)
 #pragma unroll
-      for (int v = 0; v < VEC; ++v) part += sm_po[c + v];
+      for (int v = 0; v < SUM; ++v) part += sm_po[c + v];
     for (int off = 16; off; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
     if ((vt & 31) == 0) red[vt >> 5] = part;
   }
@@ -212,7 +214,8 @@ static int launch_scores(const RowSource& q, const RowSource& k, const int32_t* 
   dim3 gridb((unsigned)d.Mq, (unsigned)bh);
   // n_d is a multiple of 64 / (block_n / 4), i.e. of 2 at least; R itself is 256-byte aligned
   constexpr int kWide = 8 / (int)sizeof(T);
-  if (d.n_d % kWide == 0) scores_pool_normalise<T, kWide><<<gridb, pool_threads(d.n_d / kWide), d.n_d * sizeof(float), st>>>(R, rowmax, (T*)po, d);
+  if (d.n_d % (2 * kWide) == 0) scores_pool_normalise<T, 2 * kWide, kWide><<<gridb, pool_threads(d.n_d / (2 * kWide)), d.n_d * sizeof(float), st>>>(R, rowmax, (T*)po, d);
+  else if (d.n_d % kWide == 0) scores_pool_normalise<T, kWide><<<gridb, pool_threads(d.n_d / kWide), d.n_d * sizeof(float), st>>>(R, rowmax, (T*)po, d);
   else if (d.n_d % 2 == 0) scores_pool_normalise<T, 2><<<gridb, pool_threads(d.n_d / 2), d.n_d * sizeof(float), st>>>(R, rowmax, (T*)po, d);
   else scores_pool_normalise<T, 1><<<gridb, pool_threads(d.n_d), d.n_d * sizeof(float), st>>>(R, rowmax, (T*)po, d);
   PSA_CHECK_LAUNCH("psa_block_scores(stage B)");
@@ -494,10 +497,13 @@ extern "C" int psa_block_scores_samples(const void* qs, const void* ks, void* po
   if (rc != PSA_OK) return rc;
   dim3 gridb((unsigned)d.Mq, (unsigned)bh);
   if (dtype == PSA_F16) {
-    if (d.n_d % 4 == 0) scores_pool_normalise<__half, 4><<<gridb, pool_threads(d.n_d / 4), d.n_d * sizeof(float), st>>>((const __half*)R, rowmax, (__half*)po, d);
+    if (d.n_d % 8 == 0) scores_pool_normalise<__half, 8, 4><<<gridb, pool_threads(d.n_d / 8), d.n_d * sizeof(float), st>>>((const __half*)R, rowmax, (__half*)po, d);
+    else if (d.n_d % 4 == 0) scores_pool_normalise<__half, 4><<<gridb, pool_threads(d.n_d / 4), d.n_d * sizeof(float), st>>>((const __half*)R, rowmax, (__half*)po, d);
     else scores_pool_normalise<__half, 2><<<gridb, pool_threads(d.n_d / 2), d.n_d * sizeof(float), st>>>((const __half*)R, rowmax, (__half*)po, d);
   } else {
-    if (d.n_d % 4 == 0)
+    if (d.n_d % 8 == 0)
+      scores_pool_normalise<__nv_bfloat16, 8, 4><<<gridb, pool_threads(d.n_d / 8), d.n_d * sizeof(float), st>>>((const __nv_bfloat16*)R, rowmax, (__nv_bfloat16*)po, d);
+    else if (d.n_d % 4 == 0)
       scores_pool_normalise<__nv_bfloat16, 4><<<gridb, pool_threads(d.n_d / 4), d.n_d * sizeof(float), st>>>((const __nv_bfloat16*)R, rowmax, (__nv_bfloat16*)po, d);
     else
       scores_pool_normalise<__nv_bfloat16, 2><<<gridb, pool_threads(d.n_d / 2), d.n_d * sizeof(float), st>>>((const __nv_bfloat16*)R, rowmax, (__nv_bfloat16*)po, d);
