@@ -1,8 +1,8 @@
 // K-similarity cap: per key block, the mean cosine similarity of token pairs (2i,2i+1), (4i,4i+3) and
 // (8i,8i+7) decides the coarsest pyramid level the block may be pooled to.
 //
-// HBM-bound: K is read once (N*e bytes), one int32 per block is written.
-// One warp per key block; the warp walks the block 8 tokens at a time, lanes split the channels.
+// K is read once (N*e bytes), one int32 per block is written.  One warp per key block; the warp walks the block 8 tokens at
+// a time, lanes split the channels.  Bound by its instructions, not by HBM: 28 x 32768 x 128 takes 89 us (101 with one butterfly per sum).
 #include "psa_common.cuh"
 
 namespace psa {
@@ -16,45 +16,57 @@ __global__ void __launch_bounds__(128) ksim_kernel(const T* __restrict__ k, cons
   const int64_t bh = blockIdx.y;
   const T* kh = k + bh * seq * D;
   float c2 = 0.f, c4 = 0.f, c8 = 0.f;
+  // which two norms divide the product this lane ends up with (see below)
+  const int held = lane >> 1;
+  const int norm_a = held < 8 ? 0 : held < 12 ? 2 * (held - 8) : held == 13 ? 4 : 0;
+  const int norm_b = held < 8 ? 0 : held < 12 ? 2 * (held - 8) + 1 : held == 12 ? 3 : 7;
   for (int g0 = 0; g0 < bn; g0 += 8) {
-    float nn[8], d2[4], d4[2], d8;
+    // sums of this lane's channels: 8 squared norms, 4 + 2 + 1 products
+    float v[16];
 #pragma unroll
-    for (int t = 0; t < 8; ++t) nn[t] = 0.f;
+    for (int t = 0; t < 16; ++t) v[t] = 0.f;
+    const T* rows[8];
 #pragma unroll
-    for (int t = 0; t < 4; ++t) d2[t] = 0.f;
-    d4[0] = d4[1] = 0.f; d8 = 0.f;
+    for (int t = 0; t < 8; ++t) {
+      int64_t tok = (int64_t)blk * bn + g0 + t;
+      tok = tok < seq ? tok : seq - 1;
+      if (perm) tok = perm[tok];              // token `tok` of the reordered sequence is stored row perm[tok]
+      rows[t] = kh + tok * D;
+    }
+#pragma unroll 4
     for (int c = lane; c < D; c += 32) {
       float x[8];
 #pragma unroll
       for (int t = 0; t < 8; ++t) {
-        int64_t tok = (int64_t)blk * bn + g0 + t;
-        tok = tok < seq ? tok : seq - 1;
-        if (perm) tok = perm[tok];              // token `tok` of the reordered sequence is stored row perm[tok]
-        x[t] = Elem<T>::to_f(kh[tok * D + c]);
-        nn[t] = fmaf(x[t], x[t], nn[t]);
+        x[t] = Elem<T>::to_f(rows[t][c]);
+        v[t] = fmaf(x[t], x[t], v[t]);
       }
 #pragma unroll
-      for (int t = 0; t < 4; ++t) d2[t] = fmaf(x[2 * t], x[2 * t + 1], d2[t]);
-      d4[0] = fmaf(x[0], x[3], d4[0]);
-      d4[1] = fmaf(x[4], x[7], d4[1]);
-      d8 = fmaf(x[0], x[7], d8);
+      for (int t = 0; t < 4; ++t) v[8 + t] = fmaf(x[2 * t], x[2 * t + 1], v[8 + t]);
+      v[12] = fmaf(x[0], x[3], v[12]);
+      v[13] = fmaf(x[4], x[7], v[13]);
+      v[14] = fmaf(x[0], x[7], v[14]);
     }
+    // All 15 sums over the 32 lanes at once: at every step of the butterfly a lane passes on half of the values it holds and
+    // adds its partner's share to the other half, so lane 2i (and 2i+1) ends up with value i after 16 shuffles instead of 75.
+    // The additions are those of 15 butterflies.
 #pragma unroll
-    for (int off = 16; off; off >>= 1) {
+    for (int n = 8; n >= 1; n >>= 1) {
+      const bool upper = (lane & (2 * n)) != 0;
 #pragma unroll
-      for (int t = 0; t < 8; ++t) nn[t] += __shfl_xor_sync(0xffffffffu, nn[t], off);
-#pragma unroll
-      for (int t = 0; t < 4; ++t) d2[t] += __shfl_xor_sync(0xffffffffu, d2[t], off);
-      d4[0] += __shfl_xor_sync(0xffffffffu, d4[0], off);
-      d4[1] += __shfl_xor_sync(0xffffffffu, d4[1], off);
-      d8 += __shfl_xor_sync(0xffffffffu, d8, off);
+      for (int i = 0; i < n; ++i) {
+        const float send = upper ? v[i] : v[i + n], keep = upper ? v[i + n] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * n);
+      }
     }
+    const float sum = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+    const float norm = sqrtf(sum + 1e-12f);
+    const float na = __shfl_sync(0xffffffffu, norm, 2 * norm_a), nb = __shfl_sync(0xffffffffu, norm, 2 * norm_b);
+    const float cosine = sum / (na * nb + 1e-6f);          // lanes 16..29
 #pragma unroll
-    for (int t = 0; t < 8; ++t) nn[t] = sqrtf(nn[t] + 1e-12f);
-#pragma unroll
-    for (int t = 0; t < 4; ++t) c2 += d2[t] / (nn[2 * t] * nn[2 * t + 1] + 1e-6f);
-    c4 += d4[0] / (nn[0] * nn[3] + 1e-6f) + d4[1] / (nn[4] * nn[7] + 1e-6f);
-    c8 += d8 / (nn[0] * nn[7] + 1e-6f);
+    for (int t = 0; t < 4; ++t) c2 += __shfl_sync(0xffffffffu, cosine, 16 + 2 * t);
+    c4 += __shfl_sync(0xffffffffu, cosine, 24) + __shfl_sync(0xffffffffu, cosine, 26);
+    c8 += __shfl_sync(0xffffffffu, cosine, 28);
   }
   if (lane == 0) {
     const float s2 = c2 / (float)(bn / 2), s4 = c4 / (float)(bn / 4), s8 = c8 / (float)(bn / 8);
