@@ -141,6 +141,13 @@ int psa_fwd(const void* q, const void* k, const void* v, const void* k2, const v
             int64_t seq_q, int64_t seq_k, int head_dim, int block_m, int block_n, int tile_n, int mask_width,
             float sm_scale, int compat_quirk, int impl, int dtype, int32_t* status, void* stream);
 
+/* psa_fwd on the tcgen05 kernel whose output row t is stored at row out_perm[t] (int32 [seq_q], a permutation): the way back
+ * of a reordered call (rearranger.py:118-132) without a copy of the output. */
+int psa_fwd_perm(const void* q, const void* k, const void* v, const void* k2, const void* k4, const void* k8,
+                 const void* v2, const void* v4, const void* v8, const int32_t* mask, void* out, const int32_t* out_perm, int64_t bh,
+                 int64_t seq_q, int64_t seq_k, int head_dim, int block_m, int block_n, int tile_n, int mask_width,
+                 float sm_scale, int compat_quirk, int dtype, int32_t* status, void* stream);
+
 /* The same forward (tcgen05 kernel only) reading K/V from the tile images of psa_pyramid_kv_images: every selected
  * block is fetched with one linear bulk copy per operand instead of one tensor-map TMA operation per 64-channel
  * slab.  Replaces the same reference code as psa_fwd. */

@@ -26,10 +26,10 @@ extern "C" const char* psa_build_info(void) {
          "built " __DATE__ " " __TIME__;
 }
 
-extern "C" int psa_fwd(const void* q, const void* k, const void* v, const void* k2, const void* k4, const void* k8,
-                       const void* v2, const void* v4, const void* v8, const int32_t* mask, void* out, int64_t bh,
-                       int64_t seq_q, int64_t seq_k, int head_dim, int block_m, int block_n, int tile_n, int mask_width,
-                       float sm_scale, int compat_quirk, int impl, int dtype, int32_t* status, void* stream) {
+static int fwd_rows(const void* q, const void* k, const void* v, const void* k2, const void* k4, const void* k8, const void* v2,
+                    const void* v4, const void* v8, const int32_t* mask, void* out, const int32_t* out_perm, int64_t bh, int64_t seq_q,
+                    int64_t seq_k, int head_dim, int block_m, int block_n, int tile_n, int mask_width, float sm_scale, int compat_quirk,
+                    int impl, int dtype, int32_t* status, void* stream) {
   using namespace psa;
   PSA_REQUIRE(q && k && v && k2 && k4 && k8 && v2 && v4 && v8 && mask && out, PSA_ERR_ARG, "psa_fwd: null pointer");
   PSA_REQUIRE(head_dim == 64 || head_dim == 128, PSA_ERR_ARG, "psa_fwd: head_dim=%d (must be 64 or 128)", head_dim);
@@ -49,11 +49,30 @@ extern "C" int psa_fwd(const void* q, const void* k, const void* v, const void* 
   for (int i = 0; i < 4; ++i) { a.k[i] = kl[i]; a.v[i] = vl[i]; a.n[i] = nl[i]; }
   a.bh = bh; a.seq_q = seq_q; a.seq_k = seq_k; a.D = head_dim; a.bm = block_m; a.bn = block_n; a.tn = tile_n;
   a.width = mask_width; a.scale = sm_scale; a.quirk = compat_quirk; a.dtype = dtype;
+  a.scatter.row_perm = out_perm;
   const bool tc_ok = fwd_tc_supported(a);
   if (impl == 2) PSA_REQUIRE(tc_ok, PSA_ERR_UNSUPPORTED, "psa_fwd: the tcgen05 kernel needs f16/bf16, block_m=128");
   if (impl == 2 || (impl == 0 && tc_ok)) return fwd_tc_launch(a, st);
   return fwd_simt_dispatch(q, kl, vl, nl, mask, out, bh, seq_q, head_dim, block_m, block_n, tile_n, mask_width, sm_scale,
                            compat_quirk, dtype, st);
+}
+
+extern "C" int psa_fwd(const void* q, const void* k, const void* v, const void* k2, const void* k4, const void* k8,
+                       const void* v2, const void* v4, const void* v8, const int32_t* mask, void* out, int64_t bh,
+                       int64_t seq_q, int64_t seq_k, int head_dim, int block_m, int block_n, int tile_n, int mask_width,
+                       float sm_scale, int compat_quirk, int impl, int dtype, int32_t* status, void* stream) {
+  return fwd_rows(q, k, v, k2, k4, k8, v2, v4, v8, mask, out, nullptr, bh, seq_q, seq_k, head_dim, block_m, block_n, tile_n, mask_width,
+                  sm_scale, compat_quirk, impl, dtype, status, stream);
+}
+
+extern "C" int psa_fwd_perm(const void* q, const void* k, const void* v, const void* k2, const void* k4, const void* k8,
+                            const void* v2, const void* v4, const void* v8, const int32_t* mask, void* out, const int32_t* out_perm,
+                            int64_t bh, int64_t seq_q, int64_t seq_k, int head_dim, int block_m, int block_n, int tile_n,
+                            int mask_width, float sm_scale, int compat_quirk, int dtype, int32_t* status, void* stream) {
+  using namespace psa;
+  PSA_REQUIRE(out_perm && seq_q < ((int64_t)1 << 31), PSA_ERR_ARG, "psa_fwd_perm: row table");
+  return fwd_rows(q, k, v, k2, k4, k8, v2, v4, v8, mask, out, out_perm, bh, seq_q, seq_k, head_dim, block_m, block_n, tile_n, mask_width,
+                  sm_scale, compat_quirk, 2, dtype, status, stream);
 }
 
 extern "C" int psa_legacy_fwd(const void* q, const void* k, const void* v, const void* k2, const void* k4,

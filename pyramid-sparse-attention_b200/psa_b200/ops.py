@@ -594,6 +594,24 @@ def psa_forward(q, k, v, mask, block_m: int, block_n: int, tile_n: int, sm_scale
     return o
 
 
+def psa_forward_to_rows(q, k, v, mask, block_m: int, block_n: int, tile_n: int, out_perm) -> torch.Tensor:
+    """psa_forward on row-major pooled tensors (any block_n, tcgen05 kernel: 16-bit, contiguous operands) with output row t
+    stored at row out_perm[t] - the way back of a reordered call without a copy of its output."""
+    _need_cuda(q, k, v, mask)
+    B, H, S, D = q.shape
+    mask, out_perm = _mask32(mask), _perm32(out_perm, S)
+    (k2, k4, k8), (v2, v4, v8) = pyramid_kv(k, v, block_n)
+    with torch.cuda.device(q.device):
+        o = torch.empty_like(q)
+        status = status_word(q.device)
+        rc = lib.psa_fwd_perm(_ptr(q), _ptr(k), _ptr(v), _ptr(k2), _ptr(k4), _ptr(k8), _ptr(v2), _ptr(v4), _ptr(v8), _ptr(mask),
+                              _ptr(o), _ptr(out_perm), B * H, S, S, D, block_m, block_n, tile_n, mask.shape[-1], float(D ** -0.5),
+                              1, _dt(q), _ptr(status), _stream(q))
+    check(rc, "psa_fwd_perm")
+    o._psa_status = status
+    return o
+
+
 class LegacyKV:
     """Pooled K/V of the legacy kernels (block 128) in the two layouts their kernels read, each built on first use: tile
     images (tcgen05 forward and backward) and row-major levels 2/4/8 (scalar and warp-level-mma kernels)."""

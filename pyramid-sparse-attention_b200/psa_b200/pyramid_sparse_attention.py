@@ -210,10 +210,7 @@ class PyramidSparseAttention(nn.Module):
         self._v_requires_grad = v.requires_grad
         if not is_warmup and self._rows_in_place_old_format(q, k):
             out, dens = self._forward_old_format_in_place(q, k, v, compute_stats, rope=rotary)
-            self.sparsity_counter += 1
-            if self.logger is not None:
-                self.logger.log_sparsity(layer_idx=layer_idx, density=dens, sequence_length=q.shape[2],
-                                         batch_size=q.shape[0], num_heads=q.shape[1], is_warmup=False)
+            self._log_call(layer_idx, q, dens)
             return out
         if not is_warmup and self._rows_in_place(q, k):
             tm = [token_major_view(x) for x in (q, k, v)]
@@ -226,15 +223,21 @@ class PyramidSparseAttention(nn.Module):
                 dens = ops.density(mask, True) if compute_stats else None
             else:
                 out, dens = self._forward_rows_in_place(q, k, v, compute_stats, rope=rotary)
-            self.sparsity_counter += 1
-            if self.logger is not None:
-                self.logger.log_sparsity(layer_idx=layer_idx, density=dens, sequence_length=q.shape[2],
-                                         batch_size=q.shape[0], num_heads=q.shape[1], is_warmup=False)
+            self._log_call(layer_idx, q, dens)
             return out
         if rotary is not None:
             # routes without rotating loads (block_n 32, no reordering): rotation, order and layout in one copy each
             perm = self.gilbert_rearranger.source_rows(q.device) if self.use_rearrange else None
             q_r, k_r, v_r = ops.gather_views(q, k, v, perm, rotary)
+            c = self.config
+            if (perm is not None and c.attn_impl == "new_mask_type" and c.block_m == 128 and c.block_n == 32 and c.tile_n == 32
+                    and -(-k.shape[2] // c.block_n) + len(c.mask_ratios) <= 1472):
+                # ... and the way back is where the forward stores its rows
+                with torch.no_grad():
+                    mask, _, _ = compute_block_mask(q_r, k_r, c, text_length=c.text_length)
+                out = ops.psa_forward_to_rows(q_r, k_r, v_r, mask, c.block_m, c.block_n, c.tile_n, perm)
+                self._log_call(layer_idx, q, ops.density(mask, True) if compute_stats else None)
+                return out
         elif self.use_rearrange:
             q_r, k_r, v_r = self.gilbert_rearranger.rearrange(q, k, v)
         else:
@@ -244,11 +247,14 @@ class PyramidSparseAttention(nn.Module):
             out_r = torch.nn.functional.scaled_dot_product_attention(q_r, k_r, v_r)
         else:
             out_r, dens, _ = adaptive_block_sparse_attn(q_r, k_r, v_r, self.config, self.sparse_attention_fn, compute_stats)
+        self._log_call(layer_idx, q, dens, is_warmup)
+        return self.gilbert_rearranger.reversed_rearrange(out_r) if self.use_rearrange else out_r
+
+    def _log_call(self, layer_idx, q, dens, is_warmup=False):
         self.sparsity_counter += 1
         if self.logger is not None:
             self.logger.log_sparsity(layer_idx=layer_idx, density=dens, sequence_length=q.shape[2], batch_size=q.shape[0],
                                      num_heads=q.shape[1], is_warmup=is_warmup)
-        return self.gilbert_rearranger.reversed_rearrange(out_r) if self.use_rearrange else out_r
 
     def close_logger(self, jsonl_path: str = None):
         """Reference name (pyramid_sparse_attention.py:408-413).  With logging enabled the per-call records go to
