@@ -5,12 +5,15 @@
 // p_it = exp(q_i.k_t scale - lse_i):
 //   ds_it = round(p_it (dO_i.v_t - delta_i)) c_t(i),   pc_it = round(p_it) c_t(i)
 //   dQ_i = scale sum_t ds_it k_t,   dK_j (j in t) += scale / l sum_i ds_it q_i,   dV_j (j in t) += 1 / l sum_i pc_it dO_i
-// Two kernels share one skeleton: a STATIONARY pair of 128-row operand tiles in shared memory, a STREAM of 128-row
-// operand tiles through a two-stage ring, both products of a stream tile computed in 64-column halves into
-// double-buffered TMEM (S and dP), one thread per accumulator row turning them into the 16-bit operand of the
-// accumulating products IN PLACE in TMEM, and a single MMA-issuing thread that runs the fixed order
-//   acc(half 0, tile t)  S/dP(half 0, tile t+1)  acc(half 1, tile t)  S/dP(half 1, tile t+1) ...
-// so the element-wise work of one half always runs under the tensor work of the other.
+// Two kernels share one skeleton: a STATIONARY pair of 128-row operand tiles in shared memory, a STREAM of 128-row operand
+// tiles through two rings, S and dP of a stream tile as products of the two, one thread per accumulator row turning them
+// into the 16-bit operand of the accumulating products IN PLACE in TMEM, and a single MMA-issuing thread.
+// The element-wise warps work in two phases per tile: the probabilities as soon as S is there (kept in registers), dS once
+// dP is.  So half of their work runs under products: in the dK/dV kernel dV and the next S under phase 2, dK and the next dP
+// under phase 1; in the dQ kernel (S double-buffered) dQ and the next dP under phase 1 of the next tile.
+// Tensor / element-wise bound.  2 x 16 heads x 32768 tokens x 128, causal, random levels: dK/dV 14.3 -> 12.2 ms, dQ 7.3 -> 6.0 ms
+// against both products of a tile before its whole element-wise pass with two stages per ring; 28 heads x 5003 tokens:
+// 492 -> 440 and 334 -> 277 us.
 //
 //   bwd_dq_tc_kernel    stationary: Q and dO of one query block (rows = queries).  Stream: the selected key blocks of
 //                       all levels, PACKED back to back into 128-token K and V tiles (tile images, one linear bulk copy
@@ -35,7 +38,7 @@ namespace {
 constexpr int kSlab = 128 * 128;          // 128 rows x 128 B (64 16-bit channels)
 constexpr int kThreadsBwd = 576;          // warp 0 producer, warp 1 MMA issuer, warps 2-17 element-wise (four groups)
 constexpr int kEwWarps = 16;
-constexpr int kMaxBlocks = 1472;          // key / query blocks per head the lists are sized for
+constexpr int kMaxBlocks = 1472;          // key / query blocks per head that the entry points take
 
 __device__ __forceinline__ float ex2f(float x) {
   float y;
@@ -68,7 +71,8 @@ struct BwdParams {
   const unsigned char* kimg; // tile images (block 128) of K and V, all levels
   const unsigned char* vimg;
   ImgLevels img;
-  const float* stat;         // [bh][s_pad / 2][4]: (-lse0, -lse1, -delta0, -delta1) of two rows, lse in log2 units; rows >= seq: (-inf, 0)
+  const float* nlse;         // [bh][s_pad]: -lse in log2 units of every query row; rows >= seq: -inf
+  const float* ndelta;       // [bh][s_pad]: -delta; rows >= seq: 0
   void* dq;                  // [bh][seq][D]
   float* dkp[4];             // pooled fp32 sums per level: [bh][s_pad / l][D]
   float* dvp[4];
@@ -85,51 +89,60 @@ struct TmapQD {
   CUtensorMap q, d;          // {64 channels, 128 rows} boxes of Q and dO, [bh][seq][D]
 };
 
-template <int D> struct BCfg {
+// Shared memory of both kernels: two stationary tiles, a ring X for the stream operand that the first and the last product
+// of a tile read (Q in the dK/dV kernel, K in the dQ kernel) and a ring Y for the one that is done with earlier (dO, V).  A
+// copy takes some 2500 cycles from its issue to its last byte, so with two stages each the dQ kernel waited for K on every
+// tile; X has one stage more, and at head_dim 128 the seven tiles, the per-column words and the control block fill the 227 KB
+// to the last byte (the base needs no slack: it is declared 1024-byte aligned, and the kernels check it).
+template <int D> struct KCfg {
   static constexpr int SLABS = D / 64;
   static constexpr int TILE = SLABS * kSlab;
-  static constexpr int OFF_A0 = 0;                      // stationary tile 0 (K or Q)
-  static constexpr int OFF_A1 = TILE;                   // stationary tile 1 (V or dO)
-  static constexpr int OFF_B0 = 2 * TILE;               // stream ring, operand 0 (Q or K): 2 stages
-  static constexpr int OFF_B1 = 4 * TILE;               // stream ring, operand 1 (dO or V): 2 stages
-  static constexpr int OFF_META = 6 * TILE;             // per stage 128 x 16 B (dK/dV: 128 x float2 row statistics)
-  static constexpr int OFF_LC = OFF_META + 2 * 2048;    // dQ: per stage 128 floats, log2(copies) of every column (-inf: none)
-  static constexpr int OFF_LIST = OFF_LC + 2 * 512;     // work lists: 3 x kMaxBlocks words
-  static constexpr int OFF_CTRL = OFF_LIST + 3 * kMaxBlocks * 4;
-  static constexpr int SMEM = OFF_CTRL + 512 + 1024;    // control block + alignment slack
+  static constexpr int NX = D == 64 ? 4 : 3, NY = D == 64 ? 3 : 2;
+  static constexpr int OFF_A0 = 0, OFF_A1 = TILE;       // stationary: K, V (dK/dV) or Q, dO (dQ)
+  static constexpr int OFF_X = 2 * TILE, OFF_Y = OFF_X + NX * TILE;
+  static constexpr int OFF_YW = OFF_Y + NY * TILE;      // dK/dV: per Y stage 128 x -lse.  dQ: per X stage 8 x (first position, level)
+  static constexpr int OFF_XW = OFF_YW + NY * 512;      // per X stage 128 words: -delta of the queries (dK/dV), log2(copies) of the keys (dQ)
+  static constexpr int OFF_CTRL = OFF_XW + NX * 512;
+  static constexpr int SMEM = OFF_CTRL + 512;
+  static_assert(SMEM <= 232448, "more than 227 KB of shared memory");
+  static_assert(NX * 64 <= NY * 512, "dQ block words");
 };
 
-struct BCtrl {
+struct KCtrl {
   uint64_t a_full, a_free;               // stationary tiles loaded / all products that read them complete
-  uint64_t b_full[2], b0_free[2], b1_free[2];
-  uint64_t s_full, p_full;               // S and dP of a tile ready / their 16-bit operands written
+  uint64_t x_full[4], x_free[4], y_full[3], y_free[3];
+  uint64_t s_full[2], p_full;            // S of a tile ready (dQ: of even / odd tiles; dK/dV: [0] only) / P^T written over it (dK/dV)
+  uint64_t dp_full, ds_full;             // dP of a tile ready / dS written over it
   uint64_t acc_full, acc_free;
   uint64_t job_ready[3], job_done[3];
-  int job_id[3], job_n[3], job_last[3];  // id < 0: no more work; n = stream tiles; last = columns of the last tile (dQ) / head (dK/dV)
-  int tile_flag[2];                      // dQ: the stage's tile holds the block on the causal diagonal
+  int job_id[3], job_n[3], job_bh[3];    // id < 0: no more work; n == 0: nothing selected
+  uint32_t ent[4];                       // per X stage, the tile's entry; bit 31: last tile of the job
   uint32_t tmem_base;
   int abort_flag;
 };
+static_assert(sizeof(KCtrl) <= 512, "control block");
 
 // ------------------------------------------------------------------------------------------------------------------
 // dK / dV
 // ------------------------------------------------------------------------------------------------------------------
 template <int D, int FMT>
 __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dkdv_tc_kernel(const __grid_constant__ TmapQD maps, const BwdParams p) {
-  using C = BCfg<D>;
-  extern __shared__ unsigned char smem_dyn[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
-  BCtrl* ctl = reinterpret_cast<BCtrl*>(smem + C::OFF_CTRL);
-  uint32_t* lists = reinterpret_cast<uint32_t*>(smem + C::OFF_LIST);
+  using C = KCfg<D>;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  KCtrl* ctl = reinterpret_cast<KCtrl*>(smem + C::OFF_CTRL);
   volatile int* abort_flag = &ctl->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (tc::smem_u32(smem) & 1023) {          // the swizzled tiles need it; nothing has been started yet
+    if (threadIdx.x == 0 && p.status) atomicExch(p.status, PSA_ERR_TIMEOUT);
+    return;
+  }
 
   if (threadIdx.x == 0) {
     tc::mbar_init(&ctl->a_full, 1); tc::mbar_init(&ctl->a_free, 1);
-    for (int i = 0; i < 2; ++i) {
-      tc::mbar_init(&ctl->b_full[i], 1); tc::mbar_init(&ctl->b0_free[i], 1); tc::mbar_init(&ctl->b1_free[i], 1);
-    }
-    tc::mbar_init(&ctl->s_full, 1); tc::mbar_init(&ctl->p_full, kEwWarps);
+    for (int i = 0; i < C::NX; ++i) { tc::mbar_init(&ctl->x_full[i], 1); tc::mbar_init(&ctl->x_free[i], 1); }
+    for (int i = 0; i < C::NY; ++i) { tc::mbar_init(&ctl->y_full[i], 1); tc::mbar_init(&ctl->y_free[i], 1); }
+    tc::mbar_init(&ctl->s_full[0], 1); tc::mbar_init(&ctl->p_full, kEwWarps);
+    tc::mbar_init(&ctl->dp_full, 1); tc::mbar_init(&ctl->ds_full, kEwWarps);
     tc::mbar_init(&ctl->acc_full, 1); tc::mbar_init(&ctl->acc_free, kEwWarps);
     for (int i = 0; i < 3; ++i) { tc::mbar_init(&ctl->job_ready[i], 1); tc::mbar_init(&ctl->job_done[i], kEwWarps + 1); }
     ctl->abort_flag = 0;
@@ -170,26 +183,36 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dkdv_tc_kernel(const __gri
       const int li = e.x, g = e.y, l = 1 << li;
       const int n0 = g * l;                                // first key block of the group
       const int nsub = min(l, nk - n0);
-      uint32_t* list = lists + slot * kMaxBlocks;
-      // query blocks that selected level l for at least one of the group's key blocks, with the sub-block bits
-      int n_pairs = 0;
-      const int m_lo = p.causal ? n0 : 0;
+      // Query blocks that selected level l for at least one of the group's key blocks, with the sub-block bits: found
+      // while the job streams, 32 query blocks (one per lane) at a time and one pair ahead of the copies, so that a job
+      // needs no list and does not start with a scan of the whole mask column.
       const int32_t* mbase = p.mask + (bh * p.mq) * (int64_t)p.mask_cols + n0;
-      for (int m0 = m_lo; m0 < p.mq; m0 += 32) {
-        const int m = m0 + lane;
-        uint32_t bits = 0;
-        if (m < p.mq) {
-          const int32_t* row = mbase + (int64_t)m * p.mask_cols;
-          for (int i = 0; i < nsub; ++i)
-            if (row[i] == l && (!p.causal || n0 + i <= m)) bits |= 1u << i;
+      int m_next = p.causal ? n0 : 0, m_win = 0;
+      uint32_t my_bits = 0;
+      unsigned hits = 0;
+      auto next_pair = [&](uint32_t& pair) -> bool {
+        while (hits == 0 && m_next < p.mq) {
+          m_win = m_next;
+          const int m = m_win + lane;
+          my_bits = 0;
+          if (m < p.mq) {
+            const int32_t* row = mbase + (int64_t)m * p.mask_cols;
+            for (int i = 0; i < nsub; ++i)
+              if (row[i] == l && (!p.causal || n0 + i <= m)) my_bits |= 1u << i;
+          }
+          hits = __ballot_sync(0xffffffffu, my_bits != 0);
+          m_next += 32;
         }
-        const unsigned hit = __ballot_sync(0xffffffffu, bits != 0);
-        if (bits) list[n_pairs + __popc(hit & ((1u << lane) - 1))] = (uint32_t)m | bits << 16;
-        n_pairs += __popc(hit);
-      }
-      __syncwarp();
+        if (hits == 0) return false;
+        const int at = __ffs(hits) - 1;
+        hits &= hits - 1;
+        pair = (uint32_t)(m_win + at) | __shfl_sync(0xffffffffu, my_bits, at) << 16;
+        return true;
+      };
+      uint32_t pair = 0;
+      bool have = next_pair(pair);
       if (lane == 0) {
-        ctl->job_id[slot] = (int)job; ctl->job_n[slot] = n_pairs; ctl->job_last[slot] = (int)bh;
+        ctl->job_id[slot] = (int)job; ctl->job_n[slot] = have; ctl->job_bh[slot] = (int)bh;
         __threadfence_block();
         tc::mbar_arrive(&ctl->job_ready[slot]);
       }
@@ -198,7 +221,7 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dkdv_tc_kernel(const __gri
       if (lane == 0) next = atomicAdd(p.counter, 1);
       next = __shfl_sync(0xffffffffu, next, 0);
       job = (int64_t)gridDim.x + next;
-      if (n_pairs == 0) continue;
+      if (!have) continue;
       // stationary K and V rows [g*128, g*128+128) of level li (fewer at the end of the level)
       ok = tc::mbar_wait(&ctl->a_free, (ic & 1) ^ 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
@@ -213,24 +236,34 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dkdv_tc_kernel(const __gri
         tc::mbar_arrive_expect_tx(&ctl->a_full, 2 * bytes);
       }
       ++ic;
-      for (int pi = 0; pi < n_pairs && ok; ++pi, ++gp) {
-        const int st = gp & 1;
-        // a stage is free when both accumulating products of its previous tile have completed
-        ok = tc::mbar_wait(&ctl->b0_free[st], ((gp >> 1) & 1) ^ 1, abort_flag);
+      while (have) {
+        uint32_t cur = pair;
+        have = next_pair(pair);
+        if (!have) cur |= 1u << 31;
+        const int m = (int)(cur & 0xffffu), qs = gp % C::NX, ds = gp % C::NY;
+        // Q: free once dK of the stage's previous tile is complete; dO: once its dV is, half a tile earlier
+        ok = tc::mbar_wait(&ctl->x_free[qs], ((gp / C::NX) & 1) ^ 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         if (lane == 0) {
-          const int m = (int)(list[pi] & 0xffffu);
-          unsigned char* sq = smem + C::OFF_B0 + st * C::TILE;
-          unsigned char* sd = smem + C::OFF_B1 + st * C::TILE;
-          for (int s = 0; s < C::SLABS; ++s) {
-            tc::tma_load_3d(sq + s * kSlab, &maps.q, &ctl->b_full[st], s * 64, m * 128, (int)bh);
-            tc::tma_load_3d(sd + s * kSlab, &maps.d, &ctl->b_full[st], s * 64, m * 128, (int)bh);
-          }
-          tc::bulk_load_a(tc::smem_u32(smem + C::OFF_META + st * 2048), p.stat + (bh * p.s_pad + (int64_t)m * 128) * 2, 1024,
-                          tc::smem_u32(&ctl->b_full[st]));
-          tc::mbar_arrive_expect_tx(&ctl->b_full[st], 2 * C::TILE + 1024);
+          ctl->ent[qs] = cur;
+          for (int s = 0; s < C::SLABS; ++s)
+            tc::tma_load_3d(smem + C::OFF_X + qs * C::TILE + s * kSlab, &maps.q, &ctl->x_full[qs], s * 64, m * 128, (int)bh);
+          tc::bulk_load_a(tc::smem_u32(smem + C::OFF_XW + qs * 512), p.ndelta + bh * p.s_pad + (int64_t)m * 128, 512,
+                          tc::smem_u32(&ctl->x_full[qs]));
+          tc::mbar_arrive_expect_tx(&ctl->x_full[qs], C::TILE + 512);
         }
+        ok = tc::mbar_wait(&ctl->y_free[ds], ((gp / C::NY) & 1) ^ 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        if (lane == 0) {
+          for (int s = 0; s < C::SLABS; ++s)
+            tc::tma_load_3d(smem + C::OFF_Y + ds * C::TILE + s * kSlab, &maps.d, &ctl->y_full[ds], s * 64, m * 128, (int)bh);
+          tc::bulk_load_a(tc::smem_u32(smem + C::OFF_YW + ds * 512), p.nlse + bh * p.s_pad + (int64_t)m * 128, 512,
+                          tc::smem_u32(&ctl->y_full[ds]));
+          tc::mbar_arrive_expect_tx(&ctl->y_full[ds], C::TILE + 512);
+        }
+        ++gp;
       }
     }
   } else if (warp == 1) {
@@ -241,66 +274,72 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dkdv_tc_kernel(const __gri
       const uint32_t idesc_acc = tc::make_idesc(FMT, 128, D, 0, 1);
       const uint64_t kdesc = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_A0), 16, C::SLABS * 1024);
       const uint64_t vdesc = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_A1), 16, C::SLABS * 1024);
-      const uint64_t qk0 = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_B0), 16, 1024);      // stream tiles as K-major B
-      const uint64_t dk0 = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_B1), 16, 1024);
-      const uint64_t qm0 = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_B0), kSlab, 1024);   // ... and as MN-major B
-      const uint64_t dm0 = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_B1), kSlab, 1024);
+      const uint64_t qk0 = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_X), 16, 1024);       // stream tiles as K-major B
+      const uint64_t dk0 = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_Y), 16, 1024);
+      const uint64_t qm0 = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_X), kSlab, 1024);    // ... and as MN-major B
+      const uint64_t dm0 = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_Y), kSlab, 1024);
       const uint32_t ctl_a = tc::smem_u32(ctl);
-      const uint32_t s_full_a = ctl_a + (uint32_t)offsetof(BCtrl, s_full), p_full_a = ctl_a + (uint32_t)offsetof(BCtrl, p_full);
-      const uint32_t b_full_a = ctl_a + (uint32_t)offsetof(BCtrl, b_full);
+      const uint32_t s_full_a = ctl_a + (uint32_t)offsetof(KCtrl, s_full), p_full_a = ctl_a + (uint32_t)offsetof(KCtrl, p_full);
+      const uint32_t dp_full_a = ctl_a + (uint32_t)offsetof(KCtrl, dp_full), ds_full_a = ctl_a + (uint32_t)offsetof(KCtrl, ds_full);
+      const uint32_t q_full_a = ctl_a + (uint32_t)offsetof(KCtrl, x_full), d_full_a = ctl_a + (uint32_t)offsetof(KCtrl, y_full);
+      const volatile uint32_t* ent = ctl->ent;
       int gp = 0, ic = 0;
-      // S^T = K Q^T and dP^T = V dO^T of the tile in stage st (N = 128 query rows); one commit for both
-      auto issue_s = [&](int st) {
-        const uint64_t off = (uint64_t)((uint32_t)(st * C::TILE) >> 4);
-        const uint64_t qd = qk0 + off, dd = dk0 + off;
+      auto q_off = [&](int u) { return (uint64_t)((uint32_t)((u % C::NX) * C::TILE) >> 4); };
+      auto d_off = [&](int u) { return (uint64_t)((uint32_t)((u % C::NY) * C::TILE) >> 4); };
+      // a stationary tile (image layout) times a stream tile, N = 128 query rows
+      auto issue_ss = [&](uint32_t dst, uint64_t adesc, uint64_t bdesc, uint32_t done) {
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks)
-          tc::umma_ss(tmem + kST, kdesc + (uint64_t)(((ks >> 2) * 1024 + (ks & 3) * 32) >> 4),
-                      qd + (uint64_t)(((ks >> 2) * kSlab + (ks & 3) * 32) >> 4), idesc_s, ks > 0 ? 1u : 0u);
-#pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks)
-          tc::umma_ss(tmem + kDP, vdesc + (uint64_t)(((ks >> 2) * 1024 + (ks & 3) * 32) >> 4),
-                      dd + (uint64_t)(((ks >> 2) * kSlab + (ks & 3) * 32) >> 4), idesc_s, ks > 0 ? 1u : 0u);
-        tc::umma_commit_a(s_full_a);
+          tc::umma_ss(dst, adesc + (uint64_t)(((ks >> 2) * 1024 + (ks & 3) * 32) >> 4),
+                      bdesc + (uint64_t)(((ks >> 2) * kSlab + (ks & 3) * 32) >> 4), idesc_s, ks > 0 ? 1u : 0u);
+        tc::umma_commit_a(done);
       };
-      // dV += P^T dO and dK += dS^T Q.  k-step ks = query rows [16 ks, 16 ks + 16); its 16-bit operand sits at column
+      // an accumulating product.  k-step ks = query rows [16 ks, 16 ks + 16); its 16-bit operand sits at column
       // 32 (ks / 2) + 8 (ks % 2) of the buffer the fp32 values came from
-      auto issue_acc = [&](int st, bool first) {
-        const uint64_t off = (uint64_t)((uint32_t)(st * C::TILE) >> 4);
-        const uint64_t qd = qm0 + off, dd = dm0 + off;
-        tc::umma_ts(tmem + kAccV, tmem + kST, dd, idesc_acc, first ? 0u : 1u);
+      auto issue_acc = [&](uint32_t acc, uint32_t src, uint64_t bdesc, bool first) {
+        tc::umma_ts(acc, src, bdesc, idesc_acc, first ? 0u : 1u);
 #pragma unroll
         for (int ks = 1; ks < 8; ++ks)
-          tc::umma_ts(tmem + kAccV, tmem + kST + (ks >> 1) * 32 + (ks & 1) * 8, dd + (uint64_t)(ks * (2048 >> 4)), idesc_acc, 1u);
-        tc::umma_ts(tmem + kAccK, tmem + kDP, qd, idesc_acc, first ? 0u : 1u);
-#pragma unroll
-        for (int ks = 1; ks < 8; ++ks)
-          tc::umma_ts(tmem + kAccK, tmem + kDP + (ks >> 1) * 32 + (ks & 1) * 8, qd + (uint64_t)(ks * (2048 >> 4)), idesc_acc, 1u);
+          tc::umma_ts(acc, src + (ks >> 1) * 32 + (ks & 1) * 8, bdesc + (uint64_t)(ks * (2048 >> 4)), idesc_acc, 1u);
       };
       for (int it = 0; ok; ++it) {
         const int slot = it % 3;
         ok = tc::mbar_wait(&ctl->job_ready[slot], (it / 3) & 1, abort_flag);
         if (!ok || ctl->job_id[slot] < 0) break;
-        const int n = ctl->job_n[slot];
-        if (n == 0) { tc::mbar_arrive(&ctl->job_done[slot]); continue; }
+        if (ctl->job_n[slot] == 0) { tc::mbar_arrive(&ctl->job_done[slot]); continue; }
         ok = tc::mbar_wait(&ctl->a_full, ic & 1, abort_flag);
-        if (ok) ok = tc::mbar_wait_a(b_full_a + (gp & 1) * 8, (gp >> 1) & 1, abort_flag);
+        if (ok) ok = tc::mbar_wait_a(q_full_a + (gp % C::NX) * 8, (gp / C::NX) & 1, abort_flag);
         if (!ok) break;
         tc::tc_fence_after();
-        issue_s(gp & 1);
-        for (int pi = 0; pi < n && ok; ++pi, ++gp) {
-          const int st = gp & 1;
+        issue_ss(tmem + kST, kdesc, qk0 + q_off(gp), s_full_a);
+        ok = tc::mbar_wait_a(d_full_a + (gp % C::NY) * 8, (gp / C::NY) & 1, abort_flag);
+        if (!ok) break;
+        tc::tc_fence_after();
+        issue_ss(tmem + kDP, vdesc, dk0 + d_off(gp), dp_full_a);
+        // dV and S^T of the next tile run while the element-wise warps turn dP^T into dS^T, dK and dP^T of the next tile
+        // while they take the probabilities of the next tile
+        for (bool first = true; ok; first = false, ++gp) {
+          const bool last = (ent[gp % C::NX] >> 31) != 0;
           ok = tc::mbar_wait_a(p_full_a, gp & 1, abort_flag);
-          if (ok && pi == 0 && ic > 0) ok = tc::mbar_wait(&ctl->acc_free, (ic - 1) & 1, abort_flag);
+          if (ok && first && ic > 0) ok = tc::mbar_wait(&ctl->acc_free, (ic - 1) & 1, abort_flag);
           if (!ok) break;
           tc::tc_fence_after();
-          issue_acc(st, pi == 0);
-          if (pi + 1 < n) {
-            ok = tc::mbar_wait_a(b_full_a + (st ^ 1) * 8, ((gp + 1) >> 1) & 1, abort_flag);
+          issue_acc(tmem + kAccV, tmem + kST, dm0 + d_off(gp), first);
+          if (!last) {
+            ok = tc::mbar_wait_a(q_full_a + ((gp + 1) % C::NX) * 8, ((gp + 1) / C::NX) & 1, abort_flag);
             if (!ok) break;
             tc::tc_fence_after();
-            issue_s(st ^ 1);      // its commit also says that both accumulating products above are complete
+            issue_ss(tmem + kST, kdesc, qk0 + q_off(gp + 1), s_full_a);      // "S ready" also says: dV of this tile is complete
           }
+          ok = tc::mbar_wait_a(ds_full_a, gp & 1, abort_flag);
+          if (!ok) break;
+          tc::tc_fence_after();
+          issue_acc(tmem + kAccK, tmem + kDP, qm0 + q_off(gp), first);
+          if (last) { ++gp; break; }
+          ok = tc::mbar_wait_a(d_full_a + ((gp + 1) % C::NY) * 8, ((gp + 1) / C::NY) & 1, abort_flag);
+          if (!ok) break;
+          tc::tc_fence_after();
+          issue_ss(tmem + kDP, vdesc, dk0 + d_off(gp + 1), dp_full_a);       // "dP ready" also says: dK of this tile is complete
         }
         if (!ok) break;
         tc::umma_commit(&ctl->acc_full);
@@ -326,8 +365,7 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dkdv_tc_kernel(const __gri
       if (!ok) break;
       const int job = ctl->job_id[slot];
       if (job < 0) break;
-      const int n = ctl->job_n[slot];
-      const int64_t bh = ctl->job_last[slot];
+      const int64_t bh = ctl->job_bh[slot];
       const int2 e = p.items[job % p.n_entries];
       const int li = e.x, g = e.y, l = 1 << li;
       const int n0 = g * l;
@@ -336,96 +374,118 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dkdv_tc_kernel(const __gri
       const bool exists = t < n_l;
       const int sub = (r << li) >> 7;                        // key block of the group this row belongs to
       const int64_t j0 = t * l, l_k = li == 0 ? p.seq : p.s_pad;
-      const float c_static = (float)copies(j0, l, l_k, 0, 0);
-      const float log2c = (float)li;                          // c_static is l = 2^li wherever it is not 0 (level 1: 1)
+      const bool any_copy = copies(j0, l, l_k, 0, 0) > 0;    // l = 2^li copies wherever there are any (level 1: 1)
       // the sums of this row: groups 0, 1 store the two halves of the dK channels, groups 2, 3 those of dV
       constexpr int HD = D / 2;
       float* dst = (cg < 2 ? p.dkp[li] : p.dvp[li]) + (bh * n_l + t) * D + (cg & 1) * HD;
-      if (n == 0) {
+      if (ctl->job_n[slot] == 0) {
         if (exists)
           for (int c = 0; c < HD; c += 4) *reinterpret_cast<float4*>(dst + c) = make_float4(0.f, 0.f, 0.f, 0.f);
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&ctl->job_done[slot]);
         continue;
       }
-      const uint32_t* list = lists + slot * kMaxBlocks;
-      for (int pi = 0; pi < n && ok; ++pi, ++gp) {
-        const int st = gp & 1;
-        const uint32_t ent = list[pi];
-        const int m = (int)(ent & 0xffffu);
-        const bool act = exists && ((ent >> (16 + sub)) & 1u);
-        const bool diag = p.causal && act && (n0 + sub == m);
-        ok = tc::mbar_wait(&ctl->b_full[st], (gp >> 1) & 1, abort_flag);      // the row statistics of this tile
-        if (ok) ok = tc::mbar_wait(&ctl->s_full, gp & 1, abort_flag);
+      for (bool first = true; ok; first = false, ++gp) {
+        const int qs = gp % C::NX, ds = gp % C::NY;
+        // ---- phase 1: P^T over S^T.  The probabilities stay in registers for phase 2.
+        ok = tc::mbar_wait(&ctl->y_full[ds], (gp / C::NY) & 1, abort_flag);        // the tile's -lse
+        if (ok) ok = tc::mbar_wait(&ctl->x_full[qs], (gp / C::NX) & 1, abort_flag);  // ... -delta and entry
+        if (ok) ok = tc::mbar_wait(&ctl->s_full[0], gp & 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        // S^T and dP^T of this tile are complete, hence also both accumulating products of the previous tile: its stage
-        // may be refilled
-        if (relay && pi > 0) tc::mbar_arrive(&ctl->b0_free[st ^ 1]);
+        // S^T of this tile was issued behind dV of the previous one: its dO stage may be refilled
+        if (relay && !first) tc::mbar_arrive(&ctl->y_free[(gp - 1) % C::NY]);
         tc::tc_fence_after();
-        const float4* stat2 = reinterpret_cast<const float4*>(smem + C::OFF_META + st * 2048) + cg * 16;   // two columns each
-        const bool slow = __any_sync(0xffffffffu, diag);
+        const uint32_t ent = ctl->ent[qs];
+        const int m = (int)(ent & 0xffffu);
+        const bool act = exists && ((ent >> (16 + sub)) & 1u);
+        const bool slow = __any_sync(0xffffffffu, p.causal && act && (n0 + sub == m));
         const int64_t qbase = (int64_t)m * 128 + cg * 32;
-        // this thread's 32 columns in two chunks of 16 (one after the other: the element-wise warps are bound by their
-        // arithmetic, not by TMEM latency, and fewer live registers spare them spills).  The packed 16-bit results go back
-        // IN PLACE into columns this thread has read itself - chunk c into [8 c, 8 c + 8) of its group's columns - because
-        // the other groups work on the same buffers at the same time; the MMA takes every 16-element k-step from its own
-        // TMEM address, so the operand need not be contiguous.
-        uint32_t sa[16], da[16];
-        auto chunk = [&](const uint32_t (&sv)[16], const uint32_t (&dv)[16], int c) {
-          uint32_t pp[8], pd[8];
-          if (!slow) {
-            // every copy that exists is visible: the count c is a power of two (or 0), so it goes into the exponent -
-            // p c = 2^(s scale - lse + log2 c), exact scaling - and one rounding after the product equals the reference's
-            // rounding before it.  c = 0 (row not selected by this query block, or no copy exists): log2 c = -inf gives
-            // p = 0 and ds = 0 * finite.  Two columns at a time on the packed fp32 pipe.
-            const float lc = (act && c_static > 0.f) ? log2c : -INFINITY;
-            const float2 lc2 = make_float2(lc, lc), sl2 = make_float2(p.scale_log2, p.scale_log2);
+        const float4* lse4 = reinterpret_cast<const float4*>(smem + C::OFF_YW + ds * 512) + cg * 8;
+        const float4* del4 = reinterpret_cast<const float4*>(smem + C::OFF_XW + qs * 512) + cg * 8;
+        // Every copy that exists is visible away from the causal diagonal: the count c is a power of two (or 0), so it goes
+        // into the exponent - p c = 2^(s scale - lse + log2 c), exact scaling - and one rounding after the product equals
+        // the reference's rounding before it.  c = 0 (row not selected by this query block, or no copy exists): log2 c =
+        // -inf gives p = 0 and ds = 0 * finite.  On the diagonal the copies a query sees depend on its position, and p is
+        // kept without the count.  Two columns at a time on the packed fp32 pipe; the packed 16-bit results go back IN
+        // PLACE into columns this thread has read itself - chunk c of 16 columns into [8 c, 8 c + 8) of its group's columns -
+        // because the other groups work on the same buffers at the same time; the MMA takes every 16-element k-step from
+        // its own TMEM address, so the operand need not be contiguous.
+        const float lc = slow ? 0.f : (act && any_copy) ? (float)li : -INFINITY;
+        const float2 lc2 = make_float2(lc, lc), sl2 = make_float2(p.scale_log2, p.scale_log2);
+        auto seen = [&](int col) { return act ? (float)copies(j0, l, l_k, 1, qbase + col) : 0.f; };
+        float2 pr[16];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t sv[16], pp[8];
+          tc::tmem_ld16(tST + 16 * c, sv);
+          tc::tmem_wait_ld();
+#pragma unroll
+          for (int k = 0; k < 8; k += 2) {
+            const float4 s4 = lse4[c * 4 + (k >> 1)];
+            const float2 xa = __ffma2_rn(make_float2(__uint_as_float(sv[2 * k]), __uint_as_float(sv[2 * k + 1])), sl2,
+                                         __fadd2_rn(lc2, make_float2(s4.x, s4.y)));
+            const float2 xb = __ffma2_rn(make_float2(__uint_as_float(sv[2 * k + 2]), __uint_as_float(sv[2 * k + 3])), sl2,
+                                         __fadd2_rn(lc2, make_float2(s4.z, s4.w)));
+            pr[c * 8 + k] = make_float2(ex2f(xa.x), ex2f(xa.y));
+            pr[c * 8 + k + 1] = make_float2(ex2f(xb.x), ex2f(xb.y));
+          }
+#pragma unroll
+          for (int k = 0; k < 8; ++k) pp[k] = pack16<FMT>(pr[c * 8 + k].x, pr[c * 8 + k].y);
+          if (slow) {
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-              const float4 s2 = stat2[c * 8 + k];                     // (-lse0, -lse1, -delta0, -delta1) of the two query columns
-              const float2 x = __ffma2_rn(make_float2(__uint_as_float(sv[2 * k]), __uint_as_float(sv[2 * k + 1])), sl2,
-                                          __fadd2_rn(lc2, make_float2(s2.x, s2.y)));
-              const float2 pc = make_float2(ex2f(x.x), ex2f(x.y));
-              const float2 y = __fmul2_rn(pc, __fadd2_rn(make_float2(__uint_as_float(dv[2 * k]), __uint_as_float(dv[2 * k + 1])),
-                                                         make_float2(s2.z, s2.w)));
-              pp[k] = pack16<FMT>(pc.x, pc.y);
-              pd[k] = pack16<FMT>(y.x, y.y);
-            }
-          } else {
-            // a key block on the causal diagonal: the copies a query sees depend on its position
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              const float4 s2 = stat2[c * 8 + k];
-              const int64_t q0 = qbase + c * 16 + 2 * k;
-              const float c0 = act ? (float)copies(j0, l, l_k, 1, q0) : 0.f, c1 = act ? (float)copies(j0, l, l_k, 1, q0 + 1) : 0.f;
-              const float p0 = ex2f(fmaf(__uint_as_float(sv[2 * k]), p.scale_log2, s2.x));
-              const float p1 = ex2f(fmaf(__uint_as_float(sv[2 * k + 1]), p.scale_log2, s2.y));
-              const float y0 = p0 * (__uint_as_float(dv[2 * k]) + s2.z), y1 = p1 * (__uint_as_float(dv[2 * k + 1]) + s2.w);
-              pp[k] = pack16<FMT>(c0 > 0.f ? round16<FMT>(p0) * c0 : 0.f, c1 > 0.f ? round16<FMT>(p1) * c1 : 0.f);
-              pd[k] = pack16<FMT>(c0 > 0.f ? round16<FMT>(y0) * c0 : 0.f, c1 > 0.f ? round16<FMT>(y1) * c1 : 0.f);
+              const float c0 = seen(c * 16 + 2 * k), c1 = seen(c * 16 + 2 * k + 1);
+              pp[k] = pack16<FMT>(c0 > 0.f ? round16<FMT>(pr[c * 8 + k].x) * c0 : 0.f, c1 > 0.f ? round16<FMT>(pr[c * 8 + k].y) * c1 : 0.f);
             }
           }
           tc::tmem_st8(tST + 8 * c, pp);
-          tc::tmem_st8(tDP + 8 * c, pd);
-        };
-        tc::tmem_ld16(tST, sa); tc::tmem_ld16(tDP, da);
-        tc::tmem_wait_ld();
-        chunk(sa, da, 0);
-        tc::tmem_ld16(tST + 16, sa); tc::tmem_ld16(tDP + 16, da);
-        tc::tmem_wait_ld();
-        chunk(sa, da, 1);
+        }
         tc::tmem_wait_st();
         tc::tc_fence_before();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&ctl->p_full);
+        // ---- phase 2: dS^T over dP^T
+        ok = tc::mbar_wait(&ctl->dp_full, gp & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        // dP^T of this tile was issued behind dK of the previous one: its Q stage may be refilled
+        if (relay && !first) tc::mbar_arrive(&ctl->x_free[(gp - 1) % C::NX]);
+        tc::tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t dv[16], pd[8];
+          tc::tmem_ld16(tDP + 16 * c, dv);
+          tc::tmem_wait_ld();
+          float2 y[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const float4 d4 = del4[c * 4 + (k >> 1)];
+            y[k] = __fmul2_rn(pr[c * 8 + k], __fadd2_rn(make_float2(__uint_as_float(dv[2 * k]), __uint_as_float(dv[2 * k + 1])),
+                                                        (k & 1) ? make_float2(d4.z, d4.w) : make_float2(d4.x, d4.y)));
+            pd[k] = pack16<FMT>(y[k].x, y[k].y);
+          }
+          if (slow) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const float c0 = seen(c * 16 + 2 * k), c1 = seen(c * 16 + 2 * k + 1);
+              pd[k] = pack16<FMT>(c0 > 0.f ? round16<FMT>(y[k].x) * c0 : 0.f, c1 > 0.f ? round16<FMT>(y[k].y) * c1 : 0.f);
+            }
+          }
+          tc::tmem_st8(tDP + 8 * c, pd);
+        }
+        tc::tmem_wait_st();
+        tc::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&ctl->ds_full);
+        if (ent >> 31) { ++gp; break; }
       }
       if (!ok) break;
       // ---- the pooled rows' sums
       ok = tc::mbar_wait(&ctl->acc_full, ic & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
-      if (relay) tc::mbar_arrive(&ctl->b0_free[(gp - 1) & 1]);   // the last tile's stage
+      if (relay) { tc::mbar_arrive(&ctl->y_free[(gp - 1) % C::NY]); tc::mbar_arrive(&ctl->x_free[(gp - 1) % C::NX]); }   // the last tile's stages
       tc::tc_fence_after();
       const uint32_t tAcc = tmem + (cg < 2 ? kAccK : kAccV) + (cg & 1) * HD + lane_base;
 #pragma unroll 1
@@ -466,21 +526,22 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dkdv_tc_kernel(const __gri
 // ------------------------------------------------------------------------------------------------------------------
 template <int D, int FMT>
 __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dq_tc_kernel(const __grid_constant__ TmapQD maps, const BwdParams p) {
-  using C = BCfg<D>;
-  extern __shared__ unsigned char smem_dyn[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
-  BCtrl* ctl = reinterpret_cast<BCtrl*>(smem + C::OFF_CTRL);
-  uint32_t* items = reinterpret_cast<uint32_t*>(smem + C::OFF_LIST);      // selected blocks of the row being streamed
+  using C = KCfg<D>;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  KCtrl* ctl = reinterpret_cast<KCtrl*>(smem + C::OFF_CTRL);
   volatile int* abort_flag = &ctl->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (tc::smem_u32(smem) & 1023) {          // the swizzled tiles need it; nothing has been started yet
+    if (threadIdx.x == 0 && p.status) atomicExch(p.status, PSA_ERR_TIMEOUT);
+    return;
+  }
 
   if (threadIdx.x == 0) {
     tc::mbar_init(&ctl->a_full, 1); tc::mbar_init(&ctl->a_free, 1);
-    for (int i = 0; i < 2; ++i) {
-      tc::mbar_init(&ctl->b_full[i], 2);            // one arrival for the V copies of the tile, one for its K copies
-      tc::mbar_init(&ctl->b0_free[i], 1); tc::mbar_init(&ctl->b1_free[i], 1);
-    }
-    tc::mbar_init(&ctl->s_full, 1); tc::mbar_init(&ctl->p_full, kEwWarps);
+    for (int i = 0; i < C::NX; ++i) { tc::mbar_init(&ctl->x_full[i], 1); tc::mbar_init(&ctl->x_free[i], 1); }
+    for (int i = 0; i < C::NY; ++i) { tc::mbar_init(&ctl->y_full[i], 1); tc::mbar_init(&ctl->y_free[i], 1); }
+    tc::mbar_init(&ctl->s_full[0], 1); tc::mbar_init(&ctl->s_full[1], 1);
+    tc::mbar_init(&ctl->dp_full, 1); tc::mbar_init(&ctl->ds_full, kEwWarps);
     tc::mbar_init(&ctl->acc_full, 1); tc::mbar_init(&ctl->acc_free, kEwWarps);
     for (int i = 0; i < 3; ++i) { tc::mbar_init(&ctl->job_ready[i], 1); tc::mbar_init(&ctl->job_done[i], kEwWarps + 1); }
     ctl->abort_flag = 0;
@@ -520,28 +581,29 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dq_tc_kernel(const __grid_
       // within a head the causal rows are walked from the last query block down, the long ones first
       const int m = p.causal ? p.mq - 1 - (int)(R % p.mq) : (int)(R % p.mq);
       const int64_t bh = R / p.mq;
-      // the row's blocks, level by level (ordered compaction of the dense level row); entry: block | level index << 12 |
-      // first column (in units of 16 tokens) << 16
+      // The row's blocks, level by level, found in the dense level row 32 entries at a time and one block ahead of the tile
+      // that is put together: entry = block | level index << 12.
       const int32_t* mrow = p.mask + (bh * p.mq + m) * (int64_t)p.mask_cols;
       const int end = p.causal ? min(nk, m + 1) : nk;
-      int n_items = 0, tokens = 0;
-      for (int li = 0; li < 4; ++li) {
-        const int level = 1 << li, P = 128 >> li;
-        for (int c0 = 0; c0 < end; c0 += 32) {
-          const int c = c0 + lane;
-          const bool hit = c < end && mrow[c] == level;
-          const unsigned bits = __ballot_sync(0xffffffffu, hit);
-          const int before = __popc(bits & ((1u << lane) - 1));
-          if (hit) items[n_items + before] = (uint32_t)c | (uint32_t)li << 12 | (uint32_t)((tokens + before * P) >> 4) << 16;
-          n_items += __popc(bits);
-          tokens += __popc(bits) * P;
+      int li_next = 0, c_next = 0, c_win = 0;
+      unsigned hits = 0;
+      auto next_block = [&](uint32_t& blk) -> bool {
+        while (hits == 0 && li_next < 4) {
+          if (c_next >= end) { ++li_next; c_next = 0; continue; }
+          c_win = c_next;
+          const int c = c_win + lane;
+          hits = __ballot_sync(0xffffffffu, c < end && mrow[c] == (1 << li_next));
+          c_next += 32;
         }
-      }
-      __syncwarp();
-      const int n_tiles = (tokens + 127) >> 7;
-      const int last_cols = tokens - (n_tiles - 1) * 128;
+        if (hits == 0) return false;
+        blk = (uint32_t)(c_win + __ffs(hits) - 1) | (uint32_t)li_next << 12;
+        hits &= hits - 1;
+        return true;
+      };
+      uint32_t blk = 0;
+      bool have = next_block(blk);
       if (lane == 0) {
-        ctl->job_id[slot] = (int)R; ctl->job_n[slot] = n_tiles; ctl->job_last[slot] = last_cols;
+        ctl->job_id[slot] = (int)R; ctl->job_n[slot] = have;
         __threadfence_block();
         tc::mbar_arrive(&ctl->job_ready[slot]);
       }
@@ -549,7 +611,7 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dq_tc_kernel(const __grid_
       if (lane == 0) next = atomicAdd(p.counter, 1);
       next = __shfl_sync(0xffffffffu, next, 0);
       R = (int64_t)gridDim.x + next;
-      if (n_tiles == 0) continue;
+      if (!have) continue;
       // stationary Q and dO tiles of the query block
       ok = tc::mbar_wait(&ctl->a_free, (rc & 1) ^ 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
@@ -562,56 +624,52 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dq_tc_kernel(const __grid_
         tc::mbar_arrive_expect_tx(&ctl->a_full, 2 * C::TILE);
       }
       ++rc;
-      int ki = 0;
-      for (int t = 0; t < n_tiles && ok; ++t, ++gt) {
-        const int st = gt & 1;
-        const int probe = ki + lane;
-        const int in_tile = __popc(__ballot_sync(0xffffffffu, probe < n_items && (int)(items[probe < n_items ? probe : 0] >> 19) == t));
-        const uint32_t x = lane < in_tile ? items[ki + lane] : 0u;
-        const int li = (x >> 12) & 3, blk = x & 0xfff, P = 128 >> li, col = ((int)(x >> 16) << 4) & 127;
-        const int64_t off = p.img.off[li] + (((int64_t)bh * p.img.groups[li] + (((int64_t)blk * P) >> 3)) * C::SLABS << 10);
-        const uint32_t dstoff = (uint32_t)(col >> 3) * kGroup;
-        const uint32_t my_bytes = lane < in_tile ? (uint32_t)(P * D * 2) : 0u;
-        const uint32_t bytes = __reduce_add_sync(0xffffffffu, my_bytes);
-        // V of the stage's previous tile is free as soon as its dP is complete: the V copies leave first
-        ok = tc::mbar_wait(&ctl->b1_free[st], ((gt >> 1) & 1) ^ 1, abort_flag);
+      while (have) {
+        // the next tile: blocks packed back to back (they come in falling width, a power of two, so none straddles a tile);
+        // lane i holds block i
+        uint32_t mine = 0, flag_diag = 0;
+        int in_tile = 0, cols = 0, my_col = 0;
+        do {
+          if (lane == in_tile) { mine = blk; my_col = cols; }
+          if (p.causal && (int)(blk & 0xfffu) == m) flag_diag = 1;
+          cols += 128 >> (blk >> 12);
+          ++in_tile;
+          have = next_block(blk);
+        } while (have && cols < 128);
+        const int xs = gt % C::NX, ys = gt % C::NY;
+        const int li = (int)(mine >> 12), b = (int)(mine & 0xfffu), P = 128 >> li;
+        const int64_t off = p.img.off[li] + (((int64_t)bh * p.img.groups[li] + (((int64_t)b * P) >> 3)) * C::SLABS << 10);
+        const uint32_t dstoff = (uint32_t)(my_col >> 3) * kGroup, my_bytes = (uint32_t)(P * D * 2), bytes = (uint32_t)(cols * D * 2);
+        // K and the words beside it: free once dQ of the stage's previous tile is complete
+        ok = tc::mbar_wait(&ctl->x_free[xs], ((gt / C::NX) & 1) ^ 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         if (lane < in_tile)
-          tc::bulk_load_a(tc::smem_u32(smem + C::OFF_B1 + st * C::TILE) + dstoff, p.vimg + off, my_bytes, tc::smem_u32(&ctl->b_full[st]));
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive_expect_tx(&ctl->b_full[st], bytes);
-        // K is read last (by dQ += dS K): its release also says that the metadata of the stage are no longer needed
-        ok = tc::mbar_wait(&ctl->b0_free[st], ((gt >> 1) & 1) ^ 1, abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        if (lane < in_tile)
-          tc::bulk_load_a(tc::smem_u32(smem + C::OFF_B0 + st * C::TILE) + dstoff, p.kimg + off, my_bytes, tc::smem_u32(&ctl->b_full[st]));
-        // per-column metadata, written by the whole warp block after block: (first original position, positions that
-        // exist from there, level, copies when nothing hides them); absent columns: zeros
-        int4* meta = reinterpret_cast<int4*>(smem + C::OFF_META + st * 2048);
-        float* lcol = reinterpret_cast<float*>(smem + C::OFF_LC + st * 512);
-        int flag_diag = 0;
-        for (int b = 0; b < in_tile; ++b) {
-          const int b_li = __shfl_sync(0xffffffffu, li, b), b_blk = __shfl_sync(0xffffffffu, blk, b);
-          const int b_col = __shfl_sync(0xffffffffu, col, b);
+          tc::bulk_load_a(tc::smem_u32(smem + C::OFF_X + xs * C::TILE) + dstoff, p.kimg + off, my_bytes, tc::smem_u32(&ctl->x_full[xs]));
+        // Per 16 columns the first original position and the level of their block (read on the causal diagonal only), per
+        // column log2 of the copies that exist (-inf: none), written by the whole warp block after block.
+        int2* units = reinterpret_cast<int2*>(smem + C::OFF_YW + xs * 64);
+        float* lcol = reinterpret_cast<float*>(smem + C::OFF_XW + xs * 512);
+        for (int i = 0; i < in_tile; ++i) {
+          const int b_li = __shfl_sync(0xffffffffu, li, i), b_b = __shfl_sync(0xffffffffu, b, i), b_col = __shfl_sync(0xffffffffu, my_col, i);
           const int b_l = 1 << b_li, b_P = 128 >> b_li;
-          const int64_t l_k = b_li == 0 ? p.seq : p.s_pad;
-          for (int c = lane; c < b_P; c += 32) {
-            const int64_t j0 = ((int64_t)b_blk * b_P + c) * b_l;
-            const int64_t avail = l_k - j0;
-            const int cs = avail < 0 ? 0 : (avail > b_l ? b_l : (int)avail);
-            meta[b_col + c] = make_int4((int)j0, (int)min(avail, (int64_t)1 << 30), b_l, 0);
-            lcol[b_col + c] = cs > 0 ? (float)b_li : -INFINITY;      // cs is 0 or the level 2^li
-          }
-          if (p.causal && b_blk == m) flag_diag = 1;
+          const int64_t l_k = b_li == 0 ? p.seq : p.s_pad, first = (int64_t)b_b * 128;
+          for (int c = lane; c < b_P; c += 32) lcol[b_col + c] = first + (int64_t)c * b_l < l_k ? (float)b_li : -INFINITY;
+          if (lane < b_P / 16) units[b_col / 16 + lane] = make_int2((int)first + lane * 16 * b_l, b_li);
         }
-        const int used = t == n_tiles - 1 ? last_cols : 128;
-        for (int c = used + lane; c < 128; c += 32) { meta[c] = make_int4(0, 0, 0, 0); lcol[c] = -INFINITY; }
-        if (lane == 0) ctl->tile_flag[st] = flag_diag;
-        ki += in_tile;
+        for (int c = cols + lane; c < 128; c += 32) lcol[c] = -INFINITY;
+        if (lane == 0) ctl->ent[xs] = (uint32_t)cols | flag_diag << 16 | (have ? 0u : 1u << 31);
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive_expect_tx(&ctl->b_full[st], bytes);
+        if (lane == 0) tc::mbar_arrive_expect_tx(&ctl->x_full[xs], bytes);
+        // V: free once dP of the stage's previous tile is complete
+        ok = tc::mbar_wait(&ctl->y_free[ys], ((gt / C::NY) & 1) ^ 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        if (lane < in_tile)
+          tc::bulk_load_a(tc::smem_u32(smem + C::OFF_Y + ys * C::TILE) + dstoff, p.vimg + off, my_bytes, tc::smem_u32(&ctl->y_full[ys]));
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive_expect_tx(&ctl->y_full[ys], bytes);
+        ++gt;
       }
     }
   } else if (warp == 1) {
@@ -622,37 +680,28 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dq_tc_kernel(const __grid_
       const uint32_t idesc_full = tc::make_idesc(FMT, 128, 128, 0, 0);
       const uint64_t qdesc = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_A0), 16, 1024);
       const uint64_t ddesc = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_A1), 16, 1024);
-      const uint64_t kk0 = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_B0), 16, kGroup);     // stream tiles as K-major B
-      const uint64_t vk0 = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_B1), 16, kGroup);
-      const uint64_t km0 = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_B0), 1024, kGroup);   // K tile as MN-major B
+      const uint64_t kk0 = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_X), 16, kGroup);      // stream tiles as K-major B
+      const uint64_t vk0 = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_Y), 16, kGroup);
+      const uint64_t km0 = tc::make_smem_desc(tc::smem_u32(smem + C::OFF_X), 1024, kGroup);    // K tile as MN-major B
       const uint32_t ctl_a = tc::smem_u32(ctl);
-      const uint32_t s_full_a = ctl_a + (uint32_t)offsetof(BCtrl, s_full), p_full_a = ctl_a + (uint32_t)offsetof(BCtrl, p_full);
-      const uint32_t b_full_a = ctl_a + (uint32_t)offsetof(BCtrl, b_full);
-      int g0 = 0, rc = 0;                                   // stream tiles of the rows before this one / rows with work
-      // S = Q K^T of tile u of the row (stage and score buffer by the running tile count), N = its columns
-      auto issue_S = [&](int gu, int cols) {
-        const uint64_t kd = kk0 + (uint64_t)((uint32_t)((gu & 1) * C::TILE) >> 4);
-        const uint32_t idesc = cols == 128 ? idesc_full : tc::make_idesc(FMT, 128, cols, 0, 0);
-        const uint32_t ts = tmem + kS + (gu & 1) * 128;
-#pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks)
-          tc::umma_ss(ts, qdesc + (uint64_t)(((ks >> 2) * kSlab + (ks & 3) * 32) >> 4),
-                      kd + (uint64_t)(((ks >> 2) * 1024 + (ks & 3) * 32) >> 4), idesc, ks > 0 ? 1u : 0u);
-      };
-      // dP = dO V^T of the same tile; its commit covers every product issued before it
-      auto issue_dP = [&](int gu, int cols) {
-        const uint64_t vd = vk0 + (uint64_t)((uint32_t)((gu & 1) * C::TILE) >> 4);
+      const uint32_t s_full_a = ctl_a + (uint32_t)offsetof(KCtrl, s_full), ds_full_a = ctl_a + (uint32_t)offsetof(KCtrl, ds_full);
+      const uint32_t dp_full_a = ctl_a + (uint32_t)offsetof(KCtrl, dp_full);
+      const uint32_t x_full_a = ctl_a + (uint32_t)offsetof(KCtrl, x_full), y_full_a = ctl_a + (uint32_t)offsetof(KCtrl, y_full);
+      const volatile uint32_t* ent = ctl->ent;
+      auto x_off = [&](int u) { return (uint64_t)((uint32_t)((u % C::NX) * C::TILE) >> 4); };
+      auto y_off = [&](int u) { return (uint64_t)((uint32_t)((u % C::NY) * C::TILE) >> 4); };
+      // a stationary tile times a stream tile, N = the tile's columns
+      auto issue_ss = [&](uint32_t dst, uint64_t adesc, uint64_t bdesc, int cols, uint32_t done) {
         const uint32_t idesc = cols == 128 ? idesc_full : tc::make_idesc(FMT, 128, cols, 0, 0);
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks)
-          tc::umma_ss(tmem + kDP, ddesc + (uint64_t)(((ks >> 2) * kSlab + (ks & 3) * 32) >> 4),
-                      vd + (uint64_t)(((ks >> 2) * 1024 + (ks & 3) * 32) >> 4), idesc, ks > 0 ? 1u : 0u);
-        tc::umma_commit_a(s_full_a);
+          tc::umma_ss(dst, adesc + (uint64_t)(((ks >> 2) * kSlab + (ks & 3) * 32) >> 4),
+                      bdesc + (uint64_t)(((ks >> 2) * 1024 + (ks & 3) * 32) >> 4), idesc, ks > 0 ? 1u : 0u);
+        tc::umma_commit_a(done);
       };
       // dQ += dS K; k-step ks = columns [16 ks, 16 ks + 16) of the tile, whose 16-bit operand sits at column
       // 32 (ks / 2) + 8 (ks % 2) of the dP buffer
-      auto issue_acc = [&](int gu, int cols, bool first) {
-        const uint64_t kd = km0 + (uint64_t)((uint32_t)((gu & 1) * C::TILE) >> 4);
+      auto issue_acc = [&](uint64_t kd, int cols, bool first) {
         if (cols == 128) {
           tc::umma_ts(tmem + kAcc, tmem + kDP, kd, idesc_acc, first ? 0u : 1u);
 #pragma unroll
@@ -664,49 +713,47 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dq_tc_kernel(const __grid_
                         (first && ks == 0) ? 0u : 1u);
         }
       };
+      int g0 = 0, rc = 0;                                   // stream tiles of the rows before this one / rows with work
       for (int it = 0; ok; ++it) {
         const int slot = it % 3;
         ok = tc::mbar_wait(&ctl->job_ready[slot], (it / 3) & 1, abort_flag);
         if (!ok || ctl->job_id[slot] < 0) break;
-        const int n = ctl->job_n[slot], last_cols = ctl->job_last[slot];
-        if (n == 0) { tc::mbar_arrive(&ctl->job_done[slot]); continue; }
-        auto cols_of = [&](int u) { return u == n - 1 ? last_cols : 128; };
+        if (ctl->job_n[slot] == 0) { tc::mbar_arrive(&ctl->job_done[slot]); continue; }
         ok = tc::mbar_wait(&ctl->a_full, rc & 1, abort_flag);
-        if (ok) ok = tc::mbar_wait_a(b_full_a + (g0 & 1) * 8, (g0 >> 1) & 1, abort_flag);
         if (!ok) break;
         tc::tc_fence_after();
-        issue_S(g0, cols_of(0));
-        issue_dP(g0, cols_of(0));
-        // S of tile u+1 is issued as soon as its operands are there, dQ of tile u and dP of tile u+1 when the element-wise
-        // warps are done with tile u: the issuer polls for whichever comes first
-        int s_issued = 1, t = 0;
+        // Running tile numbers: next S, next dP, next dQ.  S runs up to two tiles ahead of dQ (two score buffers; the scores
+        // of tile u-2 have been read once its dS is there), dP goes into the one buffer that dQ of the tile before has read
+        // (the tensor pipe runs in issue order).  The issuer polls for whichever comes first.
+        int ns = g0, np = g0, na = g0;
+        bool s_done = false, done = false;
         uint32_t idle = 0;
-        while (ok && t < n) {
+        while (ok && !done) {
           bool progressed = false;
-          if (s_issued < n && s_issued <= t + 1 && tc::mbar_test_wait_a(b_full_a + ((g0 + s_issued) & 1) * 8, ((g0 + s_issued) >> 1) & 1)) {
-            tc::tc_fence_after();
-            issue_S(g0 + s_issued, cols_of(s_issued));
-            ++s_issued;
-            progressed = true;
-          }
-          if (tc::mbar_test_wait_a(p_full_a, (g0 + t) & 1)) {
-            if (t == 0 && rc > 0) {
+          if (na < np && tc::mbar_test_wait_a(ds_full_a, na & 1)) {
+            if (na == g0 && rc > 0) {
               ok = tc::mbar_wait(&ctl->acc_free, (rc - 1) & 1, abort_flag);
               if (!ok) break;
             }
             tc::tc_fence_after();
-            issue_acc(g0 + t, cols_of(t), t == 0);
-            if (t + 1 < n) {
-              if (s_issued == t + 1) {      // its K/V stage has not landed yet
-                ok = tc::mbar_wait_a(b_full_a + ((g0 + t + 1) & 1) * 8, ((g0 + t + 1) >> 1) & 1, abort_flag);
-                if (!ok) break;
-                tc::tc_fence_after();
-                issue_S(g0 + t + 1, cols_of(t + 1));
-                ++s_issued;
-              }
-              issue_dP(g0 + t + 1, cols_of(t + 1));
-            }
-            ++t;
+            const uint32_t e = ent[na % C::NX];
+            issue_acc(km0 + x_off(na), (int)(e & 0xffffu), na == g0);
+            done = (e >> 31) != 0;
+            ++na;
+            progressed = true;
+          }
+          if (np < ns && np == na && tc::mbar_test_wait_a(y_full_a + (np % C::NY) * 8, (np / C::NY) & 1)) {
+            tc::tc_fence_after();
+            issue_ss(tmem + kDP, ddesc, vk0 + y_off(np), (int)(ent[np % C::NX] & 0xffffu), dp_full_a);   // also says: dQ of the tile before is complete
+            ++np;
+            progressed = true;
+          }
+          if (!s_done && ns <= na + 1 && tc::mbar_test_wait_a(x_full_a + (ns % C::NX) * 8, (ns / C::NX) & 1)) {
+            tc::tc_fence_after();
+            const uint32_t e = ent[ns % C::NX];
+            issue_ss(tmem + kS + (ns & 1) * 128, qdesc, kk0 + x_off(ns), (int)(e & 0xffffu), s_full_a + (ns & 1) * 8);
+            s_done = (e >> 31) != 0;
+            ++ns;
             progressed = true;
           }
           if (progressed) {
@@ -721,7 +768,7 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dq_tc_kernel(const __grid_
         tc::umma_commit(&ctl->a_free);
         tc::mbar_arrive(&ctl->job_done[slot]);
         ++rc;
-        g0 += n;
+        g0 = na;
       }
     }
   } else {
@@ -741,13 +788,12 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dq_tc_kernel(const __grid_
       if (!ok) break;
       const int64_t R = ctl->job_id[slot];
       if (R < 0) break;
-      const int n = ctl->job_n[slot], last_cols = ctl->job_last[slot];
       const int m = p.causal ? p.mq - 1 - (int)(R % p.mq) : (int)(R % p.mq);
       const int64_t bh = R / p.mq;
       const int64_t qpos = (int64_t)m * 128 + r;
       constexpr int QD = D / 4;                               // channels of the row each group stores
       uint16_t* orow = reinterpret_cast<uint16_t*>(p.dq) + ((int64_t)bh * p.seq + qpos) * D + cg * QD;
-      if (n == 0) {
+      if (ctl->job_n[slot] == 0) {
         if (qpos < p.seq)
           for (int c = 0; c < QD; c += 8) *reinterpret_cast<uint4*>(orow + c) = make_uint4(0u, 0u, 0u, 0u);
         __syncwarp();
@@ -755,79 +801,98 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dq_tc_kernel(const __grid_
         continue;
       }
       // (-lse * log2 e, -delta) of this row; -inf for rows past the end
-      const float* my_pair = p.stat + ((bh * p.s_pad + qpos) >> 1) * 4 + (qpos & 1);
-      const float2 my = make_float2(my_pair[0], my_pair[2]);
-      for (int t = 0; t < n && ok; ++t, ++gt) {
-        const int st = gt & 1;
-        const int used = t == n - 1 ? last_cols : 128;
-        ok = tc::mbar_wait(&ctl->s_full, gt & 1, abort_flag);
+      const float2 my = make_float2(p.nlse[bh * p.s_pad + qpos], p.ndelta[bh * p.s_pad + qpos]);
+      const float2 sl2 = make_float2(p.scale_log2, p.scale_log2), nlse2 = make_float2(my.x, my.x), ndel2 = make_float2(my.y, my.y);
+      for (bool first = true; ok; first = false, ++gt) {
+        const int xs = gt % C::NX;
+        // ---- phase 1: the probabilities.  They need S only, which is computed while the tile before this one is still worked
+        // on, so their ex2 (the longer half of the element-wise work) run under dQ of the previous tile and dP of this one.
+        // They stay in registers until dP is there.
+        ok = tc::mbar_wait(&ctl->s_full[gt & 1], (gt >> 1) & 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        // S and dP of this tile are complete, and so is dQ of the previous tile: V of this tile and K of the previous one
-        // may be replaced
-        if (relay) {
-          tc::mbar_arrive(&ctl->b1_free[st]);
-          if (t > 0) tc::mbar_arrive(&ctl->b0_free[st ^ 1]);
-        }
-        if (cg * 32 < used) {
+        const uint32_t ent = ctl->ent[xs];
+        const bool mine = cg * 32 < (int)(ent & 0xffffu), slow = (ent >> 16) & 1u;
+        float2 pr[16];
+        if (mine) {
           tc::tc_fence_after();
-          const uint32_t tS = tmem + kS + st * 128 + cg * 32 + lane_base;
-          const int4* meta = reinterpret_cast<const int4*>(smem + C::OFF_META + st * 2048) + cg * 32;
-          const float2* lc2 = reinterpret_cast<const float2*>(smem + C::OFF_LC + st * 512) + cg * 16;
-          const bool slow = ctl->tile_flag[st] != 0;
-          const float2 sl2 = make_float2(p.scale_log2, p.scale_log2), nlse2 = make_float2(my.x, my.x), ndel2 = make_float2(my.y, my.y);
-          uint32_t sa[16], da[16];
-          auto chunk = [&](const uint32_t (&sv)[16], const uint32_t (&dv)[16], int c) {
-            uint32_t pd[8];
-            if (!slow) {
-              // the copy count of a column is a power of two (or 0): it goes into the exponent, p c = 2^(s scale - lse +
-              // log2 c), so one rounding after the product equals the reference's rounding before it; log2 c = -inf
-              // (no copy exists) gives 0.  Two columns at a time on the packed fp32 pipe.
+          const float4* lc4 = reinterpret_cast<const float4*>(smem + C::OFF_XW + xs * 512) + cg * 8;
+          uint32_t sv[32];
+          tc::tmem_ld32(tmem + kS + (gt & 1) * 128 + cg * 32 + lane_base, sv);
+          tc::tmem_wait_ld();
+          // the copy count of a column is a power of two (or 0): it goes into the exponent, p c = 2^(s scale - lse +
+          // log2 c), so one rounding after the product equals the reference's rounding before it; log2 c = -inf
+          // (no copy exists) gives 0.  On the causal diagonal the count follows in phase 2 and p is kept without it.  Two
+          // columns at a time on the packed fp32 pipe.
+          if (!slow) {
 #pragma unroll
-              for (int k = 0; k < 8; ++k) {
-                const float2 x = __ffma2_rn(make_float2(__uint_as_float(sv[2 * k]), __uint_as_float(sv[2 * k + 1])), sl2,
-                                            __fadd2_rn(lc2[c * 8 + k], nlse2));
-                const float2 pc = make_float2(ex2f(x.x), ex2f(x.y));
-                const float2 y = __fmul2_rn(pc, __fadd2_rn(make_float2(__uint_as_float(dv[2 * k]), __uint_as_float(dv[2 * k + 1])), ndel2));
-                pd[k] = pack16<FMT>(y.x, y.y);
-              }
-            } else {
-#pragma unroll
-              for (int k = 0; k < 8; ++k) {
-                const int4 m0 = meta[c * 16 + 2 * k], m1 = meta[c * 16 + 2 * k + 1];
-                const int v0 = min(m0.y, (int)min(qpos + 1 - (int64_t)m0.x, (int64_t)1 << 30));
-                const int v1 = min(m1.y, (int)min(qpos + 1 - (int64_t)m1.x, (int64_t)1 << 30));
-                const float c0 = (float)max(0, min(v0, m0.z)), c1 = (float)max(0, min(v1, m1.z));
-                const float p0 = ex2f(fmaf(__uint_as_float(sv[2 * k]), p.scale_log2, my.x));
-                const float p1 = ex2f(fmaf(__uint_as_float(sv[2 * k + 1]), p.scale_log2, my.x));
-                const float y0 = p0 * (__uint_as_float(dv[2 * k]) + my.y), y1 = p1 * (__uint_as_float(dv[2 * k + 1]) + my.y);
-                pd[k] = pack16<FMT>(c0 > 0.f ? round16<FMT>(y0) * c0 : 0.f, c1 > 0.f ? round16<FMT>(y1) * c1 : 0.f);
-              }
+            for (int k = 0; k < 16; ++k) {
+              const float4 l4 = lc4[k >> 1];
+              const float2 x = __ffma2_rn(make_float2(__uint_as_float(sv[2 * k]), __uint_as_float(sv[2 * k + 1])), sl2,
+                                          __fadd2_rn((k & 1) ? make_float2(l4.z, l4.w) : make_float2(l4.x, l4.y), nlse2));
+              pr[k] = make_float2(ex2f(x.x), ex2f(x.y));
             }
-            tc::tmem_st8(tDP + 8 * c, pd);
-          };
+          } else {
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+              const float2 x = __ffma2_rn(make_float2(__uint_as_float(sv[2 * k]), __uint_as_float(sv[2 * k + 1])), sl2, nlse2);
+              pr[k] = make_float2(ex2f(x.x), ex2f(x.y));
+            }
+          }
+        }
+        // ---- phase 2: dS over dP
+        ok = tc::mbar_wait(&ctl->dp_full, gt & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        // dP of this tile is complete, and so is dQ of the previous tile: V of this tile and K of the previous one may be
+        // replaced
+        if (relay) {
+          tc::mbar_arrive(&ctl->y_free[gt % C::NY]);
+          if (!first) tc::mbar_arrive(&ctl->x_free[(gt - 1) % C::NX]);
+        }
+        if (mine) {
+          tc::tc_fence_after();
+          const int2* units = reinterpret_cast<const int2*>(smem + C::OFF_YW + xs * 64) + cg * 2;
           // this thread's 32 columns in two chunks of 16, one after the other; the packed results go back in place into
           // columns of the dP buffer the thread has read itself (chunk c into [8 c, 8 c + 8) of its group's columns),
           // because the other groups work on the same buffer at the same time.  Columns past the tile's end hold stale
           // bits and are never read by a product.
-          tc::tmem_ld16(tS, sa); tc::tmem_ld16(tDP, da);
-          tc::tmem_wait_ld();
-          chunk(sa, da, 0);
-          tc::tmem_ld16(tS + 16, sa); tc::tmem_ld16(tDP + 16, da);
-          tc::tmem_wait_ld();
-          chunk(sa, da, 1);
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            uint32_t dv[16], pd[8];
+            tc::tmem_ld16(tDP + 16 * c, dv);
+            tc::tmem_wait_ld();
+            float2 y[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              y[k] = __fmul2_rn(pr[c * 8 + k], __fadd2_rn(make_float2(__uint_as_float(dv[2 * k]), __uint_as_float(dv[2 * k + 1])), ndel2));
+              pd[k] = pack16<FMT>(y[k].x, y[k].y);
+            }
+            if (slow) {
+              const int2 u = units[c];
+              const int l = 1 << u.y;
+              const int64_t l_k = u.y == 0 ? p.seq : p.s_pad;
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                const float c0 = (float)copies((int64_t)u.x + 2 * k * l, l, l_k, 1, qpos), c1 = (float)copies((int64_t)u.x + (2 * k + 1) * l, l, l_k, 1, qpos);
+                pd[k] = pack16<FMT>(c0 > 0.f ? round16<FMT>(y[k].x) * c0 : 0.f, c1 > 0.f ? round16<FMT>(y[k].y) * c1 : 0.f);
+              }
+            }
+            tc::tmem_st8(tDP + 8 * c, pd);
+          }
           tc::tmem_wait_st();
           tc::tc_fence_before();
         }
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&ctl->p_full);
+        if (lane == 0) tc::mbar_arrive(&ctl->ds_full);
+        if (ent >> 31) { ++gt; break; }
       }
       if (!ok) break;
       // ---- dQ rows: each group stores a quarter of the channels
       ok = tc::mbar_wait(&ctl->acc_full, rc & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
-      if (relay) tc::mbar_arrive(&ctl->b0_free[(gt - 1) & 1]);   // K of the row's last tile
+      if (relay) tc::mbar_arrive(&ctl->x_free[(gt - 1) % C::NX]);   // K of the row's last tile
       tc::tc_fence_after();
       const uint32_t tAcc = tmem + kAcc + cg * QD + lane_base;
 #pragma unroll
@@ -871,14 +936,14 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dq_tc_kernel(const __grid_
 // ------------------------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256) bwd_stat_kernel(const T* __restrict__ o, const T* __restrict__ dout, const float* __restrict__ lse,
-                                                       float* __restrict__ stat, int64_t bh, int64_t seq, int64_t s_pad, int D) {
+                                                       float* __restrict__ nlse, float* __restrict__ ndelta, int64_t bh, int64_t seq,
+                                                       int64_t s_pad, int D) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * 8 + warp;       // over bh * s_pad
   if (row >= bh * s_pad) return;
   const int64_t b = row / s_pad, t = row - b * s_pad;
-  float* dst = stat + (row >> 1) * 4 + (row & 1);           // per pair of rows: (-lse0, -lse1, -delta0, -delta1)
   if (t >= seq) {
-    if (lane == 0) { dst[0] = -INFINITY; dst[2] = 0.f; }
+    if (lane == 0) { nlse[row] = -INFINITY; ndelta[row] = 0.f; }
     return;
   }
   const int64_t src = (b * seq + t) * D;
@@ -891,8 +956,8 @@ __global__ void __launch_bounds__(256) bwd_stat_kernel(const T* __restrict__ o, 
   if (lane == 0) {
     const float l = lse[b * seq + t];
     // a row that saw no key has lse = -inf; its probabilities are taken as 0 (the reference leaves them undefined)
-    dst[0] = l == -INFINITY ? -INFINITY : -l * 1.4426950408889634f;
-    dst[2] = -acc;
+    nlse[row] = l == -INFINITY ? -INFINITY : -l * 1.4426950408889634f;
+    ndelta[row] = -acc;
   }
 }
 
@@ -940,14 +1005,15 @@ __global__ void __launch_bounds__(256) bwd_fold_kernel(BwdParams p, T* __restric
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 struct Scratch {
-  size_t stat, pooled[8], items, counters, total;
+  size_t nlse, ndelta, pooled[8], items, counters, total;
 };
 
 Scratch scratch_layout(int64_t bh, int64_t seq, int D) {
   Scratch s;
   const int64_t nk = cdiv64(seq, 128), s_pad = nk * 128;
   size_t off = 0;
-  s.stat = off; off += align256((size_t)bh * s_pad * sizeof(float2));
+  s.nlse = off; off += align256((size_t)bh * s_pad * sizeof(float));
+  s.ndelta = off; off += align256((size_t)bh * s_pad * sizeof(float));
   for (int i = 0; i < 8; ++i) {
     s.pooled[i] = off;
     off += align256((size_t)bh * (s_pad >> (i & 3)) * D * sizeof(float));
@@ -962,14 +1028,15 @@ template <typename T, int D, int FMT>
 int launch_bwd_tc(const void* q, const void* kimg, const void* vimg, const int32_t* mask, const void* out, const float* lse,
                   const void* dout, void* dq, void* dk, void* dv, unsigned char* scratch, int64_t bh, int64_t seq, int mask_cols,
                   float scale, int causal, int32_t* status, cudaStream_t st) {
-  using C = BCfg<D>;
+  constexpr int kSmem = KCfg<D>::SMEM;
   const int nk = (int)cdiv64(seq, 128);
   const int64_t s_pad = (int64_t)nk * 128;
   const Scratch L = scratch_layout(bh, seq, D);
   BwdParams p;
   p.mask = mask; p.kimg = (const unsigned char*)kimg; p.vimg = (const unsigned char*)vimg;
   p.img = make_img_levels(bh, seq, D, 128);
-  p.stat = reinterpret_cast<const float*>(scratch + L.stat);
+  p.nlse = reinterpret_cast<const float*>(scratch + L.nlse);
+  p.ndelta = reinterpret_cast<const float*>(scratch + L.ndelta);
   p.dq = dq;
   for (int i = 0; i < 4; ++i) {
     p.dkp[i] = reinterpret_cast<float*>(scratch + L.pooled[i]);
@@ -986,7 +1053,8 @@ int launch_bwd_tc(const void* q, const void* kimg, const void* vimg, const int32
   PSA_REQUIRE(e == cudaSuccess, PSA_ERR_CUDA, "psa_legacy_bwd_tcgen05: cudaMemsetAsync failed: %s", cudaGetErrorString(e));
 
   bwd_stat_kernel<T><<<(unsigned)cdiv64(bh * s_pad, 8), 256, 0, st>>>((const T*)out, (const T*)dout, lse,
-                                                                     reinterpret_cast<float*>(scratch + L.stat), bh, seq, s_pad, D);
+                                                                     reinterpret_cast<float*>(scratch + L.nlse),
+                                                                     reinterpret_cast<float*>(scratch + L.ndelta), bh, seq, s_pad, D);
   PSA_CHECK_LAUNCH("psa_legacy_bwd_tcgen05(row statistics)");
   bwd_items_kernel<<<1, 32, 0, st>>>(reinterpret_cast<int2*>(scratch + L.items), nk);
   PSA_CHECK_LAUNCH("psa_legacy_bwd_tcgen05(work list)");
@@ -1001,19 +1069,19 @@ int launch_bwd_tc(const void* q, const void* kimg, const void* vimg, const int32
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   PSA_REQUIRE(sms > 0, PSA_ERR_CUDA, "psa_legacy_bwd_tcgen05: cannot read the SM count");
   {
-    e = cudaFuncSetAttribute(bwd_dq_tc_kernel<D, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-    PSA_REQUIRE(e == cudaSuccess, PSA_ERR_CUDA, "psa_legacy_bwd_tcgen05: shared-memory opt-in (%d B) failed: %s", C::SMEM, cudaGetErrorString(e));
+    e = cudaFuncSetAttribute(bwd_dq_tc_kernel<D, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    PSA_REQUIRE(e == cudaSuccess, PSA_ERR_CUDA, "psa_legacy_bwd_tcgen05: shared-memory opt-in (%d B) failed: %s", kSmem, cudaGetErrorString(e));
     const int64_t rows = (int64_t)nk * bh;
     p.counter = counters;
-    bwd_dq_tc_kernel<D, FMT><<<(unsigned)(rows < sms ? rows : sms), kThreadsBwd, C::SMEM, st>>>(maps, p);
+    bwd_dq_tc_kernel<D, FMT><<<(unsigned)(rows < sms ? rows : sms), kThreadsBwd, kSmem, st>>>(maps, p);
     PSA_CHECK_LAUNCH("psa_legacy_bwd_tcgen05(dq)");
   }
   {
-    e = cudaFuncSetAttribute(bwd_dkdv_tc_kernel<D, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-    PSA_REQUIRE(e == cudaSuccess, PSA_ERR_CUDA, "psa_legacy_bwd_tcgen05: shared-memory opt-in (%d B) failed: %s", C::SMEM, cudaGetErrorString(e));
+    e = cudaFuncSetAttribute(bwd_dkdv_tc_kernel<D, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    PSA_REQUIRE(e == cudaSuccess, PSA_ERR_CUDA, "psa_legacy_bwd_tcgen05: shared-memory opt-in (%d B) failed: %s", kSmem, cudaGetErrorString(e));
     const int64_t jobs = (int64_t)n_entries * bh;
     p.counter = counters + 16;
-    bwd_dkdv_tc_kernel<D, FMT><<<(unsigned)(jobs < sms ? jobs : sms), kThreadsBwd, C::SMEM, st>>>(maps, p);
+    bwd_dkdv_tc_kernel<D, FMT><<<(unsigned)(jobs < sms ? jobs : sms), kThreadsBwd, kSmem, st>>>(maps, p);
     PSA_CHECK_LAUNCH("psa_legacy_bwd_tcgen05(dk, dv)");
   }
   const int64_t work = bh * seq * (D / 4);
