@@ -934,72 +934,125 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dq_tc_kernel(const __grid_
 // ------------------------------------------------------------------------------------------------------------------
 // Small kernels around the two: row statistics, the dK/dV work list, the fold of the pooled sums.
 // ------------------------------------------------------------------------------------------------------------------
-template <typename T>
+// Row statistics; block 0 also zeroes the work counters and writes the work list of the dK/dV kernel: every (level, group
+// of 128 pooled rows), ordered by the group's first key block, so that under a causal mask the groups with the most query
+// blocks come first.  HBM-bound (o and dO are read once): D/8 lanes share a row, 16 bytes each, and a thread has the words
+// of four rows in flight.  32 heads x 32768 x 128: 204 -> 128 us (4.2 TB/s).
+template <typename T, int D>
 __global__ void __launch_bounds__(256) bwd_stat_kernel(const T* __restrict__ o, const T* __restrict__ dout, const float* __restrict__ lse,
                                                        float* __restrict__ nlse, float* __restrict__ ndelta, int64_t bh, int64_t seq,
-                                                       int64_t s_pad, int D) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t row = (int64_t)blockIdx.x * 8 + warp;       // over bh * s_pad
-  if (row >= bh * s_pad) return;
-  const int64_t b = row / s_pad, t = row - b * s_pad;
-  if (t >= seq) {
-    if (lane == 0) { nlse[row] = -INFINITY; ndelta[row] = 0.f; }
-    return;
+                                                       int64_t s_pad, int2* __restrict__ items, int nk, int* __restrict__ counters, int o_aligned) {
+  constexpr int CPR = D / 8, kRows = 256 / CPR, kUnroll = 4;
+  if (blockIdx.x == 0) {
+    if (threadIdx.x < 64) counters[threadIdx.x] = 0;
+    for (int blk = threadIdx.x; blk < nk; blk += 256) {
+      int n = blk + (blk + 1) / 2 + (blk + 3) / 4 + (blk + 7) / 8;      // entries of the blocks before this one
+      for (int li = 0; li < 4; ++li)
+        if ((blk & ((1 << li) - 1)) == 0) items[n++] = make_int2(li, blk >> li);
+    }
   }
-  const int64_t src = (b * seq + t) * D;
-  float acc = 0.f;
-  for (int c = lane * 2; c < D; c += 64) {
-    acc = fmaf(Elem<T>::to_f(o[src + c]), Elem<T>::to_f(dout[src + c]), acc);
-    acc = fmaf(Elem<T>::to_f(o[src + c + 1]), Elem<T>::to_f(dout[src + c + 1]), acc);
+  const int c = threadIdx.x % CPR;
+  const int64_t row0 = (int64_t)blockIdx.x * (kRows * kUnroll) + threadIdx.x / CPR;      // over bh * s_pad
+  uint4 a[kUnroll], d[kUnroll];
+  int64_t src[kUnroll];
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u) {
+    const int64_t row = row0 + u * kRows, b = row / s_pad, t = row - b * s_pad;
+    src[u] = row < bh * s_pad && t < seq ? b * seq + t : -1;
+    if (src[u] >= 0) {
+      if (o_aligned) {
+        a[u] = __ldg(reinterpret_cast<const uint4*>(o) + src[u] * CPR + c);
+      } else {      // dO feeds a tensor map and is always aligned, o need not be
+        T* e = reinterpret_cast<T*>(&a[u]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) e[i] = o[(src[u] * CPR + c) * 8 + i];
+      }
+      d[u] = __ldg(reinterpret_cast<const uint4*>(dout) + src[u] * CPR + c);
+    }
   }
-  for (int off = 16; off; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-  if (lane == 0) {
-    const float l = lse[b * seq + t];
-    // a row that saw no key has lse = -inf; its probabilities are taken as 0 (the reference leaves them undefined)
-    nlse[row] = l == -INFINITY ? -INFINITY : -l * 1.4426950408889634f;
-    ndelta[row] = -acc;
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u) {
+    const int64_t row = row0 + u * kRows;
+    float acc = 0.f;
+    if (src[u] >= 0) {
+      const T* x = reinterpret_cast<const T*>(&a[u]);
+      const T* y = reinterpret_cast<const T*>(&d[u]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc = fmaf(Elem<T>::to_f(x[i]), Elem<T>::to_f(y[i]), acc);
+    }
+#pragma unroll
+    for (int off = CPR / 2; off; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    if (c == 0 && row < bh * s_pad) {
+      const float l = src[u] >= 0 ? lse[src[u]] : -INFINITY;
+      // a row that saw no key has lse = -inf; its probabilities are taken as 0 (the reference leaves them undefined)
+      nlse[row] = l == -INFINITY ? -INFINITY : -l * 1.4426950408889634f;
+      ndelta[row] = src[u] >= 0 ? -acc : 0.f;
+    }
   }
-}
-
-// Work list of the dK/dV kernel: every (level, group of 128 pooled rows), ordered by the group's first key block, so
-// that under a causal mask the groups with the most query blocks come first.
-__global__ void bwd_items_kernel(int2* __restrict__ items, int nk) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int n = 0;
-  for (int blk = 0; blk < nk; ++blk)
-    for (int li = 0; li < 4; ++li)
-      if ((blk & ((1 << li) - 1)) == 0) items[n++] = make_int2(li, blk >> li);
 }
 
 // dK[j] = scale * sum_l dKp_l[j / l] / l, dV[j] = sum_l dVp_l[j / l] / l; the replicate-padded positions [seq, s_pad)
-// hand their share to token seq - 1.  One thread per (head, token, 4 channels).
+// hand their share to token seq - 1.  HBM-bound (3.75 N fp32 sums read, 2 N elements written).  blockIdx.y: dK or dV.
+// Blocks below n_main: one thread per 8 tokens (one row of level 8) and 4 channels, so that every pooled row is read once
+// and all 15 loads are in flight together.  The blocks behind them take the last token of one head each when the sequence
+// is padded: up to 128 positions, dealt to all threads (one thread walking them took 140 us of a 5003-token step).
+// 32 heads x 32768 x 128: 458 -> 359 us (7 TB/s); 28 x 5003: 185 -> 57 us.
+template <typename T>
+__device__ __forceinline__ void store4(T* dst, const float4& v, float scale) {
+  T e[4] = {Elem<T>::from_f(v.x * scale), Elem<T>::from_f(v.y * scale), Elem<T>::from_f(v.z * scale), Elem<T>::from_f(v.w * scale)};
+  *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(e);
+}
+
+__device__ __forceinline__ void fma4(float4& s, const float4& a, float w) {
+  s.x = fmaf(a.x, w, s.x); s.y = fmaf(a.y, w, s.y); s.z = fmaf(a.z, w, s.z); s.w = fmaf(a.w, w, s.w);
+}
+
 template <typename T, int D>
-__global__ void __launch_bounds__(256) bwd_fold_kernel(BwdParams p, T* __restrict__ dk, T* __restrict__ dv) {
+__global__ void __launch_bounds__(256) bwd_fold_kernel(BwdParams p, T* __restrict__ dk, T* __restrict__ dv, int n_main) {
   constexpr int CH = D / 4;
-  const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= p.bh * p.seq * CH) return;
-  const int c = (int)(w % CH) * 4;
-  const int64_t tok = (w / CH) % p.seq, bh = w / ((int64_t)CH * p.seq);
-  float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f), v4 = k4;
-  auto add = [&](int64_t j) {
-#pragma unroll
-    for (int li = 0; li < 4; ++li) {
-      const int64_t n_l = p.s_pad >> li;
-      const float w_l = 1.0f / (float)(1 << li);
-      const float4 a = *reinterpret_cast<const float4*>(p.dkp[li] + (bh * n_l + (j >> li)) * D + c);
-      const float4 b = *reinterpret_cast<const float4*>(p.dvp[li] + (bh * n_l + (j >> li)) * D + c);
-      k4.x = fmaf(a.x, w_l, k4.x); k4.y = fmaf(a.y, w_l, k4.y); k4.z = fmaf(a.z, w_l, k4.z); k4.w = fmaf(a.w, w_l, k4.w);
-      v4.x = fmaf(b.x, w_l, v4.x); v4.y = fmaf(b.y, w_l, v4.y); v4.z = fmaf(b.z, w_l, v4.z); v4.w = fmaf(b.w, w_l, v4.w);
-    }
+  float* const* src = blockIdx.y ? p.dvp : p.dkp;
+  T* out = blockIdx.y ? dv : dk;
+  const float scale = blockIdx.y ? 1.0f : p.scale;
+  const bool tail = p.s_pad > p.seq;
+  const int c = (int)(threadIdx.x % CH) * 4;
+  auto at = [&](int li, int64_t bh, int64_t row) {
+    return __ldg(reinterpret_cast<const float4*>(src[li] + (bh * (p.s_pad >> li) + row) * D + c));
   };
-  add(tok);
-  if (tok == p.seq - 1)
-    for (int64_t j = p.seq; j < p.s_pad; ++j) add(j);
-  const int64_t dst = (bh * p.seq + tok) * D + c;
-  dk[dst] = Elem<T>::from_f(k4.x * p.scale); dk[dst + 1] = Elem<T>::from_f(k4.y * p.scale);
-  dk[dst + 2] = Elem<T>::from_f(k4.z * p.scale); dk[dst + 3] = Elem<T>::from_f(k4.w * p.scale);
-  dv[dst] = Elem<T>::from_f(v4.x); dv[dst + 1] = Elem<T>::from_f(v4.y);
-  dv[dst + 2] = Elem<T>::from_f(v4.z); dv[dst + 3] = Elem<T>::from_f(v4.w);
+  if ((int)blockIdx.x < n_main) {
+    const int64_t n8 = p.s_pad / 8, g = (int64_t)blockIdx.x * (256 / CH) + threadIdx.x / CH;
+    if (g >= p.bh * n8) return;
+    const int64_t bh = g / n8, j = g - bh * n8;
+    if (j * 8 >= p.seq) return;
+    float4 a1[8], a2[4], a4[2];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a1[i] = at(0, bh, j * 8 + i);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a2[i] = at(1, bh, j * 4 + i);
+    a4[0] = at(2, bh, j * 2); a4[1] = at(2, bh, j * 2 + 1);
+    const float4 a8 = at(3, bh, j);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int64_t tok = j * 8 + i;
+      float4 s = a1[i];
+      fma4(s, a2[i >> 1], 0.5f);
+      fma4(s, a4[i >> 2], 0.25f);
+      fma4(s, a8, 0.125f);
+      if (tok < p.seq && !(tail && tok == p.seq - 1)) store4(out + (bh * p.seq + tok) * D + c, s, scale);
+    }
+    return;
+  }
+  __shared__ float4 part[256];
+  const int64_t bh = (int64_t)blockIdx.x - n_main;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int64_t j = p.seq - 1 + threadIdx.x / CH; j < p.s_pad; j += 256 / CH)
+#pragma unroll
+    for (int li = 0; li < 4; ++li) fma4(s, at(li, bh, j >> li), 1.0f / (float)(1 << li));
+  part[threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.x < CH) {
+    for (int i = 1; i < 256 / CH; ++i) fma4(s, part[i * CH + threadIdx.x], 1.0f);
+    store4(out + (bh * p.seq + p.seq - 1) * D + c, s, scale);
+  }
 }
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -1049,15 +1102,11 @@ int launch_bwd_tc(const void* q, const void* kimg, const void* vimg, const int32
   p.status = status; p.seq = seq; p.s_pad = s_pad; p.bh = bh; p.mq = nk; p.mask_cols = mask_cols; p.causal = causal ? 1 : 0;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   int* counters = reinterpret_cast<int*>(scratch + L.counters);
-  cudaError_t e = cudaMemsetAsync(counters, 0, 256, st);
-  PSA_REQUIRE(e == cudaSuccess, PSA_ERR_CUDA, "psa_legacy_bwd_tcgen05: cudaMemsetAsync failed: %s", cudaGetErrorString(e));
-
-  bwd_stat_kernel<T><<<(unsigned)cdiv64(bh * s_pad, 8), 256, 0, st>>>((const T*)out, (const T*)dout, lse,
-                                                                     reinterpret_cast<float*>(scratch + L.nlse),
-                                                                     reinterpret_cast<float*>(scratch + L.ndelta), bh, seq, s_pad, D);
+  bwd_stat_kernel<T, D><<<(unsigned)cdiv64(bh * s_pad, 256 / (D / 8) * 4), 256, 0, st>>>(
+      (const T*)out, (const T*)dout, lse, reinterpret_cast<float*>(scratch + L.nlse), reinterpret_cast<float*>(scratch + L.ndelta), bh, seq,
+      s_pad, reinterpret_cast<int2*>(scratch + L.items), nk, counters,
+      ((uintptr_t)out & 15) == 0);
   PSA_CHECK_LAUNCH("psa_legacy_bwd_tcgen05(row statistics)");
-  bwd_items_kernel<<<1, 32, 0, st>>>(reinterpret_cast<int2*>(scratch + L.items), nk);
-  PSA_CHECK_LAUNCH("psa_legacy_bwd_tcgen05(work list)");
 
   TmapQD maps;
   int rc = encode_tmap_3d(&maps.q, q, 2, FMT == 1, D, seq, bh, 128);
@@ -1069,7 +1118,7 @@ int launch_bwd_tc(const void* q, const void* kimg, const void* vimg, const int32
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   PSA_REQUIRE(sms > 0, PSA_ERR_CUDA, "psa_legacy_bwd_tcgen05: cannot read the SM count");
   {
-    e = cudaFuncSetAttribute(bwd_dq_tc_kernel<D, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    cudaError_t e = cudaFuncSetAttribute(bwd_dq_tc_kernel<D, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
     PSA_REQUIRE(e == cudaSuccess, PSA_ERR_CUDA, "psa_legacy_bwd_tcgen05: shared-memory opt-in (%d B) failed: %s", kSmem, cudaGetErrorString(e));
     const int64_t rows = (int64_t)nk * bh;
     p.counter = counters;
@@ -1077,15 +1126,15 @@ int launch_bwd_tc(const void* q, const void* kimg, const void* vimg, const int32
     PSA_CHECK_LAUNCH("psa_legacy_bwd_tcgen05(dq)");
   }
   {
-    e = cudaFuncSetAttribute(bwd_dkdv_tc_kernel<D, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    cudaError_t e = cudaFuncSetAttribute(bwd_dkdv_tc_kernel<D, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
     PSA_REQUIRE(e == cudaSuccess, PSA_ERR_CUDA, "psa_legacy_bwd_tcgen05: shared-memory opt-in (%d B) failed: %s", kSmem, cudaGetErrorString(e));
     const int64_t jobs = (int64_t)n_entries * bh;
     p.counter = counters + 16;
     bwd_dkdv_tc_kernel<D, FMT><<<(unsigned)(jobs < sms ? jobs : sms), kThreadsBwd, kSmem, st>>>(maps, p);
     PSA_CHECK_LAUNCH("psa_legacy_bwd_tcgen05(dk, dv)");
   }
-  const int64_t work = bh * seq * (D / 4);
-  bwd_fold_kernel<T, D><<<(unsigned)cdiv64(work, 256), 256, 0, st>>>(p, (T*)dk, (T*)dv);
+  const int64_t n_main = cdiv64(bh * (s_pad / 8), 256 / (D / 4));
+  bwd_fold_kernel<T, D><<<dim3((unsigned)(n_main + (s_pad > seq ? bh : 0)), 2), 256, 0, st>>>(p, (T*)dk, (T*)dv, (int)n_main);
   PSA_CHECK_LAUNCH("psa_legacy_bwd_tcgen05(fold)");
   return PSA_OK;
 }
