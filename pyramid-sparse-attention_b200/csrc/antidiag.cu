@@ -6,8 +6,8 @@
 // channels of a group row is 128 contiguous bytes of one token of q or k.  Then a row softmax (causal: groups j <= i)
 // and the sum of the probabilities over (block/stride x block/stride) cells give the mass per (query block, key block).
 //
-// Lengths that are a multiple of the stride take the tcgen05 route (antidiag_tc.cu: GEMM with a partial softmax in its
-// epilogue + a combine kernel, no logits in HBM).  Other lengths run the two kernels of this file:
+// Lengths of at least one group take the tcgen05 route (antidiag_tc.cu: GEMM with a partial softmax in its epilogue + a
+// combine kernel, no logits in HBM).  Shorter ones, and calls that ask for it, run the two kernels of this file:
 // Kernel 1, warp-level mma.sync: 128x128 logit
 // tiles, 8 warps of 32x64, K streamed in chunks of 64 through registers into padded shared-memory tiles; it writes the
 // logits as fp32, already multiplied by log2(e)/sqrt(D)/stride, and skips the tiles above the diagonal when causal.
@@ -248,7 +248,7 @@ extern "C" int psa_antidiag_scores_impl(const void* q, const void* k, void* out,
   const size_t smem = (size_t)8 * (d.n / d.rb) * sizeof(float);
   dim3 grid2((unsigned)d.nb, (unsigned)bh);
   const bool tc_ok = antidiag_tc_supported(seq, head_dim, stride, d.n, dtype);
-  PSA_REQUIRE(impl != 2 || tc_ok, PSA_ERR_UNSUPPORTED,
+  PSA_REQUIRE(impl != 2 || (tc_ok && seq % stride == 0), PSA_ERR_UNSUPPORTED,
               "psa_antidiag_scores: the tcgen05 kernel needs a length that is a multiple of the stride (seq=%lld, stride=%d)",
               (long long)seq, stride);
   const bool use_tc = tc_ok && impl != 3;

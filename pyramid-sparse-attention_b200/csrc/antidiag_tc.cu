@@ -1,5 +1,5 @@
-// Antidiagonal block-importance estimate of the causal call site on tcgen05 tensor cores (f16/bf16, lengths that are a
-// multiple of the stride).  Replaces flat_group_gemm_fuse_reshape and softmax_fuse_block_sum
+// Antidiagonal block-importance estimate of the causal call site on tcgen05 tensor cores (f16/bf16, at least one whole
+// group of tokens).  Replaces flat_group_gemm_fuse_reshape and softmax_fuse_block_sum
 // (qwen2.5-vl-example/src/attention/PSA_casual/kernels/block_importance_kernels.py:255-323, 6-192); the fp32 logits
 // never reach HBM.
 //
@@ -7,7 +7,10 @@
 // Neither matrix is materialised: q and k are described to TMA as 4-D tensors {channel, token in group, group,
 // batch*head}, so a K-chunk (64 channels of token s of every group) of 128 consecutive groups is ONE box
 // {64, 1, 128, 1}, landing in shared memory as a 128-byte-swizzled [128 rows][128 B] operand tile; the query side
-// simply asks for token stride-1-s.  Groups past the end are zero-filled by TMA.
+// simply asks for token stride-1-s.  Groups past the end are zero-filled by TMA.  A length that is no multiple of the stride
+// has one group more for its first seq mod stride token positions than for the others, so those positions go through a
+// second pair of maps with one group more: every token is in bounds, every missing one is zero.  (Such lengths ran on the
+// mma.sync kernel with the logits in HBM; prompts hardly ever come in whole groups.)
 //
 // Persistent CTAs (one per SM) walk the 128x128 logit tiles (tiles above the diagonal are skipped when causal):
 //   warp 0   producer: per K-chunk two boxes (A, B) into a 4-stage ring (32 KB per stage)
@@ -49,6 +52,7 @@ struct Params {
   int row_tiles;       // tiles that hold a valid query group
   int col_tiles;       // non-causal: tiles per row
   int stride;
+  int tail;            // token positions of a group that have one group more (seq mod stride)
   int causal;
   int64_t bh;
   float scale_log2;
@@ -69,6 +73,11 @@ __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 
+// [0]: token positions with one group for every whole group of the sequence, [1]: those with one more
+struct GroupMaps {
+  CUtensorMap q[2], k[2];
+};
+
 // tile number t of one head -> (row tile, column tile); causal heads enumerate the lower triangle row by row
 __device__ __forceinline__ void tile_of(int t, const Params& p, int& it, int& jt) {
   if (!p.causal) {
@@ -84,8 +93,7 @@ __device__ __forceinline__ void tile_of(int t, const Params& p, int& it, int& jt
 }
 
 template <int D, int FMT>
-__global__ void __launch_bounds__(kThreads, 1) antidiag_logits_tc_kernel(const __grid_constant__ CUtensorMap tm_q,
-                                                                        const __grid_constant__ CUtensorMap tm_k, const Params p) {
+__global__ void __launch_bounds__(kThreads, 1) antidiag_logits_tc_kernel(const __grid_constant__ GroupMaps maps, const Params p) {
   constexpr int SLABS = D / 64;
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
@@ -127,8 +135,9 @@ __global__ void __launch_bounds__(kThreads, 1) antidiag_logits_tc_kernel(const _
           if (!ok) break;
           const int s = kc / SLABS, d0 = (kc - s * SLABS) * 64;
           unsigned char* dst = smem + stage * kStageBytes;
-          tma_load_4d(dst, &tm_q, &ctl->full[stage], d0, p.stride - 1 - s, it * 128, bh);
-          tma_load_4d(dst + kOperandBytes, &tm_k, &ctl->full[stage], d0, s, jt * 128, bh);
+          const int sq = p.stride - 1 - s;
+          tma_load_4d(dst, &maps.q[sq < p.tail], &ctl->full[stage], d0, sq, it * 128, bh);
+          tma_load_4d(dst + kOperandBytes, &maps.k[s < p.tail], &ctl->full[stage], d0, s, jt * 128, bh);
           tc::mbar_arrive_expect_tx(&ctl->full[stage], kStageBytes);
         }
       }
@@ -292,8 +301,9 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// {channel, token in group, group, batch*head} over a [bh][seq][D] tensor whose length is a multiple of the stride
-int encode_groups_4d(CUtensorMap* map, const void* base, int is_bf16, int D, int stride, int64_t seq, int64_t bh) {
+// {channel, token in group, group, batch*head} over a [bh][seq][D] tensor: the first `positions` tokens of `groups` groups
+int encode_groups_4d(CUtensorMap* map, const void* base, int is_bf16, int D, int stride, int positions, int64_t groups, int64_t seq,
+                     int64_t bh) {
   static EncodeTiledFn fn = nullptr;
   if (!fn) {
     void* ptr = nullptr;
@@ -303,7 +313,7 @@ int encode_groups_4d(CUtensorMap* map, const void* base, int is_bf16, int D, int
       fn = (EncodeTiledFn)ptr;
   }
   PSA_REQUIRE(fn != nullptr, PSA_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-  cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)stride, (cuuint64_t)(seq / stride), (cuuint64_t)bh};
+  cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)positions, (cuuint64_t)groups, (cuuint64_t)bh};
   cuuint64_t strides[3] = {(cuuint64_t)D * 2, (cuuint64_t)stride * D * 2, (cuuint64_t)seq * D * 2};
   cuuint32_t box[4] = {64, 1, 128, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
@@ -317,12 +327,17 @@ int encode_groups_4d(CUtensorMap* map, const void* base, int is_bf16, int D, int
 template <int D, int FMT>
 int launch(const void* q, const void* k, void* out, float* scratch, int64_t bh, int64_t seq, int stride, int n, int n_valid, int rb,
            int nb, int causal, float scale_log2, int32_t* status, cudaStream_t st) {
-  CUtensorMap tq, tk;
-  int rc = encode_groups_4d(&tq, q, FMT, D, stride, seq, bh);
-  if (rc != PSA_OK) return rc;
-  rc = encode_groups_4d(&tk, k, FMT, D, stride, seq, bh);
-  if (rc != PSA_OK) return rc;
+  GroupMaps maps;
+  const int tail = (int)(seq % stride);
+  for (int i = 0; i < 2; ++i) {
+    if (i == 1 && tail == 0) { maps.q[1] = maps.q[0]; maps.k[1] = maps.k[0]; break; }
+    int rc = encode_groups_4d(&maps.q[i], q, FMT, D, stride, i ? tail : stride, seq / stride + i, seq, bh);
+    if (rc != PSA_OK) return rc;
+    rc = encode_groups_4d(&maps.k[i], k, FMT, D, stride, i ? tail : stride, seq / stride + i, seq, bh);
+    if (rc != PSA_OK) return rc;
+  }
   Params p;
+  p.tail = tail;
   p.tile_max = scratch;
   p.block_sum = scratch + (size_t)bh * n * ((n + 127) / 128);
   p.n = n; p.n_valid = n_valid; p.rb = rb; p.stride = stride; p.causal = causal; p.bh = bh; p.scale_log2 = scale_log2; p.status = status;
@@ -337,7 +352,7 @@ int launch(const void* q, const void* k, void* out, float* scratch, int64_t bh, 
   if (sms <= 0) sms = 148;
   const int64_t tiles = bh * (causal ? (int64_t)p.row_tiles * (p.row_tiles + 1) / 2 : (int64_t)p.row_tiles * p.col_tiles);
   const unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
-  antidiag_logits_tc_kernel<D, FMT><<<grid, kThreads, smem, st>>>(tq, tk, p);
+  antidiag_logits_tc_kernel<D, FMT><<<grid, kThreads, smem, st>>>(maps, p);
   PSA_CHECK_LAUNCH("psa_antidiag_scores(tcgen05 logits)");
   dim3 grid2((unsigned)nb, (unsigned)bh);
   antidiag_combine_kernel<FMT><<<grid2, 256, (size_t)8 * (n / rb) * sizeof(float), st>>>(p.tile_max, p.block_sum, (uint16_t*)out, n, n_valid,
@@ -350,8 +365,7 @@ int launch(const void* q, const void* k, void* out, float* scratch, int64_t bh, 
 
 bool antidiag_tc_supported(int64_t seq, int head_dim, int stride, int n, int dtype) {
   (void)n;
-  return (dtype == PSA_F16 || dtype == PSA_BF16) && (head_dim == 64 || head_dim == 128) && stride >= 1 && seq % stride == 0 &&
-         seq / stride >= 1;
+  return (dtype == PSA_F16 || dtype == PSA_BF16) && (head_dim == 64 || head_dim == 128) && stride >= 1 && seq >= stride;
 }
 
 // Whole estimate: out [bh][nb][nb] in the element type.  scratch: bh * n * ceil(n/128) * (1 + 128/rb) floats (at most
