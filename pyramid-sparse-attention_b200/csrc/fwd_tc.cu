@@ -1113,7 +1113,8 @@ bool fwd_tc_supported(const FwdArgs& a) {
 constexpr int kCounterRing = 256;
 __device__ int g_row_counters[kCounterRing];
 
-static int next_row_counter(int** out, cudaStream_t st) {
+// n (1 to 3) neighbouring words, zeroed by one memset.
+static int next_counters(int n, int** out, cudaStream_t st) {
   constexpr int kMaxDevices = 64;
   static int* base[kMaxDevices] = {nullptr};
   static unsigned next[kMaxDevices] = {0};
@@ -1128,15 +1129,18 @@ static int next_row_counter(int** out, cudaStream_t st) {
     PSA_REQUIRE(e == cudaSuccess && ptr, PSA_ERR_CUDA, "psa_fwd: cudaGetSymbolAddress failed: %s", cudaGetErrorString(e));
     base[dev] = (int*)ptr;
   }
-  int* c = base[dev] + (next[dev]++ % kCounterRing);
-  e = cudaMemsetAsync(c, 0, sizeof(int), st);
+  unsigned pos = next[dev] % kCounterRing;
+  if (pos + n > kCounterRing) pos = 0;      // the words of one call do not wrap around
+  next[dev] = pos + n;
+  int* c = base[dev] + pos;
+  e = cudaMemsetAsync(c, 0, n * sizeof(int), st);
   PSA_REQUIRE(e == cudaSuccess, PSA_ERR_CUDA, "psa_fwd: cudaMemsetAsync failed: %s", cudaGetErrorString(e));
   *out = c;
   return PSA_OK;
 }
 
-template <int D, int FMT, bool IMG, bool CAUSAL = false, bool FIXED = false>
-static int launch_tc(const FwdArgs& a, cudaStream_t st, int* guard = nullptr, const int* only_if = nullptr) {
+template <int D, int FMT, bool IMG, bool CAUSAL, bool FIXED>
+static int launch_tc(const FwdArgs& a, cudaStream_t st, int* row_counter, int* guard = nullptr, const int* only_if = nullptr) {
   using C = Cfg<D, FIXED>;
   TmapPack maps;
   const int is_bf16 = FMT == 1;
@@ -1170,8 +1174,7 @@ static int launch_tc(const FwdArgs& a, cudaStream_t st, int* guard = nullptr, co
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   PSA_REQUIRE(sms > 0, PSA_ERR_CUDA, "psa_fwd: cannot read the SM count");
   const unsigned grid = (unsigned)(p.total_rows < sms ? p.total_rows : sms);
-  rc = next_row_counter(&p.row_counter, st);
-  if (rc != PSA_OK) return rc;
+  p.row_counter = row_counter;
   psa_fwd_tc_kernel<D, FMT, IMG, CAUSAL, FIXED><<<grid, kThreads, C::SMEM_BYTES, st>>>(maps, p);
   PSA_CHECK_LAUNCH("psa_fwd(tcgen05)");
   return PSA_OK;
@@ -1182,12 +1185,19 @@ static int launch_tc(const FwdArgs& a, cudaStream_t st, int* guard = nullptr, co
 template <int D, int FMT, bool IMG, bool CAUSAL>
 static int launch_fixed_then_exact(const FwdArgs& a, cudaStream_t st) {
   static_assert(FMT == 1, "bf16 only");
-  int* guard = nullptr;
-  int rc = next_row_counter(&guard, st);      // a zeroed device word of this launch
+  int* words = nullptr;                       // row counters of both kernels and the guard word
+  int rc = next_counters(3, &words, st);
   if (rc != PSA_OK) return rc;
-  rc = launch_tc<D, FMT, IMG, CAUSAL, true>(a, st, guard, nullptr);
+  rc = launch_tc<D, FMT, IMG, CAUSAL, true>(a, st, words, words + 2, nullptr);
   if (rc != PSA_OK) return rc;
-  return launch_tc<D, FMT, IMG, CAUSAL, false>(a, st, nullptr, guard);
+  return launch_tc<D, FMT, IMG, CAUSAL, false>(a, st, words + 1, nullptr, words + 2);
+}
+
+template <int D, int FMT, bool IMG, bool CAUSAL>
+static int launch_exact(const FwdArgs& a, cudaStream_t st) {
+  int* words = nullptr;
+  const int rc = next_counters(1, &words, st);
+  return rc != PSA_OK ? rc : launch_tc<D, FMT, IMG, CAUSAL, false>(a, st, words);
 }
 
 int fwd_tc_launch(const FwdArgs& a, cudaStream_t st) {
@@ -1197,15 +1207,15 @@ int fwd_tc_launch(const FwdArgs& a, cudaStream_t st) {
     PSA_REQUIRE(a.bn >= 64, PSA_ERR_UNSUPPORTED, "tile images need block_n >= 64 (blocks of at least 8 pooled rows)");
     PSA_REQUIRE((((uintptr_t)a.kimg | (uintptr_t)a.vimg) & 15) == 0, PSA_ERR_ARG, "tile images must be 16-byte aligned");
     if (a.causal) {   // only the legacy forward asks for it; a variant of its own keeps the common kernel lean
-      if (a.D == 64) return fmt ? launch_fixed_then_exact<64, 1, true, true>(a, st) : launch_tc<64, 0, true, true>(a, st);
-      return fmt ? launch_fixed_then_exact<128, 1, true, true>(a, st) : launch_tc<128, 0, true, true>(a, st);
+      if (a.D == 64) return fmt ? launch_fixed_then_exact<64, 1, true, true>(a, st) : launch_exact<64, 0, true, true>(a, st);
+      return fmt ? launch_fixed_then_exact<128, 1, true, true>(a, st) : launch_exact<128, 0, true, true>(a, st);
     }
-    if (a.D == 64) return fmt ? launch_fixed_then_exact<64, 1, true, false>(a, st) : launch_tc<64, 0, true, false>(a, st);
-    return fmt ? launch_fixed_then_exact<128, 1, true, false>(a, st) : launch_tc<128, 0, true, false>(a, st);
+    if (a.D == 64) return fmt ? launch_fixed_then_exact<64, 1, true, false>(a, st) : launch_exact<64, 0, true, false>(a, st);
+    return fmt ? launch_fixed_then_exact<128, 1, true, false>(a, st) : launch_exact<128, 0, true, false>(a, st);
   }
   PSA_REQUIRE(!a.causal, PSA_ERR_UNSUPPORTED, "the causal rule needs the tile-image path");
-  if (a.D == 64) return fmt ? launch_fixed_then_exact<64, 1, false, false>(a, st) : launch_tc<64, 0, false, false>(a, st);
-  return fmt ? launch_fixed_then_exact<128, 1, false, false>(a, st) : launch_tc<128, 0, false, false>(a, st);
+  if (a.D == 64) return fmt ? launch_fixed_then_exact<64, 1, false, false>(a, st) : launch_exact<64, 0, false, false>(a, st);
+  return fmt ? launch_fixed_then_exact<128, 1, false, false>(a, st) : launch_exact<128, 0, false, false>(a, st);
 }
 
 }  // namespace psa

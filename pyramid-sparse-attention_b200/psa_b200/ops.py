@@ -1,7 +1,9 @@
 """Tensor-level wrappers around the C-ABI kernels.  torch is used for device memory and streams only."""
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
+import functools
 import math
 from typing import Dict, List, Optional, Sequence, Tuple
 
@@ -21,12 +23,20 @@ def _need_cuda(*ts):
             raise RuntimeError("psa_b200 kernels need CUDA tensors; there is no CPU path in this package")
 
 
-def _stream(t: torch.Tensor):
-    return C.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+def _stream(t: torch.Tensor) -> int:
+    return torch._C._cuda_getCurrentRawStream(t.device.index)     # no Stream object per call
 
 
-def _ptr(t: Optional[torch.Tensor]):
-    return C.c_void_p(0 if t is None else t.data_ptr())
+def _ptr(t: Optional[torch.Tensor]) -> int:
+    return 0 if t is None else t.data_ptr()
+
+
+_HERE = contextlib.nullcontext()
+
+
+def _on(t: torch.Tensor):
+    """Context in which t's device is the current one (entering torch.cuda.device costs 7 us even where it already is)."""
+    return _HERE if t.device.index == torch._C._cuda_getDevice() else torch.cuda.device(t.device)
 
 
 def _dt(t: torch.Tensor) -> int:
@@ -81,7 +91,7 @@ def pyramid_kv(k: torch.Tensor, v: torch.Tensor, block_n: int):
     k, v = _flat_bh(k), _flat_bh(v)
     B, H, S, D = k.shape
     s_pad = -(-S // block_n) * block_n
-    with torch.cuda.device(k.device):
+    with _on(k):
         outs = [torch.empty((B, H, s_pad // l, D), dtype=k.dtype, device=k.device) for l in (2, 4, 8) for _ in (0, 1)]
         k2, v2, k4, v4, k8, v8 = outs
         rc = lib.psa_pyramid_kv(_ptr(k), _ptr(v), _ptr(k2), _ptr(k4), _ptr(k8), _ptr(v2), _ptr(v4), _ptr(v8),
@@ -116,7 +126,7 @@ def gather_rows(x: torch.Tensor, perm: Optional[torch.Tensor], rope=None) -> tor
     x = _flat_bh(x)
     B, H, S, D = x.shape
     perm = None if perm is None else _perm32(perm, S)
-    with torch.cuda.device(x.device):
+    with _on(x):
         out = torch.empty_like(x)
         if rope is None:
             rc = lib.psa_gather_rows(_ptr(x), _ptr(perm), _ptr(out), B * H, S, D, x.element_size(), _stream(x))
@@ -139,7 +149,7 @@ def pyramid_kv_images(k: torch.Tensor, v: torch.Tensor, block_n: int, perm: Opti
     nbytes = lib.psa_kv_image_bytes(B * H, S, D, block_n)
     if nbytes == 0:
         raise ValueError(f"tile images need head_dim 64/128 and block_n 64/128 (got {D}, {block_n})")
-    with torch.cuda.device(k.device):
+    with _on(k):
         kimg = torch.empty(nbytes, dtype=torch.uint8, device=k.device)
         vimg = torch.empty(nbytes, dtype=torch.uint8, device=k.device)
         if rope is not None:
@@ -223,7 +233,7 @@ def gather_views(q, k, v, perm: Optional[torch.Tensor] = None, rope: Optional[Ro
     # rows the kernel cannot address word by word are laid out first
     views = [x if x.stride(3) == 1 and all(s % 8 == 0 for s in x.stride()[:3]) and x.data_ptr() % 16 == 0
              else x.clone(memory_format=torch.contiguous_format) for x in (q, k, v)]
-    with torch.cuda.device(q.device):
+    with _on(q):
         outs = [torch.empty((B, H, S, D), dtype=q.dtype, device=q.device) for _ in range(3)]
         rc = lib.psa_gather_views((C.c_void_p * 3)(*[x.data_ptr() for x in views]),
                                   (C.c_int64 * 9)(*[s for x in views for s in x.stride()[:3]]), (C.c_int32 * 3)(*([int(rope is not None)] * 2), 0),
@@ -238,7 +248,7 @@ def gather_heads(x: torch.Tensor, perm: Optional[torch.Tensor] = None, rope: Opt
     way if rope is given."""
     S, H, D = _tm_check(x)
     perm = None if perm is None else _perm32(perm, S)
-    with torch.cuda.device(x.device):
+    with _on(x):
         out = torch.empty((1, H, S, D), dtype=x.dtype, device=x.device)
         if rope is None:
             rc = lib.psa_gather_heads(_ptr(x), _ptr(perm), _ptr(out), H, S, D, x.element_size(), _stream(x))
@@ -259,7 +269,7 @@ def pyramid_kv_images_tm(k: torch.Tensor, v: torch.Tensor, block_n: int, perm: O
     nbytes = lib.psa_kv_image_bytes(H, S, D, block_n)
     if nbytes == 0:
         raise ValueError(f"tile images need head_dim 64/128 and block_n 64/128 (got {D}, {block_n})")
-    with torch.cuda.device(k.device):
+    with _on(k):
         kimg = torch.empty(nbytes, dtype=torch.uint8, device=k.device)
         vimg = torch.empty(nbytes, dtype=torch.uint8, device=k.device)
         if rope is None:
@@ -284,7 +294,7 @@ def block_scores_tm(q, k, idx_q, idx_k, block_m: int, block_n: int, perm: Option
     iq = idx_q.to(torch.int32).contiguous()
     ik = idx_k.to(torch.int32).contiguous()
     Mq, Nk = -(-S // block_m), -(-S // block_n)
-    with torch.cuda.device(q.device):
+    with _on(q):
         po = torch.empty((1, H, Mq, Nk), dtype=q.dtype, device=q.device)
         nbytes = lib.psa_block_scores_scratch_bytes(H, S, S, block_m, block_n, _dt(q))
         if nbytes == 0:
@@ -313,7 +323,7 @@ def psa_forward_tm(q_heads, images: KVImages, mask, out_tm, block_m: int, block_
     out_perm = None if out_perm is None else _perm32(out_perm, S)
     if sm_scale is None:
         sm_scale = D ** -0.5
-    with torch.cuda.device(q_heads.device):
+    with _on(q_heads):
         status = status_word(q_heads.device)
         rc = lib.psa_fwd_images_tm(_ptr(q_heads), _ptr(images.kimg), _ptr(images.vimg), _ptr(mask), _ptr(out_tm), _ptr(out_perm),
                                    H, S, D, block_m, block_n, tile_n, mask.shape[-1], float(sm_scale), int(compat_quirk),
@@ -343,7 +353,7 @@ def block_scores(q, k, idx_q, idx_k, block_m: int, block_n: int, impl: int = IMP
     iq = idx_q.to(torch.int32).contiguous()
     ik = idx_k.to(torch.int32).contiguous()
     Mq, Nk = -(-Sq // block_m), -(-Sk // block_n)
-    with torch.cuda.device(q.device):
+    with _on(q):
         po = torch.empty((B, H, Mq, Nk), dtype=q.dtype, device=q.device)
         nbytes = lib.psa_block_scores_scratch_bytes(B * H, Sq, Sk, block_m, block_n, _dt(q))
         if nbytes == 0:
@@ -406,6 +416,30 @@ def _round_to_dtype(x: float, dtype: torch.dtype) -> float:
     return float(torch.tensor(x, dtype=torch.float64).to(dtype).to(torch.float64))
 
 
+@functools.lru_cache(maxsize=128)
+def _level_plan(items, nk: int, threshold: bool, newtype: bool, block_n: int, tile_n: int, dtype: torch.dtype, min_full_attn_ratio: float):
+    """What psa_assign_levels is told about the levels: their values, rank intervals or thresholds, alignments and the first
+    rank that need not be level 1.  A function of plain numbers only, kept by their values: every layer of a model asks for
+    the same one (in the cumulative-mass mode it costs 15 tensor operations)."""
+    n = len(items)
+    I32 = C.c_int32 * n
+    F32 = C.c_float * n
+    if threshold:
+        items = sorted(items, key=lambda x: x[2])
+        levels = I32(*[int(l) for l, _, _ in items])
+        thr = F32(*[_round_to_dtype(end + 1e-6, dtype) for _, _, end in items])
+        aligns = I32(*[_align_multiple(int(l), block_n, tile_n, False) for l, _, _ in items])
+        return levels, None, None, thr, aligns, min(nk, int(nk * min_full_attn_ratio) + 1)
+    iv = topk_intervals(nk, {l: (start, end) for l, start, end in items}, block_n, tile_n, newtype)
+    return I32(*[int(l) for l, _, _ in iv]), I32(*[s for _, s, _ in iv]), I32(*[e for _, _, e in iv]), None, None, 0
+
+
+def _plan_of(mask_ratios, nk, threshold, newtype, block_n, tile_n, dtype, min_full_attn_ratio=0.06):
+    items = tuple((l, *r) for l, r in mask_ratios.items())
+    plain = all(len(x) == 3 and all(type(e) in (int, float) for e in x) for x in items) and type(min_full_attn_ratio) is float
+    return (_level_plan if plain else _level_plan.__wrapped__)(items, nk, threshold, newtype, block_n, tile_n, dtype, min_full_attn_ratio)
+
+
 def assign_levels(po: torch.Tensor, mask_ratios: Dict[int, Tuple[float, float]], mode: str, block_n: int,
                   tile_n: int, text_length: int = 0, min_full_attn_ratio: float = 0.06) -> torch.Tensor:
     """Score rows -> level mask.  Same modes, argument meaning and errors as transfer_attn_to_mask
@@ -422,25 +456,10 @@ def assign_levels(po: torch.Tensor, mask_ratios: Dict[int, Tuple[float, float]],
     n = len(mask_ratios)
     if n > 8:
         raise ValueError("at most 8 levels")
-    I32 = C.c_int32 * n
-    F32 = C.c_float * n
-    if threshold:
-        items = sorted(mask_ratios.items(), key=lambda x: x[1][1])
-        levels = I32(*[int(l) for l, _ in items])
-        thr = F32(*[_round_to_dtype(r[1] + 1e-6, po.dtype) for _, r in items])
-        aligns = I32(*[_align_multiple(int(l), block_n, tile_n, False) for l, _ in items])
-        starts = ends = None
-        min_index = min(Nk, int(Nk * min_full_attn_ratio) + 1)
-    else:
-        iv = topk_intervals(Nk, mask_ratios, block_n, tile_n, newtype)
-        levels = I32(*[int(l) for l, _, _ in iv])
-        starts = I32(*[s for _, s, _ in iv])
-        ends = I32(*[e for _, _, e in iv])
-        thr = aligns = None
-        min_index = 0
+    levels, starts, ends, thr, aligns, min_index = _plan_of(mask_ratios, Nk, threshold, newtype, block_n, tile_n, po.dtype, min_full_attn_ratio)
     text_blocks = 0 if (newtype or text_length == 0) else (text_length + block_n - 1) // block_n
     width = Nk + n if newtype else Nk
-    with torch.cuda.device(po.device):
+    with _on(po):
         mask = torch.empty((B, H, Mq, width), dtype=torch.int32, device=po.device)
         rc = lib.psa_assign_levels(_ptr(po), _ptr(mask), B * H * Mq, Nk, _dt(po), int(threshold), int(newtype), n,
                                    levels, starts, ends, thr, aligns, min_index, text_blocks, _stream(po))
@@ -462,7 +481,7 @@ def antidiag_block_scores(q, k, block_size: int, stride: int, chunk_size: int, c
         raise ValueError(f"antidiagonal estimate: unsupported sizes (head_dim {D}, block {block_size}, stride {stride}, "
                          f"chunk {chunk_size})")
     nb = -(-L // block_size)
-    with torch.cuda.device(q.device):
+    with _on(q):
         out = torch.empty((B, H, nb, nb), dtype=q.dtype, device=q.device)
         scratch = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
         status = status_word(q.device)
@@ -503,7 +522,7 @@ def assign_levels_causal(attn: torch.Tensor, mask_ratios: Dict[int, Tuple[float,
         lo = F32(*[_round_to_dtype(x, attn.dtype) for x in lows])
         hi = F32(*[_round_to_dtype(r[1], attn.dtype) for _, r in items])
     special = min((text_length + block_size - 1) // block_size if text_length > 0 else 0, n)
-    with torch.cuda.device(attn.device):
+    with _on(attn):
         mask = torch.empty((B, H, n, n), dtype=torch.int32, device=attn.device)
         rc = lib.psa_assign_levels_causal(_ptr(attn), _ptr(mask), B * H, n, _dt(attn), int(mode == "energybound"), int(causal),
                                           nl, levels, rs, re, lo, hi, special, _stream(attn))
@@ -517,7 +536,7 @@ def density(mask: torch.Tensor, newtype: bool) -> torch.Tensor:
     _need_cuda(mask)
     mask = _flat_bh(mask)
     B, H, Mq, W = mask.shape
-    with torch.cuda.device(mask.device):
+    with _on(mask):
         out = torch.empty((B, H), dtype=torch.float32, device=mask.device)
         rc = lib.psa_density(_ptr(mask), _ptr(out), B * H, Mq, W, int(newtype), _stream(mask))
     check(rc, "psa_density")
@@ -532,7 +551,7 @@ def k_similarity(k: torch.Tensor, block_n: int, t2: float, t4: float, t8: float,
     k = _flat_bh(k)
     B, H, S, D = k.shape
     assert block_n % 8 == 0, "blocksize must be divisible by 8"
-    with torch.cuda.device(k.device):
+    with _on(k):
         out = torch.empty((B, H, -(-S // block_n)), dtype=torch.int32, device=k.device)
         if perm is None:
             rc = lib.psa_ksim(_ptr(k), _ptr(out), B * H, S, D, block_n, t2, t4, t8, _dt(k), _stream(k))
@@ -563,7 +582,7 @@ def psa_forward(q, k, v, mask, block_m: int, block_n: int, tile_n: int, sm_scale
     if use_images:
         if pyramid is None:
             pyramid = pyramid_kv_images(k, v, block_n)
-        with torch.cuda.device(q.device):
+        with _on(q):
             o = out if out is not None else torch.empty_like(q)
             status = status_word(q.device)
             if out_perm is None:
@@ -583,7 +602,7 @@ def psa_forward(q, k, v, mask, block_m: int, block_n: int, tile_n: int, sm_scale
     if pyramid is None:
         pyramid = pyramid_kv(k, v, block_n)
     (k2, k4, k8), (v2, v4, v8) = pyramid
-    with torch.cuda.device(q.device):
+    with _on(q):
         o = out if out is not None else torch.empty_like(q)
         status = status_word(q.device)
         rc = lib.psa_fwd(_ptr(q), _ptr(k), _ptr(v), _ptr(k2), _ptr(k4), _ptr(k8), _ptr(v2), _ptr(v4), _ptr(v8),
@@ -601,7 +620,7 @@ def psa_forward_to_rows(q, k, v, mask, block_m: int, block_n: int, tile_n: int, 
     B, H, S, D = q.shape
     mask, out_perm = _mask32(mask), _perm32(out_perm, S)
     (k2, k4, k8), (v2, v4, v8) = pyramid_kv(k, v, block_n)
-    with torch.cuda.device(q.device):
+    with _on(q):
         o = torch.empty_like(q)
         status = status_word(q.device)
         rc = lib.psa_fwd_perm(_ptr(q), _ptr(k), _ptr(v), _ptr(k2), _ptr(k4), _ptr(k8), _ptr(v2), _ptr(v4), _ptr(v8), _ptr(mask),
@@ -654,7 +673,7 @@ def legacy_forward(q, k, v, mask, causal: bool = False, sm_scale: Optional[float
     if impl != IMPL_SCALAR and _legacy_tc_ok(q, sm_scale):
         # 16-bit tensors: the tcgen05 forward on tile images (which the tcgen05 backward reads again)
         imgs = kv.images()
-        with torch.cuda.device(q.device):
+        with _on(q):
             o = torch.empty_like(q)
             lse = torch.empty((B, H, S), dtype=torch.float32, device=q.device) if need_lse else None
             scratch = torch.empty(lib.psa_legacy_index_bytes(B * H, S) // 4, dtype=torch.int32, device=q.device)
@@ -665,7 +684,7 @@ def legacy_forward(q, k, v, mask, causal: bool = False, sm_scale: Optional[float
         o._psa_status = status
         return o, lse, (kv if need_lse else None)
     (k2, k4, k8), (v2, v4, v8) = kv.rows()
-    with torch.cuda.device(q.device):
+    with _on(q):
         o = torch.empty_like(q)
         lse = torch.empty((B, H, S), dtype=torch.float32, device=q.device) if need_lse else None
         rc = lib.psa_legacy_fwd(_ptr(q), _ptr(k), _ptr(v), _ptr(k2), _ptr(k4), _ptr(k8), _ptr(v2), _ptr(v4), _ptr(v8),
@@ -696,7 +715,7 @@ def legacy_forward_gathered(q_r, imgs: KVImages, mask, perm: torch.Tensor, sm_sc
     B, H, S, D = q_r.shape
     sm_scale = D ** -0.5 if sm_scale is None else sm_scale
     perm = _perm32(perm, S)
-    with torch.cuda.device(q_r.device):
+    with _on(q_r):
         o = torch.empty_like(q_r)
         scratch = torch.empty(lib.psa_legacy_index_bytes(B * H, S) // 4, dtype=torch.int32, device=q_r.device)
         status = status_word(q_r.device)
@@ -728,7 +747,7 @@ def legacy_backward(q, k, v, mask, o, lse, do, causal: bool, sm_scale: float, py
     half = q.dtype in (torch.float16, torch.bfloat16)
     if impl == IMPL_AUTO:
         impl = IMPL_TENSOR if (half and _legacy_tc_ok(q, sm_scale)) else IMPL_SCALAR
-    with torch.cuda.device(q.device):
+    with _on(q):
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         if impl == IMPL_TENSOR:
             if not (half and _legacy_tc_ok(q, sm_scale)):
