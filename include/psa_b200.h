@@ -155,6 +155,17 @@ int psa_fwd_images(const void* q, const void* kimg, const void* vimg, const int3
                    int64_t seq_q, int64_t seq_k, int head_dim, int block_m, int block_n, int tile_n, int mask_width,
                    float sm_scale, int compat_quirk, int dtype, int32_t* status, void* stream);
 
+/* The plug-and-play layer (src/psa_triton/attention.py:276-310, separator-format mask, no similarity cap) in one call: the
+ * kernels of psa_block_scores, psa_assign_levels (newtype), psa_pyramid_kv_images and psa_fwd_images, in that order, on
+ * scratch of psa_layer_scratch_bytes (0: sizes or dtype not covered; f16/bf16, block_n 64/128).  idx_q [bh][block_m/4],
+ * idx_k [bh][block_n/4]: 64-bit sample offsets.  mask: int32 [bh][ceil(seq_q/block_m)][ceil(seq_k/block_n) + n_levels], written. */
+size_t psa_layer_scratch_bytes(int64_t bh, int64_t seq_q, int64_t seq_k, int head_dim, int block_m, int block_n, int dtype);
+int psa_layer(const void* q, const void* k, const void* v, const int64_t* idx_q, const int64_t* idx_k, int32_t* mask, void* out,
+              void* scratch, size_t scratch_bytes, int64_t bh, int64_t seq_q, int64_t seq_k, int head_dim, int block_m,
+              int block_n, int tile_n, int threshold_mode, int n_levels, const int32_t* level_values, const int32_t* starts,
+              const int32_t* ends, const float* thresholds, const int32_t* aligns, int min_index, float sm_scale,
+              int compat_quirk, int dtype, int32_t* status, void* stream);
+
 /* Token reordering folded into the kernels.  Replaces GilbertRearranger.rearrange / rearrange_single / reversed_rearrange,
  * src/psa_triton/utils/rearranger.py:69-132 (three index_select copies of q, k, v before the attention and one of the
  * output after it; the text tokens move from the front of the sequence to its end and back).

@@ -185,7 +185,7 @@ static unsigned pool_threads(int packs) {
 template <typename T>
 static int launch_scores(const RowSource& q, const RowSource& k, const int32_t* idx_q, const int32_t* idx_k, void* po,
                          void* scratch, const ScoreDims& d, int64_t bh, int impl, cudaStream_t st,
-                         const RopeTables& rope = RopeTables{}) {
+                         const RopeTables& rope = RopeTables{}, int idx_step = 1) {
   T* R = (T*)scratch;
   const size_t r_bytes = ((size_t)bh * d.nq_s * d.n_d * sizeof(T) + 255) & ~(size_t)255;
   float* rowmax = (float*)((char*)scratch + r_bytes);
@@ -194,10 +194,10 @@ static int launch_scores(const RowSource& q, const RowSource& k, const int32_t* 
   bool use_tc = (impl == 2) || (impl == 0 && sizeof(T) == 2 && scores_tc_supported(d));
   if (use_tc) {
     int rc = launch_scores_cellmax_tc(q, k, idx_q, idx_k, R, rowmax, extra, d, bh, sizeof(T) == 4 ? PSA_F32 :
-                                      (std::is_same<T, __half>::value ? PSA_F16 : PSA_BF16), st, rope);
+                                      (std::is_same<T, __half>::value ? PSA_F16 : PSA_BF16), st, rope, idx_step);
     if (rc != PSA_OK) return rc;
   } else {
-    PSA_REQUIRE(q.n_peers == 0 && k.n_peers == 0 && !rope.a, PSA_ERR_UNSUPPORTED, "the scalar score kernel reads local tensors only");
+    PSA_REQUIRE(q.n_peers == 0 && k.n_peers == 0 && !rope.a && idx_step == 1, PSA_ERR_UNSUPPORTED, "the scalar score kernel reads local tensors only");
     // Few query tiles (4096 tokens x 2 heads: 32) leave most SMs idle: the key tiles of each are then shared by up to 16
     // CTAs, whose row maxima meet through atomics (a maximum does not depend on the order): 128 -> 25 us.
     dim3 grid((unsigned)cdiv64(d.nq_s, 64), (unsigned)bh);
@@ -276,6 +276,18 @@ extern "C" int psa_block_scores(const void* q, const void* k, const int32_t* idx
   cudaStream_t st = (cudaStream_t)stream;
   PSA_DISPATCH_DTYPE(dtype, T, return launch_scores<T>(local_rows(q), local_rows(k), idx_q, idx_k, po, scratch, d, bh, impl, st));
   return PSA_OK;
+}
+
+int psa::block_scores_idx64(const void* q, const void* k, const int64_t* idx_q, const int64_t* idx_k, void* po, void* scratch,
+                            int64_t bh, int64_t seq_q, int64_t seq_k, int head_dim, int block_m, int block_n, int dtype, cudaStream_t st) {
+  ScoreDims d;
+  int rc = make_score_dims(d, seq_q, seq_k, head_dim, block_m, block_n);
+  if (rc != PSA_OK) return rc;
+  PSA_REQUIRE(scores_tc_supported(d), PSA_ERR_UNSUPPORTED, "64-bit sample indices: block sizes not covered by the tcgen05 path");
+  const int32_t* iq = reinterpret_cast<const int32_t*>(idx_q);      // little-endian: the low words, every second one
+  const int32_t* ik = reinterpret_cast<const int32_t*>(idx_k);
+  if (dtype == PSA_F16) return launch_scores<__half>(local_rows(q), local_rows(k), iq, ik, po, scratch, d, bh, 2, st, RopeTables{}, 2);
+  return launch_scores<__nv_bfloat16>(local_rows(q), local_rows(k), iq, ik, po, scratch, d, bh, 2, st, RopeTables{}, 2);
 }
 
 // ---------------------------------------------------------------------------------------------------------

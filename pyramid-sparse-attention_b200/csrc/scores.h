@@ -27,11 +27,15 @@ bool scores_tc_supported(const ScoreDims& d);
 size_t scores_tc_extra_scratch(const ScoreDims& d, int64_t bh);
 int launch_scores_cellmax_tc(const RowSource& q, const RowSource& k, const int32_t* idx_q, const int32_t* idx_k, void* R,
                              float* rowmax, void* extra, const ScoreDims& d, int64_t bh, int dtype, cudaStream_t st,
-                             const RopeTables& rope = RopeTables{});
+                             const RopeTables& rope = RopeTables{}, int idx_step = 1);
 
 // the same stage A on sample matrices that are already compacted: qs [bh][nq_s][D], ks [bh][nk_cols][D]
 int launch_scores_cellmax_tc_samples(const void* qs, const void* ks, void* R, float* rowmax, const ScoreDims& d, int64_t bh,
                                      int dtype, cudaStream_t st);
+
+// Block scores of 16-bit tensors with 64-bit sample offsets (what torch.topk returns); scratch as for psa_block_scores.
+int block_scores_idx64(const void* q, const void* k, const int64_t* idx_q, const int64_t* idx_k, void* po, void* scratch, int64_t bh,
+                       int64_t seq_q, int64_t seq_k, int head_dim, int block_m, int block_n, int dtype, cudaStream_t st);
 
 // rowmax[0, n) = -inf, before row maxima meet through atomic_max_float
 int launch_fill_neg_inf(float* x, int64_t n, cudaStream_t st);

@@ -24,11 +24,12 @@ constexpr int kSlabBytes = 128 * 128;
 constexpr int kThreads = 192;
 constexpr int kStages = 2;
 
-// One operand of the sample gather: rows of x picked by idx (keep per block of `block` tokens), n_out rows per head, those
-// past n_valid repeating the last one.
+// One operand of the sample gather: rows of x picked by idx (keep per block of `block` tokens; idx_step 2: the low words of
+// 64-bit indices), n_out rows per head, those past n_valid repeating the last one.
 struct SampleSet {
   RowSource x;
   const int32_t* idx;
+  int idx_step;
   uint4* out;
   int64_t seq;
   int block, keep, n_valid, n_out;
@@ -49,14 +50,14 @@ __global__ void __launch_bounds__(256) gather_samples_kernel(const SampleSet q, 
   if (unit >= n_blocks * bh_count) return;
   const int bh = heads_fastest ? unit % bh_count : unit / n_blocks, blk = heads_fastest ? unit / bh_count : unit % n_blocks;
   const int c = threadIdx.x % CPR, i0 = blk * (kRows * kUnroll) + (int)threadIdx.x / CPR;
-  const int32_t* idx = s.idx + (int64_t)bh * s.keep;
+  const int32_t* idx = s.idx + (int64_t)bh * s.keep * s.idx_step;
   uint4* dst = s.out + ((int64_t)bh * s.n_out) * CPR + c;
   int64_t tok[kUnroll];
   uint4 w[kUnroll];
 #pragma unroll
   for (int u = 0; u < kUnroll; ++u) {
     const int i = min(i0 + u * kRows, s.n_valid - 1);
-    const int64_t t = (int64_t)(i / s.keep) * s.block + idx[i % s.keep];
+    const int64_t t = (int64_t)(i / s.keep) * s.block + idx[i % s.keep * s.idx_step];
     tok[u] = t < s.seq ? t : s.seq - 1;
   }
 #pragma unroll
@@ -313,15 +314,15 @@ size_t scores_tc_extra_scratch(const ScoreDims& d, int64_t bh) {
 
 int launch_scores_cellmax_tc(const RowSource& q, const RowSource& k, const int32_t* idx_q, const int32_t* idx_k, void* R,
                              float* rowmax, void* extra, const ScoreDims& d, int64_t bh, int dtype, cudaStream_t st,
-                             const RopeTables& rope) {
+                             const RopeTables& rope, int idx_step) {
   PSA_REQUIRE(dtype == PSA_F16 || dtype == PSA_BF16, PSA_ERR_UNSUPPORTED, "the tcgen05 score kernel needs f16/bf16 inputs");
   PSA_REQUIRE(scores_tc_supported(d), PSA_ERR_UNSUPPORTED, "the tcgen05 score kernel does not cover this block size");
   const size_t qb = ((size_t)bh * d.nq_s * d.D * 2 + 255) & ~(size_t)255;
   void* qs = extra;
   void* ks = (char*)extra + qb;
   {
-    const SampleSet sq = {q, idx_q, (uint4*)qs, d.seq_q, d.bm, d.kq, d.nq_s, d.nq_s};
-    const SampleSet sk = {k, idx_k, (uint4*)ks, d.seq_k, d.bn, d.kk, d.nk_s, d.nk_cols};
+    const SampleSet sq = {q, idx_q, idx_step, (uint4*)qs, d.seq_q, d.bm, d.kq, d.nq_s, d.nq_s};
+    const SampleSet sk = {k, idx_k, idx_step, (uint4*)ks, d.seq_k, d.bn, d.kk, d.nk_s, d.nk_cols};
     const int rows_per_block = 256 / (d.D / 8) * 4;
     const int64_t units = cdiv64(std::max(d.nq_s, d.nk_cols), rows_per_block) * bh;
     PSA_REQUIRE(units < ((int64_t)1 << 31), PSA_ERR_ARG, "psa_block_scores: too many sampled rows");

@@ -131,6 +131,12 @@ class PSAAttention(nn.Module):
 
     def forward(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, idx_q=None, idx_k=None) -> torch.Tensor:
         config = self.config
+        if ops.layer_supported(q, k, v, config):
+            if idx_q is None:
+                idx_q = ops.draw_sample_indices(q.shape[0], q.shape[1], config.block_m, config.block_m // 4, q.device)
+            if idx_k is None:
+                idx_k = ops.draw_sample_indices(q.shape[0], q.shape[1], config.block_n, config.block_n // 4, q.device)
+            return ops.psa_layer(q, k, v, idx_q, idx_k, config)
         with torch.no_grad():
             mask, _, _ = compute_block_mask(q, k, config, text_length=0, idx_q=idx_q, idx_k=idx_k)
         return self.sparse_attention_fn(q.contiguous(), k.contiguous(), v.contiguous(), mask, None)

@@ -631,6 +631,45 @@ def psa_forward_to_rows(q, k, v, mask, block_m: int, block_n: int, tile_n: int, 
     return o
 
 
+def layer_supported(q, k, v, config) -> bool:
+    """Whether psa_layer takes this call (what it does not take goes through the single entry points)."""
+    if not (q.is_cuda and q.dim() == 4 and k.shape == v.shape and q.shape[:2] == k.shape[:2] and q.shape[3] == k.shape[3]
+            and q.dtype == k.dtype == v.dtype and q.device == k.device == v.device and q.numel() and k.numel()):
+        return False
+    n = len(config.mask_ratios) if config.mask_ratios else 0
+    return (config.attn_impl == "new_mask_type" and not config.use_sim_mask and config.mask_mode in ("topk", "thresholdbound")
+            and images_supported(k, config.block_m, config.block_n, config.tile_n) and 0 < n <= 8
+            and -(-k.shape[2] // config.block_n) + n <= 1472 and q.shape[0] * q.shape[1] < 65536)
+
+
+def psa_layer(q, k, v, idx_q, idx_k, config) -> torch.Tensor:
+    """Block scores, level mask, tile images and forward of one layer in a single call into the library (the same kernels
+    as block_scores, assign_levels, pyramid_kv_images and psa_forward: on short clips the four calls' host work is longer
+    than their kernels).  idx_q, idx_k: int64 sample offsets, as draw_sample_indices returns them."""
+    _need_cuda(q, k, v, idx_q, idx_k)
+    q, k, v = _flat_bh(q), _flat_bh(k), _flat_bh(v)
+    B, H, Sq, D = q.shape
+    Sk, bm, bn = k.shape[2], config.block_m, config.block_n
+    assert idx_q.shape == (B, H, bm // 4) and idx_k.shape == (B, H, bn // 4)
+    iq, ik = idx_q.to(torch.int64).contiguous(), idx_k.to(torch.int64).contiguous()
+    Mq, Nk, n = -(-Sq // bm), -(-Sk // bn), len(config.mask_ratios)
+    threshold = config.mask_mode == "thresholdbound"
+    levels, starts, ends, thr, aligns, min_index = _plan_of(config.mask_ratios, Nk, threshold, True, bn, config.tile_n, q.dtype)
+    with _on(q):
+        dt = _dt(q)
+        nbytes = lib.psa_layer_scratch_bytes(B * H, Sq, Sk, D, bm, bn, dt)
+        scratch = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
+        mask = torch.empty((B, H, Mq, Nk + n), dtype=torch.int32, device=q.device)
+        o = torch.empty_like(q)
+        status = status_word(q.device)
+        rc = lib.psa_layer(_ptr(q), _ptr(k), _ptr(v), _ptr(iq), _ptr(ik), _ptr(mask), _ptr(o), _ptr(scratch), nbytes, B * H, Sq, Sk, D,
+                           bm, bn, config.tile_n, int(threshold), n, levels, starts, ends, thr, aligns, min_index, float(D ** -0.5), 1,
+                           dt, _ptr(status), _stream(q))
+    check(rc, "psa_layer")
+    o._psa_status = status
+    return o
+
+
 class LegacyKV:
     """Pooled K/V of the legacy kernels (block 128) in the two layouts their kernels read, each built on first use: tile
     images (tcgen05 forward and backward) and row-major levels 2/4/8 (scalar and warp-level-mma kernels)."""
