@@ -8,13 +8,15 @@ namespace psa {
 // row from shared memory 16 bytes at a time (the four read 64 consecutive bytes, the other rows of the warp the same ones):
 // one shared-memory load feeds four multiply-adds.  With every fourth channel (one load per multiply-add) the loads were the
 // bound.  2 heads x 4096 tokens x 64, default ratios, with the rows of a block dealt to four CTAs: 238 -> 207 us,
-// and 166 us with eight staging loads in flight.
+// 166 us with eight staging loads in flight, 130 us with the chunks of a row dealt to four sets of threads.
 template <typename T, int D>
 struct FwdCore {
   static constexpr int DPT = D / 4;
   static __device__ __forceinline__ int channel(int d, int g) { return (d >> 2) * 16 + g * 4 + (d & 3); }
   float q[DPT], acc[DPT];
   float m, l;
+
+  static __device__ __forceinline__ void sync(int bar, int nt) { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(nt) : "memory"); }
 
   __device__ __forceinline__ void init(const T* qrow, bool valid, int g) {
 #pragma unroll
@@ -24,28 +26,29 @@ struct FwdCore {
 
   // Attend to C (<= 32) consecutive pooled tokens [t0, t0+C) of one level; only the first nv exist.
   // causal_level > 0: pooled token j is visible iff (j+1)*causal_level - 1 <= qpos.
+  // Called by nt threads (this one is number tid) that share Ks, Vs and the hardware barrier `bar`.
   __device__ __forceinline__ void chunk(const T* __restrict__ Kl, const T* __restrict__ Vl, int64_t t0, int C, int nv,
                                         float bias, float scale, float (*Ks)[D], float (*Vs)[D], int g,
-                                        int causal_level, int64_t qpos) {
-    __syncthreads();
+                                        int causal_level, int64_t qpos, int tid, int nt, int bar) {
+    sync(bar, nt);
     // eight elements of each operand in flight per thread (a block of 128 threads stages 16 to 32 of each)
     constexpr int kUnroll = 8;
-    for (int e0 = threadIdx.x; e0 < C * D; e0 += kUnroll * blockDim.x) {
+    for (int e0 = tid; e0 < C * D; e0 += kUnroll * nt) {
       float kx[kUnroll], vx[kUnroll];
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) {
-        const int e = e0 + u * blockDim.x;
+        const int e = e0 + u * nt;
         const bool ok = e < C * D && e / D < nv;
         kx[u] = ok ? Elem<T>::to_f(Kl[t0 * D + e]) : 0.f;
         vx[u] = ok ? Elem<T>::to_f(Vl[t0 * D + e]) : 0.f;
       }
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) {
-        const int e = e0 + u * blockDim.x;
+        const int e = e0 + u * nt;
         if (e < C * D) { Ks[e / D][e % D] = kx[u]; Vs[e / D][e % D] = vx[u]; }
       }
     }
-    __syncthreads();
+    sync(bar, nt);
     // 8 tokens per softmax step keeps the scores in registers without unrolling the whole chunk
     for (int c0 = 0; c0 < C; c0 += 8) {
       float s[8];

@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(512) psa_legacy_fwd_simt_kernel(const T* __res
     for (int c0 = 0; c0 < P; c0 += C) {
       const int64_t t0 = (int64_t)pb * P + c0;
       int64_t nv = lp.n[li] - t0; nv = nv < 0 ? 0 : (nv > C ? C : nv);
-      st.chunk(Kl, Vl, t0, C, (int)nv, bias, scale, Ks, Vs, g, causal ? level : 0, qrow);
+      st.chunk(Kl, Vl, t0, C, (int)nv, bias, scale, Ks, Vs, g, causal ? level : 0, qrow, threadIdx.x, blockDim.x, 0);
     }
   }
   if (valid) {
