@@ -133,6 +133,35 @@ __global__ void __launch_bounds__(256) gather_views_kernel(const ViewSet v, cons
   }
 }
 
+int launch_views(const ViewSet& v, int n, const int32_t* perm, const RopeTables& rope, int64_t batch, int heads, int64_t seq, int head_dim,
+                 cudaStream_t st) {
+  const int64_t blocks = cdiv64(seq, 256 / (head_dim / 8) * 4) * batch * heads;
+  PSA_REQUIRE(blocks < ((int64_t)1 << 31), PSA_ERR_ARG, "row copy: too many rows");
+  const dim3 grid((unsigned)blocks, 1, (unsigned)n);
+  const int bh = (int)(batch * heads);
+  if (head_dim == 64) {
+    if (rope.a) gather_views_kernel<8, true><<<grid, 256, 0, st>>>(v, perm, seq, heads, bh, rope);
+    else gather_views_kernel<8, false><<<grid, 256, 0, st>>>(v, perm, seq, heads, bh, rope);
+  } else {
+    if (rope.a) gather_views_kernel<16, true><<<grid, 256, 0, st>>>(v, perm, seq, heads, bh, rope);
+    else gather_views_kernel<16, false><<<grid, 256, 0, st>>>(v, perm, seq, heads, bh, rope);
+  }
+  PSA_CHECK_LAUNCH("row copy");
+  return PSA_OK;
+}
+
+// One operand of 16-bit rows of 64 or 128 channels, its strides in elements.
+int launch_one_view(const void* src, void* dst, int64_t head_stride, int64_t token_stride, const int32_t* perm, const RopeTables& rope,
+                    int heads, int64_t seq, int head_dim, cudaStream_t st) {
+  ViewSet v = {};
+  v.src[0] = (const uint4*)src;
+  v.dst[0] = (uint4*)dst;
+  v.head_stride[0] = head_stride / 8;
+  v.token_stride[0] = token_stride / 8;
+  v.rotate[0] = rope.a != nullptr;
+  return launch_views(v, 1, perm, rope, 1, heads, seq, head_dim, st);
+}
+
 }  // namespace
 }  // namespace psa
 
@@ -163,22 +192,7 @@ extern "C" int psa_gather_views(const void* const* src, const int64_t* strides, 
     v.token_stride[i] = strides[3 * i + 2] / 8;
     v.rotate[i] = rotate[i] != 0;
   }
-  const RopeTables rope = {rope_a, rope_b, rope_first, dtype == PSA_BF16};
-  const int rows_per_block = 256 / (head_dim / 8) * 4;
-  const int64_t blocks = cdiv64(seq, rows_per_block) * batch * heads;
-  PSA_REQUIRE(blocks < ((int64_t)1 << 31), PSA_ERR_ARG, "psa_gather_views: too many rows");
-  const dim3 grid((unsigned)blocks, 1, (unsigned)n);
-  const int bh = (int)(batch * heads);
-  cudaStream_t st = (cudaStream_t)stream;
-  if (head_dim == 64) {
-    if (rope_a) gather_views_kernel<8, true><<<grid, 256, 0, st>>>(v, perm, seq, heads, bh, rope);
-    else gather_views_kernel<8, false><<<grid, 256, 0, st>>>(v, perm, seq, heads, bh, rope);
-  } else {
-    if (rope_a) gather_views_kernel<16, true><<<grid, 256, 0, st>>>(v, perm, seq, heads, bh, rope);
-    else gather_views_kernel<16, false><<<grid, 256, 0, st>>>(v, perm, seq, heads, bh, rope);
-  }
-  PSA_CHECK_LAUNCH("psa_gather_views");
-  return PSA_OK;
+  return launch_views(v, n, perm, {rope_a, rope_b, rope_first, dtype == PSA_BF16}, batch, heads, seq, head_dim, (cudaStream_t)stream);
 }
 
 extern "C" int psa_gather_rows(const void* src, const int32_t* perm, void* dst, int64_t bh, int64_t seq, int head_dim,
@@ -191,6 +205,8 @@ extern "C" int psa_gather_rows(const void* src, const int32_t* perm, void* dst, 
   PSA_REQUIRE(head_dim > 0 && (head_dim * elem_bytes) % 16 == 0, PSA_ERR_ARG,
               "psa_gather_rows: rows of %d bytes are not a multiple of 16", head_dim * elem_bytes);
   PSA_REQUIRE((((uintptr_t)src | (uintptr_t)dst) & 15) == 0, PSA_ERR_ARG, "psa_gather_rows: src and dst must be 16-byte aligned");
+  if (elem_bytes == 2 && (head_dim == 64 || head_dim == 128))
+    return launch_one_view(src, dst, seq * head_dim, head_dim, perm, RopeTables{}, (int)bh, seq, head_dim, (cudaStream_t)stream);
   const int cpr = head_dim * elem_bytes / 16;
   int64_t blocks = cdiv64(seq * cpr, 256);
   // enough CTAs to cover the machine several times over once the heads (grid.y) are counted in
@@ -212,6 +228,8 @@ extern "C" int psa_gather_heads(const void* src, const int32_t* perm, void* dst,
   PSA_REQUIRE(head_dim > 0 && (head_dim * elem_bytes) % 16 == 0, PSA_ERR_ARG,
               "psa_gather_heads: rows of %d bytes are not a multiple of 16", head_dim * elem_bytes);
   PSA_REQUIRE((((uintptr_t)src | (uintptr_t)dst) & 15) == 0, PSA_ERR_ARG, "psa_gather_heads: src and dst must be 16-byte aligned");
+  if (elem_bytes == 2 && (head_dim == 64 || head_dim == 128))
+    return launch_one_view(src, dst, head_dim, (int64_t)heads * head_dim, perm, RopeTables{}, heads, seq, head_dim, (cudaStream_t)stream);
   const int cpr = head_dim * elem_bytes / 16;
   int64_t blocks = cdiv64(seq * cpr, 256);
   const int64_t cap = cdiv64(148 * 16, heads);
@@ -233,6 +251,9 @@ extern "C" int psa_gather_heads_rope(const void* src, const int32_t* perm, const
   PSA_REQUIRE(head_dim > 0 && head_dim % 8 == 0, PSA_ERR_ARG, "psa_gather_heads_rope: head_dim=%d is not a multiple of 8", head_dim);
   PSA_REQUIRE((((uintptr_t)src | (uintptr_t)dst | (uintptr_t)rope_a | (uintptr_t)rope_b) & 15) == 0, PSA_ERR_ARG,
               "psa_gather_heads_rope: src, dst and the tables must be 16-byte aligned");
+  if (head_dim == 64 || head_dim == 128)
+    return launch_one_view(src, dst, head_dim, (int64_t)heads * head_dim, perm, {rope_a, rope_b, rope_first, dtype == PSA_BF16}, heads, seq,
+                           head_dim, (cudaStream_t)stream);
   const int cpr = head_dim * 2 / 16;
   int64_t blocks = cdiv64(seq * cpr, 256);
   const int64_t cap = cdiv64(148 * 16, heads);
@@ -255,6 +276,9 @@ extern "C" int psa_gather_rows_rope(const void* src, const int32_t* perm, const 
   PSA_REQUIRE(head_dim > 0 && head_dim % 8 == 0, PSA_ERR_ARG, "psa_gather_rows_rope: head_dim=%d is not a multiple of 8", head_dim);
   PSA_REQUIRE((((uintptr_t)src | (uintptr_t)dst | (uintptr_t)rope_a | (uintptr_t)rope_b) & 15) == 0, PSA_ERR_ARG,
               "psa_gather_rows_rope: src, dst and the tables must be 16-byte aligned");
+  if (head_dim == 64 || head_dim == 128)
+    return launch_one_view(src, dst, seq * head_dim, head_dim, perm, {rope_a, rope_b, rope_first, dtype == PSA_BF16}, (int)bh, seq, head_dim,
+                           (cudaStream_t)stream);
   const int cpr = head_dim * 2 / 16;
   int64_t blocks = cdiv64(seq * cpr, 256);
   const int64_t cap = cdiv64(148 * 16, bh);
