@@ -626,10 +626,17 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
         int qk_next = 0, pv_next = 0;
           while (ok && pv_next < n_tiles) {
             bool progressed = false;
+            // The looks at the three barriers of a round overlap (~170 cycles each, complete or not); a phase that completes in
+            // between is found in the next round.  One look after the other, each where its answer was needed: 740 instead of
+            // 715 us at 12 x 32760 x 128, 2733 instead of 2610 us for a causal prefill of 28 x 32768.
+            const int gv = g0 + pv_next, gk = g0 + qk_next;
+            const bool p_there = tc::mbar_test_wait_a(p_full_a + ((gv & 1) * 2 + ((gv >> 1) & 1)) * 8, (gv >> 2) & 1);
+            const bool v_there = tc::mbar_test_wait_a(v_full_a + (gv % C::NV) * 8, (gv / C::NV) & 1);
+            const bool k_there = tc::mbar_test_wait_a(k_full_a + (gk % C::NK) * 8, (gk / C::NK) & 1);
             if (pv_next < qk_next) {
-              const int t = pv_next, gt = g0 + t, b = gt & 1, stage = gt % C::NV;
+              const int t = pv_next, gt = gv, b = gt & 1, stage = gt % C::NV;
               if (!o_ok) o_ok = tc::mbar_test_wait_a(o_free_a, (q_rows - 1) & 1);
-            if (o_ok && tc::mbar_test_wait_a(p_full_a + (b * 2 + ((gt >> 1) & 1)) * 8, (gt >> 2) & 1) && tc::mbar_test_wait_a(v_full_a + stage * 8, (gt / C::NV) & 1)) {
+            if (o_ok && p_there && v_there) {
                 tc::tc_fence_after();
                 const uint64_t vdesc = vdesc0 + (uint64_t)(stage * (C::TILE_BYTES >> 4));
                 const uint32_t tP = tmem + (gt % C::NSB) * 128;              // probabilities overwrite the scores they came from
@@ -658,8 +665,8 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
             // issue order, so "S_t ready" then also means that P V of tile t-NSB has finished reading the probabilities that
             // were written over the scores of buffer t mod NSB
             if (qk_next < n_tiles && qk_next <= pv_next + C::NSB - 1) {
-              const int t = qk_next, gt = g0 + t, stage = gt % C::NK;
-              if (tc::mbar_test_wait_a(k_full_a + stage * 8, (gt / C::NK) & 1)) {
+              const int t = qk_next, gt = gk, stage = gt % C::NK;
+              if (k_there) {
                 tc::tc_fence_after();
                 const uint64_t kdesc = kdesc0 + (uint64_t)(stage * (C::TILE_BYTES >> 4));
                 const uint32_t idesc_qk = t == n_tiles - 1 ? tc::make_idesc(FMT, 128, last_cols, 0, 0) : idesc_qk_full;
