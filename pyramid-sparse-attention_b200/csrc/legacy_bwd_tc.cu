@@ -11,9 +11,10 @@
 // The element-wise warps work in two phases per tile: the probabilities as soon as S is there (kept in registers), dS once
 // dP is.  So half of their work runs under products: in the dK/dV kernel dV and the next S under phase 2, dK and the next dP
 // under phase 1; in the dQ kernel (S double-buffered) dQ and the next dP under phase 1 of the next tile.
-// Tensor / element-wise bound.  2 x 16 heads x 32768 tokens x 128, causal, random levels: dK/dV 14.3 -> 12.2 ms, dQ 7.3 -> 6.0 ms
-// against both products of a tile before its whole element-wise pass with two stages per ring; 28 heads x 5003 tokens:
-// 492 -> 440 and 334 -> 277 us.
+// Bound by the issuing thread and its hand-overs with the element-wise warps: with empty element-wise bodies 10.1 of 12.1 ms
+// remained, without ex2 or with half of the copies all of it.  2 x 16 heads x 32768 tokens x 128, causal, random levels: dK/dV
+// 14.3 -> 11.4 ms, dQ 7.3 -> 6.0 ms against both products of a tile before its whole element-wise pass with two stages per
+// ring; 28 heads x 5003 tokens: 492 -> 410 and 334 -> 273 us.
 //
 //   bwd_dq_tc_kernel    stationary: Q and dO of one query block (rows = queries).  Stream: the selected key blocks of
 //                       all levels, PACKED back to back into 128-token K and V tiles (tile images, one linear bulk copy
@@ -286,13 +287,19 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dkdv_tc_kernel(const __gri
       int gp = 0, ic = 0;
       auto q_off = [&](int u) { return (uint64_t)((uint32_t)((u % C::NX) * C::TILE) >> 4); };
       auto d_off = [&](int u) { return (uint64_t)((uint32_t)((u % C::NY) * C::TILE) >> 4); };
-      // a stationary tile (image layout) times a stream tile, N = 128 query rows
-      auto issue_ss = [&](uint32_t dst, uint64_t adesc, uint64_t bdesc, uint32_t done) {
+      // a stationary tile (image layout) times a stream tile, N = 128 query rows.  A look at a barrier takes ~170 cycles whether
+      // its phase is complete or not, so the one the next product needs is looked at behind the last but two MMAs of this one (dK/dV
+      // 12.5 -> 11.4 ms, the look at the next stage before an accumulating product included).
+      auto issue_ss = [&](uint32_t dst, uint64_t adesc, uint64_t bdesc, uint32_t done, uint32_t next_bar, uint32_t next_par) -> bool {
+        bool there = false;
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks)
+        for (int ks = 0; ks < D / 16; ++ks) {
           tc::umma_ss(dst, adesc + (uint64_t)(((ks >> 2) * 1024 + (ks & 3) * 32) >> 4),
                       bdesc + (uint64_t)(((ks >> 2) * kSlab + (ks & 3) * 32) >> 4), idesc_s, ks > 0 ? 1u : 0u);
+          if (ks == D / 16 - 3) there = tc::mbar_test_wait_a(next_bar, next_par);
+        }
         tc::umma_commit_a(done);
+        return there;
       };
       // an accumulating product.  k-step ks = query rows [16 ks, 16 ks + 16); its 16-bit operand sits at column
       // 32 (ks / 2) + 8 (ks % 2) of the buffer the fp32 values came from
@@ -311,35 +318,40 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dkdv_tc_kernel(const __gri
         if (ok) ok = tc::mbar_wait_a(q_full_a + (gp % C::NX) * 8, (gp / C::NX) & 1, abort_flag);
         if (!ok) break;
         tc::tc_fence_after();
-        issue_ss(tmem + kST, kdesc, qk0 + q_off(gp), s_full_a);
-        ok = tc::mbar_wait_a(d_full_a + (gp % C::NY) * 8, (gp / C::NY) & 1, abort_flag);
+        if (!issue_ss(tmem + kST, kdesc, qk0 + q_off(gp), s_full_a, d_full_a + (gp % C::NY) * 8, (gp / C::NY) & 1))
+          ok = tc::mbar_wait_a(d_full_a + (gp % C::NY) * 8, (gp / C::NY) & 1, abort_flag);
         if (!ok) break;
         tc::tc_fence_after();
-        issue_ss(tmem + kDP, vdesc, dk0 + d_off(gp), dp_full_a);
+        bool p_there = issue_ss(tmem + kDP, vdesc, dk0 + d_off(gp), dp_full_a, p_full_a, gp & 1);
         // dV and S^T of the next tile run while the element-wise warps turn dP^T into dS^T, dK and dP^T of the next tile
         // while they take the probabilities of the next tile
         for (bool first = true; ok; first = false, ++gp) {
           const bool last = (ent[gp % C::NX] >> 31) != 0;
-          ok = tc::mbar_wait_a(p_full_a, gp & 1, abort_flag);
+          if (!p_there) ok = tc::mbar_wait_a(p_full_a, gp & 1, abort_flag);
           if (ok && first && ic > 0) ok = tc::mbar_wait(&ctl->acc_free, (ic - 1) & 1, abort_flag);
           if (!ok) break;
           tc::tc_fence_after();
+          bool ds_there = false;
+          const uint32_t q_bar = q_full_a + ((gp + 1) % C::NX) * 8, q_par = ((gp + 1) / C::NX) & 1;
+          const bool q_there = tc::mbar_test_wait_a(q_bar, q_par);
           issue_acc(tmem + kAccV, tmem + kST, dm0 + d_off(gp), first);
           if (!last) {
-            ok = tc::mbar_wait_a(q_full_a + ((gp + 1) % C::NX) * 8, ((gp + 1) / C::NX) & 1, abort_flag);
+            if (!q_there) ok = tc::mbar_wait_a(q_bar, q_par, abort_flag);
             if (!ok) break;
             tc::tc_fence_after();
-            issue_ss(tmem + kST, kdesc, qk0 + q_off(gp + 1), s_full_a);      // "S ready" also says: dV of this tile is complete
+            ds_there = issue_ss(tmem + kST, kdesc, qk0 + q_off(gp + 1), s_full_a, ds_full_a, gp & 1);   // "S ready" also says: dV of this tile is complete
           }
-          ok = tc::mbar_wait_a(ds_full_a, gp & 1, abort_flag);
+          if (!ds_there) ok = tc::mbar_wait_a(ds_full_a, gp & 1, abort_flag);
           if (!ok) break;
           tc::tc_fence_after();
+          const uint32_t d_bar = d_full_a + ((gp + 1) % C::NY) * 8, d_par = ((gp + 1) / C::NY) & 1;
+          const bool d_there = tc::mbar_test_wait_a(d_bar, d_par);
           issue_acc(tmem + kAccK, tmem + kDP, qm0 + q_off(gp), first);
           if (last) { ++gp; break; }
-          ok = tc::mbar_wait_a(d_full_a + ((gp + 1) % C::NY) * 8, ((gp + 1) / C::NY) & 1, abort_flag);
+          if (!d_there) ok = tc::mbar_wait_a(d_bar, d_par, abort_flag);
           if (!ok) break;
           tc::tc_fence_after();
-          issue_ss(tmem + kDP, vdesc, dk0 + d_off(gp + 1), dp_full_a);       // "dP ready" also says: dK of this tile is complete
+          p_there = issue_ss(tmem + kDP, vdesc, dk0 + d_off(gp + 1), dp_full_a, p_full_a, (gp + 1) & 1);   // "dP ready" also says: dK of this tile is complete
         }
         if (!ok) break;
         tc::umma_commit(&ctl->acc_full);
@@ -730,7 +742,11 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dq_tc_kernel(const __grid_
         uint32_t idle = 0;
         while (ok && !done) {
           bool progressed = false;
-          if (na < np && tc::mbar_test_wait_a(ds_full_a, na & 1)) {
+          // the three looks overlap (~170 cycles each); a phase that completes in between is found in the next round
+          const bool ds_there = tc::mbar_test_wait_a(ds_full_a, na & 1);
+          const bool y_there = tc::mbar_test_wait_a(y_full_a + (np % C::NY) * 8, (np / C::NY) & 1);
+          const bool x_there = tc::mbar_test_wait_a(x_full_a + (ns % C::NX) * 8, (ns / C::NX) & 1);
+          if (na < np && ds_there) {
             if (na == g0 && rc > 0) {
               ok = tc::mbar_wait(&ctl->acc_free, (rc - 1) & 1, abort_flag);
               if (!ok) break;
@@ -742,13 +758,13 @@ __global__ void __launch_bounds__(kThreadsBwd, 1) bwd_dq_tc_kernel(const __grid_
             ++na;
             progressed = true;
           }
-          if (np < ns && np == na && tc::mbar_test_wait_a(y_full_a + (np % C::NY) * 8, (np / C::NY) & 1)) {
+          if (np < ns && np == na && y_there) {
             tc::tc_fence_after();
             issue_ss(tmem + kDP, ddesc, vk0 + y_off(np), (int)(ent[np % C::NX] & 0xffffu), dp_full_a);   // also says: dQ of the tile before is complete
             ++np;
             progressed = true;
           }
-          if (!s_done && ns <= na + 1 && tc::mbar_test_wait_a(x_full_a + (ns % C::NX) * 8, (ns / C::NX) & 1)) {
+          if (!s_done && ns <= na + 1 && x_there) {
             tc::tc_fence_after();
             const uint32_t e = ent[ns % C::NX];
             issue_ss(tmem + kS + (ns & 1) * 128, qdesc, kk0 + x_off(ns), (int)(e & 0xffffu), s_full_a + (ns & 1) * 8);
