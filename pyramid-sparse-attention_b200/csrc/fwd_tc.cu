@@ -64,8 +64,8 @@ namespace psa {
 
 namespace {
 
-constexpr int kMaxWidth = 1472;        // longest index list (entries) the kernel handles
-constexpr int kMaxItems = 1504;        // item table capacity (entries + extra + padding blocks); two tables
+constexpr int kMaxWidth = 1472;        // longest index list (entries) of the common kernel
+constexpr int kMaxWidthWide = 4096;    // ... and of the WIDE variant (row-major K/V; a block number has 12 bits)
 constexpr int kSlabBytes = 128 * 128;  // 128 rows x 128 B (64 16-bit channels)
 constexpr int kProducerWarps = 3;
 constexpr int kProducerThreads = kProducerWarps * 32;
@@ -104,9 +104,12 @@ struct TcParams {
 // FIXED: the reference exponent of a query row is the maximum of its FIRST tile and is never raised (see the head of the
 // file).  No maximum pass after the first tile, no rescaling of the accumulator, hence ONE accumulator for both softmax
 // groups and room for a third score buffer.
-template <int D, bool FIXED = false> struct Cfg {
+// WIDE: longer index lists.  At head_dim 128 their tables take the place of the third K stage.
+template <int D, bool FIXED = false, bool WIDE = false> struct Cfg {
   static constexpr int SLABS = D / 64;
-  static constexpr int NK = D == 64 ? 4 : 3;   // K-tile ring
+  static constexpr int MAX_WIDTH = WIDE ? kMaxWidthWide : kMaxWidth;
+  static constexpr int MAX_ITEMS = MAX_WIDTH + 32;      // item table capacity (entries + extra + padding blocks); two tables
+  static constexpr int NK = D == 64 ? 4 : WIDE ? 2 : 3;   // K-tile ring
   static constexpr int NV = D == 64 ? 4 : 2;   // V-tile ring
   // Score buffers in TMEM.  At D = 128 the two accumulators leave room for two; at D = 64 for three, and the third one
   // lets Q K^T run two tiles ahead of P V, so that a softmax group finds its next scores ready when it is done with a tile.
@@ -130,9 +133,10 @@ template <int D, bool FIXED = false> struct Cfg {
   static constexpr int OFF_MINROW = OFF_BIASG + kBiasSlots * (32 + 4) * 4;   // causal: first query row that sees a column
   static constexpr int OFF_XCH = OFF_MINROW + kBiasSlots * 128;
   static constexpr int OFF_ROW = OFF_XCH + 2 * 2 * 2 * 128 * 4 + 4 * 128 * 4;   // (max, sum) of both groups, two rows in flight; reference exponents of four rows
-  static constexpr int OFF_RAW = OFF_ROW + 2 * kMaxItems * 4;      // raw index list of the row being decoded
-  static constexpr int OFF_CTRL = OFF_RAW + kMaxWidth * 4;
+  static constexpr int OFF_RAW = OFF_ROW + 2 * MAX_ITEMS * 4;      // raw index list of the row being decoded
+  static constexpr int OFF_CTRL = OFF_RAW + MAX_WIDTH * 4;
   static constexpr int SMEM_BYTES = OFF_CTRL + 1024 + 1024;   // control block + alignment slack
+  static_assert(SMEM_BYTES <= 232448, "more than 227 KB of shared memory");
 };
 
 struct Ctrl {
@@ -192,9 +196,9 @@ constexpr uint32_t kItemQuirk = 1u << 14, kItemPad = 1u << 15;
 
 // IMG = true: K/V tiles use the image layout [8-row group][slab][8 rows][128 B] and are filled by linear bulk copies from
 // the tile-image buffers; IMG = false: [slab][128 rows][128 B] filled by tensor-map TMA boxes from row-major tensors.
-template <int D, int FMT, bool IMG, bool CAUSAL, bool FIXED>
+template <int D, int FMT, bool IMG, bool CAUSAL, bool FIXED, bool WIDE>
 __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_constant__ TmapPack maps, const TcParams p) {
-  using C = Cfg<D, FIXED>;
+  using C = Cfg<D, FIXED, WIDE>;
   if (p.only_if && *p.only_if == 0) return;
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
@@ -302,7 +306,7 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
         }
         return good;
       }
-      uint32_t* table = sItems + (rit_n & 1) * kMaxItems;
+      uint32_t* table = sItems + (rit_n & 1) * C::MAX_ITEMS;
       asm volatile("cp.async.wait_all;" ::: "memory");
       if (!warps_rendezvous(&ctl->prod_sync, syncs, abort_flag)) return false;
       for (int i = ptid; i < p.width; i += kProducerThreads)
@@ -392,7 +396,7 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
       const int R = ctl->claimed[rit & 1];         // fixed since the decode of this row
       if (R >= p.total_rows) break;
       const int m = R % p.mq, bh = R / p.mq;
-      const uint32_t* sIt = sItems + (rit & 1) * kMaxItems;     // this row's item table
+      const uint32_t* sIt = sItems + (rit & 1) * C::MAX_ITEMS;     // this row's item table
       // the decode (by every producer thread) ended with a rendezvous, so the row's figures are visible
       const int n_tiles = ctl->dec[rit & 1].n_tiles, last_cols = ctl->dec[rit & 1].last_cols, n_items = ctl->dec[rit & 1].n_items;
       const float qb0 = ctl->dec[rit & 1].qbias2[0], qb1 = ctl->dec[rit & 1].qbias2[1], qb2 = ctl->dec[rit & 1].qbias2[2],
@@ -1105,7 +1109,7 @@ bool fwd_tc_supported(const FwdArgs& a) {
   if (a.dtype != PSA_F16 && a.dtype != PSA_BF16) return false;
   if (a.bm != 128 || a.tn != 32) return false;
   if (a.D != 64 && a.D != 128) return false;
-  if (a.width > kMaxWidth) return false;
+  if (a.width > (a.kimg || a.causal ? kMaxWidth : kMaxWidthWide)) return false;
   if (a.bh > 65535) return false;
   if (!(a.scale > 0.f)) return false;
   const void* ptrs[] = {a.q, a.out, a.k[0], a.k[1], a.k[2], a.k[3], a.v[0], a.v[1], a.v[2], a.v[3]};
@@ -1146,9 +1150,9 @@ static int next_counters(int n, int** out, cudaStream_t st) {
   return PSA_OK;
 }
 
-template <int D, int FMT, bool IMG, bool CAUSAL, bool FIXED>
+template <int D, int FMT, bool IMG, bool CAUSAL, bool FIXED, bool WIDE>
 static int launch_tc(const FwdArgs& a, cudaStream_t st, int* row_counter, int* guard = nullptr, const int* only_if = nullptr) {
-  using C = Cfg<D, FIXED>;
+  using C = Cfg<D, FIXED, WIDE>;
   TmapPack maps;
   const int is_bf16 = FMT == 1;
   int rc = encode_tmap_3d(&maps.q, a.q, 2, is_bf16, D, a.seq_q, a.bh, 128);
@@ -1171,7 +1175,7 @@ static int launch_tc(const FwdArgs& a, cudaStream_t st, int* row_counter, int* g
   p.scatter = a.scatter;
   p.lse = a.lse; p.legacy = a.legacy; p.causal = a.causal;
   p.guard = guard; p.only_if = only_if;
-  cudaError_t e = cudaFuncSetAttribute(psa_fwd_tc_kernel<D, FMT, IMG, CAUSAL, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+  cudaError_t e = cudaFuncSetAttribute(psa_fwd_tc_kernel<D, FMT, IMG, CAUSAL, FIXED, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
   PSA_REQUIRE(e == cudaSuccess, PSA_ERR_CUDA, "psa_fwd: shared-memory opt-in (%d B) failed: %s", C::SMEM_BYTES,
               cudaGetErrorString(e));
   // persistent: one CTA per SM (221 KB of shared memory and all 512 TMEM columns each), rows dealt round-robin so that
@@ -1182,29 +1186,29 @@ static int launch_tc(const FwdArgs& a, cudaStream_t st, int* row_counter, int* g
   PSA_REQUIRE(sms > 0, PSA_ERR_CUDA, "psa_fwd: cannot read the SM count");
   const unsigned grid = (unsigned)(p.total_rows < sms ? p.total_rows : sms);
   p.row_counter = row_counter;
-  psa_fwd_tc_kernel<D, FMT, IMG, CAUSAL, FIXED><<<grid, kThreads, C::SMEM_BYTES, st>>>(maps, p);
+  psa_fwd_tc_kernel<D, FMT, IMG, CAUSAL, FIXED, WIDE><<<grid, kThreads, C::SMEM_BYTES, st>>>(maps, p);
   PSA_CHECK_LAUNCH("psa_fwd(tcgen05)");
   return PSA_OK;
 }
 
 // The fixed-reference kernel, then the exact one, which returns at once unless the first one raised its guard word (a row
 // whose probabilities came near the end of the exponent range) - no host round trip.
-template <int D, int FMT, bool IMG, bool CAUSAL>
+template <int D, int FMT, bool IMG, bool CAUSAL, bool WIDE = false>
 static int launch_fixed_then_exact(const FwdArgs& a, cudaStream_t st) {
   static_assert(FMT == 1, "bf16 only");
   int* words = nullptr;                       // row counters of both kernels and the guard word
   int rc = next_counters(3, &words, st);
   if (rc != PSA_OK) return rc;
-  rc = launch_tc<D, FMT, IMG, CAUSAL, true>(a, st, words, words + 2, nullptr);
+  rc = launch_tc<D, FMT, IMG, CAUSAL, true, WIDE>(a, st, words, words + 2, nullptr);
   if (rc != PSA_OK) return rc;
-  return launch_tc<D, FMT, IMG, CAUSAL, false>(a, st, words + 1, nullptr, words + 2);
+  return launch_tc<D, FMT, IMG, CAUSAL, false, WIDE>(a, st, words + 1, nullptr, words + 2);
 }
 
-template <int D, int FMT, bool IMG, bool CAUSAL>
+template <int D, int FMT, bool IMG, bool CAUSAL, bool WIDE = false>
 static int launch_exact(const FwdArgs& a, cudaStream_t st) {
   int* words = nullptr;
   const int rc = next_counters(1, &words, st);
-  return rc != PSA_OK ? rc : launch_tc<D, FMT, IMG, CAUSAL, false>(a, st, words);
+  return rc != PSA_OK ? rc : launch_tc<D, FMT, IMG, CAUSAL, false, WIDE>(a, st, words);
 }
 
 int fwd_tc_launch(const FwdArgs& a, cudaStream_t st) {
@@ -1221,6 +1225,10 @@ int fwd_tc_launch(const FwdArgs& a, cudaStream_t st) {
     return fmt ? launch_fixed_then_exact<128, 1, true, false>(a, st) : launch_exact<128, 0, true, false>(a, st);
   }
   PSA_REQUIRE(!a.causal, PSA_ERR_UNSUPPORTED, "the causal rule needs the tile-image path");
+  if (a.width > kMaxWidth) {      // e.g. 75600 tokens in blocks of 32: lists of 2368 entries, which ran on the scalar kernel
+    if (a.D == 64) return fmt ? launch_fixed_then_exact<64, 1, false, false, true>(a, st) : launch_exact<64, 0, false, false, true>(a, st);
+    return fmt ? launch_fixed_then_exact<128, 1, false, false, true>(a, st) : launch_exact<128, 0, false, false, true>(a, st);
+  }
   if (a.D == 64) return fmt ? launch_fixed_then_exact<64, 1, false, false>(a, st) : launch_exact<64, 0, false, false>(a, st);
   return fmt ? launch_fixed_then_exact<128, 1, false, false>(a, st) : launch_exact<128, 0, false, false>(a, st);
 }

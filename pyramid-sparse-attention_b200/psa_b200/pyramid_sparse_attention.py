@@ -231,7 +231,7 @@ class PyramidSparseAttention(nn.Module):
             q_r, k_r, v_r = ops.gather_views(q, k, v, perm, rotary)
             c = self.config
             if (perm is not None and c.attn_impl == "new_mask_type" and c.block_m == 128 and c.block_n == 32 and c.tile_n == 32
-                    and -(-k.shape[2] // c.block_n) + len(c.mask_ratios) <= 1472):
+                    and -(-k.shape[2] // c.block_n) + len(c.mask_ratios) <= 4096):
                 # ... and the way back is where the forward stores its rows
                 with torch.no_grad():
                     mask, _, _ = compute_block_mask(q_r, k_r, c, text_length=c.text_length)
