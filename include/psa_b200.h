@@ -120,7 +120,8 @@ int psa_ksim(const void* k, int32_t* out, int64_t bh, int64_t seq, int head_dim,
  * mask: int32 [BH, ceil(seq_q/block_m), mask_width], per row: level-1 block indices, -1, level-2, -1,
  * level-4, -1, level-8, -1, rest ignored.  compat_quirk != 0 reproduces the reference's handling of levels
  * whose pooled block is narrower than half a tile (:261-278): each merged pair also attends pooled tokens
- * [2P, tile_n) of that level.  impl: 0 = pick, 1 = scalar kernel, 2 = tcgen05 kernel (f16/bf16, block_m 128).
+ * [2P, tile_n) of that level.  impl: 0 = pick, 1 = scalar kernel, 2 = tcgen05 kernel (f16/bf16, block_m 128; lists of up to
+ * 1472 entries over up to 16384 key blocks, or of up to 4096 entries over up to 8192 - what 0 picks it for).
  * status: device int32 word, written non-zero if a bounded wait inside the kernel expired (may be NULL).
  * The tcgen05 kernel is persistent: its CTAs claim query blocks from a counter.  The counters are a ring of 256 device
  * words inside the library (one per launch, zeroed on the launching stream right before the kernel); the first

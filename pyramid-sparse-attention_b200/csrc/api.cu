@@ -51,7 +51,9 @@ static int fwd_rows(const void* q, const void* k, const void* v, const void* k2,
   a.width = mask_width; a.scale = sm_scale; a.quirk = compat_quirk; a.dtype = dtype;
   a.scatter.row_perm = out_perm;
   const bool tc_ok = fwd_tc_supported(a);
-  if (impl == 2) PSA_REQUIRE(tc_ok, PSA_ERR_UNSUPPORTED, "psa_fwd: the tcgen05 kernel needs f16/bf16, block_m=128");
+  if (impl == 2) PSA_REQUIRE(tc_ok, PSA_ERR_UNSUPPORTED, 
+                              "psa_fwd: the tcgen05 kernel needs f16/bf16, block_m=128, lists of at most 4096 entries and 8192 key blocks (16384 "
+                              "up to 1472 entries)");
   if (impl == 2 || (impl == 0 && tc_ok)) return fwd_tc_launch(a, st);
   return fwd_simt_dispatch(q, kl, vl, nl, mask, out, bh, seq_q, head_dim, block_m, block_n, tile_n, mask_width, sm_scale,
                            compat_quirk, dtype, st);

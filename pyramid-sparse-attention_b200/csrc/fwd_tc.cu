@@ -65,7 +65,7 @@ namespace psa {
 namespace {
 
 constexpr int kMaxWidth = 1472;        // longest index list (entries) of the common kernel
-constexpr int kMaxWidthWide = 4096;    // ... and of the WIDE variant (row-major K/V; a block number has 12 bits)
+constexpr int kMaxWidthWide = 4096;    // ... and of the WIDE variant (row-major K/V)
 constexpr int kSlabBytes = 128 * 128;  // 128 rows x 128 B (64 16-bit channels)
 constexpr int kProducerWarps = 3;
 constexpr int kProducerThreads = kProducerWarps * 32;
@@ -188,17 +188,32 @@ __device__ __forceinline__ bool warps_rendezvous(uint64_t* bar, int& uses, volat
   return __all_sync(0xffffffffu, ok);
 }
 
-// Item table entry (one gathered block): bits 0-11 block index, 12-13 level index, 14 extra block of a narrow level
-// (reference compatibility), 15 inert padding block, 16-31 first tile column of the block counted from the start
-// of the row's token stream, in units of 4 tokens.
-constexpr uint32_t kItemQuirk = 1u << 14, kItemPad = 1u << 15;
-
+// Item table entry (one gathered block), from bit 0: block index, 2 bits level index, extra block of a narrow level (reference
+// compatibility), inert padding block, first column of the block counted from the start of the row's token stream in units
+// of the narrowest block (block_n / 8 tokens).  A row gathers at most block_n tokens per entry of its list (the extra blocks of
+// a level take less than two of its own entries leave), so a list of w entries needs columns below 8 w: 14 bits for the common
+// lists and 15 for the wide ones, whatever block_n.  The rest is the block index's.
+template <bool WIDE> struct Item {
+  static constexpr int kBlockBits = WIDE ? 13 : 14;
+  static constexpr int kColShift = kBlockBits + 4;
+  static constexpr uint32_t kBlockMask = (1u << kBlockBits) - 1, kQuirk = 4u << kBlockBits, kPad = 8u << kBlockBits;
+  static constexpr int kMaxBlocks = 1 << kBlockBits;
+  static_assert((WIDE ? kMaxWidthWide : kMaxWidth) * 8 <= 1 << (32 - kColShift), "columns of the longest list");
+  static __device__ __forceinline__ uint32_t make(int blk, int li, uint32_t flags, int col, int unit_shift) {
+    return ((uint32_t)blk & kBlockMask) | (uint32_t)li << kBlockBits | flags | (uint32_t)(col >> unit_shift) << kColShift;
+  }
+  static __device__ __forceinline__ int block(uint32_t x) { return (int)(x & kBlockMask); }
+  static __device__ __forceinline__ int level(uint32_t x) { return (int)(x >> kBlockBits) & 3; }
+  static __device__ __forceinline__ int tile(uint32_t x, int unit_shift) { return (int)(x >> (kColShift + 7 - unit_shift)); }
+  static __device__ __forceinline__ int col(uint32_t x, int unit_shift) { return (int)((x >> kColShift) << unit_shift) & 127; }   // in its tile
+};
 
 // IMG = true: K/V tiles use the image layout [8-row group][slab][8 rows][128 B] and are filled by linear bulk copies from
 // the tile-image buffers; IMG = false: [slab][128 rows][128 B] filled by tensor-map TMA boxes from row-major tensors.
 template <int D, int FMT, bool IMG, bool CAUSAL, bool FIXED, bool WIDE>
 __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_constant__ TmapPack maps, const TcParams p) {
   using C = Cfg<D, FIXED, WIDE>;
+  using I = Item<WIDE>;
   if (p.only_if && *p.only_if == 0) return;
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
@@ -274,6 +289,7 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
     const uint64_t kmap0 = reinterpret_cast<uint64_t>(&maps.k[0]), vmap0 = reinterpret_cast<uint64_t>(&maps.v[0]);
     const int n0 = (int)p.n[0], n1 = (int)p.n[1], n2 = (int)p.n[2], n3 = (int)p.n[3];
     const int ptid = threadIdx.x;                     // 0..95
+    const int unit_shift = 28 - __clz(p.bn);          // log2(block_n / 8)
     int g0 = 0, q_rows = 0, syncs = 0;
     bool ok = true;
     // The raw index list of a row is fetched (cp.async, 4 bytes per entry) long before it is decoded.
@@ -341,10 +357,10 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
         const bool quirk = p.quirk && P < p.tn && cnt >= 2;
         const int ib = n_items, tb = tokens;
         for (int e = ptid; e < cnt; e += kProducerThreads)
-          table[ib + e] = ((uint32_t)sRaw[start + e] & 0xfffu) | (uint32_t)li << 12 | ((uint32_t)((tb + e * P) >> 2) << 16);
+          table[ib + e] = I::make(sRaw[start + e], li, 0u, tb + e * P, unit_shift);
         if (quirk)
           for (int j = 2 + ptid; j < p.tn / P; j += kProducerThreads)
-            table[ib + cnt + j - 2] = (uint32_t)j | (uint32_t)li << 12 | kItemQuirk | ((uint32_t)((tb + (cnt + j - 2) * P) >> 2) << 16);
+            table[ib + cnt + j - 2] = I::make(j, li, I::kQuirk, tb + (cnt + j - 2) * P, unit_shift);
         const int items = cnt + (quirk ? p.tn / P - 2 : 0);
         qb[li] = quirk ? (float)li + log2f((float)(cnt / 2)) : 0.f;
         if (items > 0) last_P = P;
@@ -358,7 +374,7 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
       if (ptid == 0) {
         const int last_li = 31 - __clz(p.bn / last_P);
         for (int t = tokens; t < padded; t += last_P)
-          table[n_items++] = (uint32_t)last_li << 12 | kItemPad | ((uint32_t)(t >> 2) << 16);
+          table[n_items++] = I::make(0, last_li, I::kPad, t, unit_shift);
         Ctrl::RowDec& d = ctl->dec[rit_n & 1];
         d.n_items = n_items;
         d.n_tiles = n_tiles;
@@ -453,14 +469,14 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
             ready = __all_sync(0xffffffffu, ready);
             if (ready) {
             const int probe = vi + lane;
-            const int in_tile = __popc(__ballot_sync(0xffffffffu, probe < n_items && (int)(sIt[probe < n_items ? probe : 0] >> 21) == t));
+            const int in_tile = __popc(__ballot_sync(0xffffffffu, probe < n_items && I::tile(sIt[probe < n_items ? probe : 0], unit_shift) == t));
             if ((2 * gt + 1) % kProducerWarps == warp) {
             const uint32_t tile_a = sV_a + stage * C::TILE_BYTES, bar_a = v_full_a + stage * 8;
             const int mine = vi + lane;
             uint32_t my_bytes = 0;
             if (lane < in_tile) {
               const uint32_t x = sIt[mine];
-              const int li = (x >> 12) & 3, blk = x & 0xfff, P = p.bn >> li, col = ((int)(x >> 16) << 2) & 127;
+              const int li = I::level(x), blk = I::block(x), P = p.bn >> li, col = I::col(x, unit_shift);
               if (IMG) {
                 const unsigned char* src = p.vimg + p.img.off[li] + (((int64_t)bh * p.img.groups[li] + ((blk * P) >> 3)) * C::SLABS << 10);
                 tc::bulk_load_a(tile_a + (col >> 3) * (C::SLABS * 1024), src, (uint32_t)(P * D * 2), bar_a);
@@ -496,7 +512,7 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
               ready = __all_sync(0xffffffffu, ready);
               if (ready) {
             const int probe = ki + lane;
-            const int in_tile = __popc(__ballot_sync(0xffffffffu, probe < n_items && (int)(sIt[probe < n_items ? probe : 0] >> 21) == t));
+            const int in_tile = __popc(__ballot_sync(0xffffffffu, probe < n_items && I::tile(sIt[probe < n_items ? probe : 0], unit_shift) == t));
             // Every producer warp waits for every tile's stage, in order (a parity wait is only valid for a waiter at most
             // one phase ahead of its barrier), but ONE warp gathers the whole tile and the warps take turns: an mbarrier
             // arrive costs its thread ~250 cycles and a wait ~170, so three warps that each handle a third of every tile
@@ -507,13 +523,13 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
             float* biasg_row = sBiasG + slot * 36;
             const bool active = lane < in_tile;
             const uint32_t x = active ? sIt[ki + lane] : 0u;
-            const int li = (x >> 12) & 3, blk = x & 0xfff, P = p.bn >> li, col = ((int)(x >> 16) << 2) & 127, row0 = blk * P;
+            const int li = I::level(x), blk = I::block(x), P = p.bn >> li, col = I::col(x, unit_shift), row0 = blk * P;
             // logit bias of the block's columns
             const int nl = li == 0 ? n0 : (li == 1 ? n1 : (li == 2 ? n2 : n3));
             const float qb = li == 0 ? qb0 : (li == 1 ? qb1 : (li == 2 ? qb2 : qb3));
-            const float bias2 = (x & kItemPad) ? -INFINITY : ((x & kItemQuirk) ? qb : (float)li);
+            const float bias2 = (x & I::kPad) ? -INFINITY : ((x & I::kQuirk) ? qb : (float)li);
             const int nvalid = nl - row0;
-            const bool diag = CAUSAL && active && blk == m && !(x & (kItemPad | kItemQuirk));
+            const bool diag = CAUSAL && active && blk == m && !(x & (I::kPad | I::kQuirk));
             unsigned char* minrow_row = sMinRow + slot * 128;
             uint32_t my_bytes = 0;
             if (active) {
@@ -1110,6 +1126,7 @@ bool fwd_tc_supported(const FwdArgs& a) {
   if (a.bm != 128 || a.tn != 32) return false;
   if (a.D != 64 && a.D != 128) return false;
   if (a.width > (a.kimg || a.causal ? kMaxWidth : kMaxWidthWide)) return false;
+  if (cdiv64(a.seq_k, a.bn) > (a.width > kMaxWidth ? Item<true>::kMaxBlocks : Item<false>::kMaxBlocks)) return false;
   if (a.bh > 65535) return false;
   if (!(a.scale > 0.f)) return false;
   const void* ptrs[] = {a.q, a.out, a.k[0], a.k[1], a.k[2], a.k[3], a.v[0], a.v[1], a.v[2], a.v[3]};
