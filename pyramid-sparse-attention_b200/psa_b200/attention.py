@@ -128,10 +128,11 @@ class PSAAttention(nn.Module):
         else:
             self.sparse_attention_fn = sparse_attention_factory(self.config.block_m, self.config.tile_n,
                                                                 self.config.block_n)
+        self._own_attention_fn = self.sparse_attention_fn      # a caller may put another one in its place
 
     def forward(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, idx_q=None, idx_k=None) -> torch.Tensor:
         config = self.config
-        if ops.layer_supported(q, k, v, config):
+        if self.sparse_attention_fn is self._own_attention_fn and ops.layer_supported(q, k, v, config):
             if idx_q is None:
                 idx_q = ops.draw_sample_indices(q.shape[0], q.shape[1], config.block_m, config.block_m // 4, q.device)
             if idx_k is None:

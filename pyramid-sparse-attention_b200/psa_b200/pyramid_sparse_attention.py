@@ -131,6 +131,7 @@ class PyramidSparseAttention(nn.Module):
             self.sparse_attention_fn = sparse_attention_factory(config.block_m, config.tile_n, config.block_n)
         else:
             raise ValueError(f"Unknown attn_impl: {config.attn_impl}")
+        self._own_attention_fn = self.sparse_attention_fn      # a caller may put another one in its place
         self.logger = SparsityLog() if config.enable_logging else None
 
     def get_current_time(self):
@@ -230,8 +231,8 @@ class PyramidSparseAttention(nn.Module):
             perm = self.gilbert_rearranger.source_rows(q.device) if self.use_rearrange else None
             q_r, k_r, v_r = ops.gather_views(q, k, v, perm, rotary)
             c = self.config
-            if (perm is not None and c.attn_impl == "new_mask_type" and c.block_m == 128 and c.block_n == 32 and c.tile_n == 32
-                    and -(-k.shape[2] // c.block_n) + len(c.mask_ratios) <= 4096):
+            if (perm is not None and self.sparse_attention_fn is self._own_attention_fn and c.attn_impl == "new_mask_type"
+                    and c.block_m == 128 and c.block_n == 32 and c.tile_n == 32 and -(-k.shape[2] // c.block_n) + len(c.mask_ratios) <= 4096):
                 # ... and the way back is where the forward stores its rows
                 with torch.no_grad():
                     mask, _, _ = compute_block_mask(q_r, k_r, c, text_length=c.text_length)

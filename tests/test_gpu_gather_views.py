@@ -82,3 +82,24 @@ def test_what_the_copy_kernel_does_not_take_goes_the_old_way():
     assert not ops.views_supported(q, k, v[:, :, :32]) and not ops.views_supported(q.requires_grad_(), k, v)
     with torch.no_grad():
         assert ops.views_supported(q, k, v) and not ops.views_supported(q, k, v, _tables(65, 0, 64))
+
+
+def test_an_attention_function_put_in_place_of_the_modules_own_is_called():
+    from psa_b200.pyramid_sparse_attention import AttentionConfig, PyramidSparseAttention
+    cfg = AttentionConfig(width=12, height=8, depth=9, text_length=20, use_rearrange=True, rearrange_method="Gilbert", block_m=128, block_n=32,
+                          tile_n=32, use_sim_mask=False, mask_ratios=C.DEFAULT_RATIOS, mask_mode="topk", warmup_steps=0,
+                          attn_impl="new_mask_type")
+    mod = PyramidSparseAttention(cfg, inference_num=10, layer_num=1, model_type="cogvideo")
+    S = 12 * 8 * 9 + 20
+    q, k, v = (_layout(x.to(DEV), "token") for x in C.qkv(982, 1, 2, S, 128, torch.bfloat16, smooth=16))
+    rope = _tables(S, 20, 128)
+    torch.manual_seed(22)
+    plain = mod(q, k, v, 0, rotary=rope)
+    own, calls = mod.sparse_attention_fn, []
+
+    def negated(*args):
+        calls.append(args[3].shape)
+        return -own(*args)
+    mod.sparse_attention_fn = negated
+    torch.manual_seed(22)
+    assert torch.equal(mod(q, k, v, 0, rotary=rope), -plain) and len(calls) == 1

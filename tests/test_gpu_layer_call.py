@@ -50,3 +50,27 @@ def test_other_calls_take_the_single_entry_points():
     for mode, err in (("mass", ValueError), (None, Exception)):
         with pytest.raises(err):
             psa_b200.PSAAttention(psa_b200.PSAConfig(mask_mode=mode))(q, q, q)
+
+
+def test_an_attention_function_put_in_place_of_the_modules_own_is_called():
+    import psa_b200
+    from psa_b200 import ops
+    from psa_b200.attention import compute_block_mask
+    cfg = psa_b200.PSAConfig()
+    q, k, v = (x.to(DEV) for x in C.qkv(65, 1, 2, 1500, 64, torch.bfloat16))
+    iq, ik = C.sample_idx(9, 1, 2, 128, 32).to(DEV), C.sample_idx(10, 1, 2, 64, 16).to(DEV)
+    module = psa_b200.PSAAttention(cfg)
+    plain = module(q, k, v, idx_q=iq, idx_k=ik)
+    own, calls = module.sparse_attention_fn, []
+
+    def recorded(*args):
+        calls.append(args[3].shape)
+        return own(*args)
+    module.sparse_attention_fn = recorded
+    assert _same(module(q, k, v, idx_q=iq, idx_k=ik), plain) and len(calls) == 1
+    module.sparse_attention_fn = psa_b200.sparse_attention_factory(128, 32, 64, compat_quirk=False)
+    got = module(q, k, v, idx_q=iq, idx_k=ik)
+    mask, _, _ = compute_block_mask(q, k, cfg, idx_q=iq, idx_k=ik)
+    assert _same(got, ops.psa_forward(q, k, v, mask, 128, 64, 32, compat_quirk=False)) and not _same(got, plain)
+    module.sparse_attention_fn = own
+    assert _same(module(q, k, v, idx_q=iq, idx_k=ik), plain) and len(calls) == 1
