@@ -132,7 +132,8 @@ int psa_ksim(const void* k, int32_t* out, int64_t bh, int64_t seq, int head_dim,
  * A bf16 call is TWO launches of the tcgen05 kernel (an fp16 one is the second of them alone).  The first takes the probabilities of a query row
  * relative to the maximum of the row's first tile instead of a running maximum (same result: the factor cancels against
  * the row sum; bf16 probabilities and the fp32 sum have the exponent range for it), which saves the maximum pass and
- * the rescaling; a row whose sum leaves the safe range sets a guard word (another slot of the counter ring).  The
+ * the rescaling; a row whose sum leaves the safe range, or whose accumulated values are not finite, sets a guard word
+ * (another slot of the counter ring).  The
  * second launch is the running-maximum kernel: it reads the guard word, returns at once if it is zero and recomputes
  * the call otherwise.  Both are ordered on `stream`; nothing is read back by the host.  A bf16 call therefore takes THREE
  * words of the ring (two row counters and the guard word): about 85 such calls may be in flight on one device before words are

@@ -47,8 +47,9 @@
 // score buffer fits at head_dim 128 as well, and the row's end needs only the two sums.  With the causal rule a row sees a
 // key of its first tile or none at all: only the diagonal block hides keys; at level 1 it shows every row at least one, and
 // at the other levels it fills half a tile at most, with any other block of the row packed beside it.
-// A row whose sum of probabilities exceeds 2^90, or is NaN, sets a guard word; the exact kernel is launched right behind on the
-// same stream and returns at once unless that word is set, in which case it redoes the call.
+// A row whose sum of probabilities exceeds 2^90 or is NaN, or whose accumulated values are not all finite (probabilities above 1
+// times values beyond 2^37 can overflow fp32 where probabilities of at most 2^8 do not), sets a guard word; the exact kernel is
+// launched right behind on the same stream and returns at once unless that word is set, in which case it redoes the call.
 //
 // Every wait is bounded - mbarrier waits, the issuer's polling loop and the warp-group rendezvous (mbarriers, never
 // bar.sync, inside the role loops); on expiry the CTA records PSA_ERR_TIMEOUT in the status word, lets copies in
@@ -1003,7 +1004,6 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
         const bool dead = p.legacy && (FIXED ? l_all == 0.f : m_all == -INFINITY);
         const float inv = dead ? 0.f : 1.0f / l_all;              // otherwise an empty row is 0/0 like the reference
         const float w = w_me * inv, wo = w_ot * inv;
-        if (FIXED && p.guard && !(l_all < kSumMax) && qrow < p.seq_q) *p.guard = 1;   // near the end of the exponent range (or NaN)
         if (p.lse && g == 0 && qrow < p.seq_q)
           p.lse[(int64_t)bh * p.seq_q + qrow] = dead ? -INFINITY : (m_all + log2f(l_all)) * 0.6931471805599453f;
         const bool other_has = !FIXED && n_tiles - my_tiles > 0;
@@ -1024,6 +1024,14 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
         tc::tc_fence_before();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&ctl->o_free);
+        if (FIXED && p.guard) {
+          // the sum near the end of the exponent range (or NaN), or a product of such probabilities with large values past it
+          float z[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int i = 0; i < HALF; ++i) z[i & 3] = fmaf(f[i], 0.f, z[i & 3]);      // NaN if any value is not finite
+          const bool finite = (z[0] + z[1]) + (z[2] + z[3]) == 0.f;
+          if (!(l_all < kSumMax && finite) && qrow < p.seq_q) *p.guard = 1;
+        }
         // A thread holds HALF channels of its own row; stored as they are, every store instruction of a warp would touch 32
         // different 128-byte lines.  The 16-byte pieces are transposed inside groups of 8 lanes first (three butterfly
         // stages), so that 8 lanes write one row's contiguous 128 bytes.

@@ -579,3 +579,34 @@ def test_legacy_rows_far_above_their_first_tile(P, D, dt, octaves, causal):
     assert torch.equal(torch.isinf(lse), dead) and float(o[dead].abs().sum()) == 0.0
     # scores of one key are exact to an fp32 rounding of a sum of D products; the sum behind the logarithm to 2^-8
     assert float((lse - ref_lse)[~dead].abs().max()) <= 2e-2
+
+
+@pytest.mark.parametrize("kind", ["images", "rows", "legacy", "legacy causal"])
+@pytest.mark.parametrize("D", [64, 128])
+def test_large_values_under_scores_far_above_a_rows_first_tile(P, D, kind):
+    """One key 75 octaves above its row's first tile keeps the sum of the probabilities in range, but times values of 2^60 the
+    fp32 accumulator is not: the call must go to the exact kernel."""
+    S, lead, big = 640, 350, 2.0 ** 60
+    g = torch.Generator().manual_seed(79)
+    q, k = 0.1 * torch.randn(1, 2, S, D, generator=g), 0.1 * torch.randn(1, 2, S, D, generator=g)
+    v = (torch.randn(1, 2, S, D, generator=g) * big).to(torch.bfloat16)
+    q[..., 0] = 40.0
+    k[0, 0, lead, 0] = 75 * 0.6931 * D ** 0.5 / 40.0
+    q, k = q.to(torch.bfloat16), k.to(torch.bfloat16)
+    nk = S // 128
+    if kind.startswith("legacy"):
+        causal = kind.endswith("causal")
+        mask = torch.ones(1, 2, nk, nk, dtype=torch.int32)
+        out = P.ops.legacy_forward(q.to(DEV), k.to(DEV), v.to(DEV), mask.to(DEV), causal)[0]
+        ref = O.legacy_forward(q, k, v, mask, causal)[0]
+    else:
+        row = torch.tensor([*range(nk), -1, -1, -1, -1], dtype=torch.int32)
+        mask = row.expand(1, 2, nk, nk + 4).contiguous()
+        dev = [x.to(DEV) for x in (q, k, v)]
+        pyramid = P.ops.pyramid_kv(*dev[1:], 128) if kind == "rows" else None
+        out = P.ops.psa_forward(*dev, mask.to(DEV), 128, 128, 32, pyramid=pyramid)
+        ref = O.psa_forward_newmask(q, k, v, mask, 128, 128, 32)
+    assert int(out._psa_status.item()) == 0
+    out, ref = out.float().cpu() / big, ref.float() / big
+    assert torch.isfinite(out).all()
+    assert float((out - ref).abs().max()) <= ATOL_OUT and cosine(out, ref) >= COS_OUT
