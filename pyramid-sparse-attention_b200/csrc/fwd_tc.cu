@@ -47,9 +47,10 @@
 // score buffer fits at head_dim 128 as well, and the row's end needs only the two sums.  With the causal rule a row sees a
 // key of its first tile or none at all: only the diagonal block hides keys; at level 1 it shows every row at least one, and
 // at the other levels it fills half a tile at most, with any other block of the row packed beside it.
-// A row whose sum of probabilities exceeds 2^90 or is NaN, or whose accumulated values are not all finite (probabilities above 1
-// times values beyond 2^37 can overflow fp32 where probabilities of at most 2^8 do not), sets a guard word; the exact kernel is
-// launched right behind on the same stream and returns at once unless that word is set, in which case it redoes the call.
+// A row whose sum of probabilities exceeds 2^90, is below 2^-60 or is NaN, or whose accumulated values are not all finite
+// (probabilities above 1 times values beyond 2^37 can overflow fp32 where probabilities of at most 2^8 do not), sets a guard
+// word; the exact kernel is launched right behind on the same stream and returns at once unless that word is set, in which case
+// it redoes the call.
 //
 // Every wait is bounded - mbarrier waits, the issuer's polling loop and the warp-group rendezvous (mbarriers, never
 // bar.sync, inside the role loops); on expiry the CTA records PSA_ERR_TIMEOUT in the status word, lets copies in
@@ -735,7 +736,7 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
     bool ok = true;
     int g0 = 0, q_rows = 0, pv_rows = 0;
     float* sMref = sXch + 1024;                   // fixed reference: [row & 3][128], behind the exchange area
-    constexpr float kSumMax = 1.2379400e27f;      // 2^90
+    constexpr float kSumMax = 1.2379400e27f, kSumMin = 8.6736174e-19f;      // 2^90, 2^-60
     for (int rit = 0; ok; ++rit) {
       const int rslot = rit & 3;
       ok = tc::mbar_wait(&ctl->row_ready[rslot], (rit >> 2) & 1, abort_flag);
@@ -1025,12 +1026,14 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&ctl->o_free);
         if (FIXED && p.guard) {
-          // the sum near the end of the exponent range (or NaN), or a product of such probabilities with large values past it
+          // The sum near the end of the exponent range (or NaN), or a product of such probabilities with large values past it.
+          // A sum far below 1: every score of the first tile was -inf, which leaves the reference at 0 (a row of one tile
+          // is then a row without a key in the exact kernel as well).
           float z[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
           for (int i = 0; i < HALF; ++i) z[i & 3] = fmaf(f[i], 0.f, z[i & 3]);      // NaN if any value is not finite
           const bool finite = (z[0] + z[1]) + (z[2] + z[3]) == 0.f;
-          if (!(l_all < kSumMax && finite) && qrow < p.seq_q) *p.guard = 1;
+          if (!(l_all < kSumMax && (l_all > kSumMin || n_tiles == 1) && finite) && qrow < p.seq_q) *p.guard = 1;
         }
         // A thread holds HALF channels of its own row; stored as they are, every store instruction of a warp would touch 32
         // different 128-byte lines.  The 16-byte pieces are transposed inside groups of 8 lanes first (three butterfly

@@ -610,3 +610,29 @@ def test_large_values_under_scores_far_above_a_rows_first_tile(P, D, kind):
     out, ref = out.float().cpu() / big, ref.float() / big
     assert torch.isfinite(out).all()
     assert float((out - ref).abs().max()) <= ATOL_OUT and cosine(out, ref) >= COS_OUT
+
+
+@pytest.mark.parametrize("causal", [False, True], ids=["full", "causal"])
+@pytest.mark.parametrize("D", [64, 128])
+def test_rows_whose_first_tile_has_no_finite_score(P, D, causal):
+    """The keys of block 0 score -inf (the product overflows), those of the others around -360 octaves: a row that sees others is
+    their softmax, a row that sees block 0 alone has no key."""
+    S = 640
+    g = torch.Generator().manual_seed(80)
+    q, k = 0.1 * torch.randn(1, 2, S, D, generator=g), 0.1 * torch.randn(1, 2, S, D, generator=g)
+    v = torch.randn(1, 2, S, D, generator=g)
+    q[..., 0] = 2e19
+    k[..., :128, 0] = -1e20
+    k[..., 128:, 0] = -1e-16 * D ** 0.5 / 8 * (1 + torch.randint(0, 4, (1, 2, S - 128), generator=g) / 128)
+    q, k, v = (x.to(torch.bfloat16) for x in (q, k, v))
+    mask = torch.ones(1, 2, S // 128, S // 128, dtype=torch.int32)
+    o, lse, _ = P.ops.legacy_forward(q.to(DEV), k.to(DEV), v.to(DEV), mask.to(DEV), causal, need_lse=True)
+    assert int(o._psa_status.item()) == 0
+    ref, ref_lse = O.legacy_forward(q, k, v, mask, causal)
+    o, lse, ref, ref_lse = o.float().cpu(), lse.cpu(), ref.float(), ref_lse.float()
+    lead = 128 if causal else 0
+    assert torch.equal(torch.isinf(lse), (torch.arange(S) < lead).expand(1, 2, S)) and float(o[:, :, :lead].abs().sum()) == 0.0
+    o, lse, ref, ref_lse = (x[:, :, lead:] for x in (o, lse, ref, ref_lse))
+    assert float((o - ref).abs().max()) <= ATOL_OUT and cosine(o, ref) >= COS_OUT
+    # scores of -250: fp32 sums of D products, the largest 250 (rounded to 2^-16 of it in the last place)
+    assert float((lse - ref_lse).abs().max()) <= 2e-2
