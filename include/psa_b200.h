@@ -276,8 +276,9 @@ int psa_gather_views(const void* const* src, const int64_t* strides, const int32
  * i sees groups j <= i, else all groups of the padded length; out [BH, nb, nb] (dtype), nb = ceil(seq/block_size) =
  * softmax mass per (query block, key block).  block_size/stride must be a power of two in 2..32.
  * scratch: psa_antidiag_scratch_bytes() bytes (the fp32 logits), 16-byte aligned.
- * psa_antidiag_scores_impl: impl 0 = pick (the tcgen05 kernel when seq is a multiple of stride, else the warp-level
- * mma.sync kernel), 2 = tcgen05 (PSA_ERR_UNSUPPORTED otherwise), 3 = mma.sync; status (may be NULL): device word that
+ * psa_antidiag_scores_impl: impl 0 = pick (the tcgen05 kernel when seq holds at least one group of stride tokens, else the
+ * warp-level mma.sync kernel), 2 = tcgen05, for lengths that are a multiple of stride only (PSA_ERR_UNSUPPORTED
+ * otherwise, although 0 takes that kernel for other lengths too), 3 = mma.sync; status (may be NULL): device word that
  * receives PSA_ERR_TIMEOUT if a bounded wait of the tcgen05 kernel expires (the output is then incomplete). */
 size_t psa_antidiag_scratch_bytes(int64_t bh, int64_t seq, int head_dim, int block_size, int stride, int chunk_size);
 int psa_antidiag_scores(const void* q, const void* k, void* out, void* scratch, size_t scratch_bytes, int64_t bh, int64_t seq,

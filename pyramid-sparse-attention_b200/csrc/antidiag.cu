@@ -249,7 +249,8 @@ extern "C" int psa_antidiag_scores_impl(const void* q, const void* k, void* out,
   dim3 grid2((unsigned)d.nb, (unsigned)bh);
   const bool tc_ok = antidiag_tc_supported(seq, head_dim, stride, d.n, dtype);
   PSA_REQUIRE(impl != 2 || (tc_ok && seq % stride == 0), PSA_ERR_UNSUPPORTED,
-              "psa_antidiag_scores: the tcgen05 kernel needs a length that is a multiple of the stride (seq=%lld, stride=%d)",
+              "psa_antidiag_scores: impl 2 takes lengths that are a multiple of the stride only (seq=%lld, stride=%d); impl 0 picks "
+              "the tcgen05 kernel for other lengths of at least one stride",
               (long long)seq, stride);
   const bool use_tc = tc_ok && impl != 3;
   if (use_tc)      // GEMM with a partial softmax in its epilogue, then a small combine kernel: no logits in HBM

@@ -471,7 +471,7 @@ def antidiag_block_scores(q, k, block_size: int, stride: int, chunk_size: int, c
                           impl: int = 0) -> torch.Tensor:
     """Antidiagonal block-importance estimate [B, H, nb, nb] (q.dtype), nb = ceil(L/block_size): estimate_block_importance
     with select_mode='inverse' (qwen2.5-vl-example/src/attention/PSA_casual/utils/block_importance.py:282-562).
-    impl: 0 pick (tcgen05 GEMM when L is a multiple of stride), IMPL_TENSOR, IMPL_WARP_MMA."""
+    impl: 0 pick (tcgen05 GEMM when L >= stride), IMPL_TENSOR (multiples of stride only), IMPL_WARP_MMA."""
     _need_cuda(q, k)
     q, k = _flat_bh(q), _flat_bh(k)
     B, H, L, D = q.shape
