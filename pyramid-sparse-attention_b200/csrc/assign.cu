@@ -235,7 +235,11 @@ __global__ void __launch_bounds__(256) assign_levels_kernel(const T* __restrict_
 // (match.any) and take their rank from the warp's running counter of that digit, the counters of all warps are summed up
 // digit by digit, and every word is written to its place.  Instruction-bound: 2 x ~25 instructions per 32 words and no
 // padding to a power of two.  (A bitonic network in registers needs 66 exchange stages for 2048 words.)  23640 rows of 1182
-// blocks: 850 -> 364 us; 5040 rows of 840: 272 -> 103 us; 10240 rows of 256 with running sums: 208 -> 101 us.
+// blocks: 850 -> 330 us; 5040 rows of 840: 272 -> 103 us; 10240 rows of 256 with running sums: 208 -> 101 us.
+// E: the steps a warp holds in registers.  It only has to be large enough (the loops end at the row's own steps), so there is one
+// instance per number of blocks that fit an SM: 40 registers and six up to E = 6, 48 and five up to 12, 62 and four at 16.  Rows
+// of 256 / 840 / 1182 blocks take 102 / 129 / 330 us with E = 6 (as with their own 1 / 4 / 5: 102 / 129 / 328), 111 / 135 / 336
+// with 12 and 119 / 146 / 364 with 16 (20000 / 12000 / 23640 rows); rows of 2048 take 194 us with 12 or their own 8, 198 with 16.
 template <typename T, int E>
 __global__ void __launch_bounds__(256) assign_levels_radix_kernel(const T* __restrict__ po, int32_t* __restrict__ mask,
                                                                  AssignParams p) {
@@ -409,8 +413,7 @@ static int launch_assign(const void* po, int32_t* mask, int64_t rows, AssignPara
   } while (0)
 #define PSA_ASSIGN_RADIX_E(TT)                                                                                  \
   do {                                                                                                         \
-    if (steps <= 2) PSA_ASSIGN_RADIX(TT, 2); else if (steps <= 5) PSA_ASSIGN_RADIX(TT, 5);                      \
-    else if (steps <= 8) PSA_ASSIGN_RADIX(TT, 8); else PSA_ASSIGN_RADIX(TT, 16);                                \
+    if (steps <= 6) PSA_ASSIGN_RADIX(TT, 6); else if (steps <= 12) PSA_ASSIGN_RADIX(TT, 12); else PSA_ASSIGN_RADIX(TT, 16); \
   } while (0)
     if (dtype == PSA_F16) PSA_ASSIGN_RADIX_E(__half); else PSA_ASSIGN_RADIX_E(__nv_bfloat16);
 #undef PSA_ASSIGN_RADIX_E

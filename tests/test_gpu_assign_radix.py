@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
-@pytest.mark.parametrize("nk", [2, 31, 33, 255, 256, 257, 512, 513, 1280, 1281, 2048, 2049, 4095, 4096, 4097])
+@pytest.mark.parametrize("nk", [2, 31, 33, 255, 256, 257, 512, 513, 1280, 1281, 1536, 1537, 2048, 2049, 3072, 3073, 4095, 4096, 4097])
 @pytest.mark.parametrize("dt,mode", [(torch.bfloat16, "topk_newtype"), (torch.float16, "thresholdbound_newtype"),
                                      (torch.bfloat16, "thresholdbound"), (torch.float32, "thresholdbound")])
 def test_row_lengths(nk, dt, mode):
