@@ -12,7 +12,9 @@
 namespace psa {
 namespace {
 
-// dst[bh][t][:] = src[bh][perm[t]][:], rows of cpr 16-byte words.
+// The four kernels up to gather_heads_rope_kernel take rows of any whole number cpr of 16-byte words: fp32 rows, and 16-bit
+// rows of other widths than the 64 and 128 channels that gather_views_kernel below is made for.
+// dst[bh][t][:] = src[bh][perm[t]][:].
 __global__ void __launch_bounds__(256) gather_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ perm,
                                                           uint4* __restrict__ dst, int64_t seq, int cpr) {
   const int64_t bh = blockIdx.y;

@@ -114,8 +114,8 @@ struct alignas(VEC * sizeof(T)) CellPack { T e[VEC]; };
 
 // VEC neighbouring cells per thread and load; the launcher picks the widest VEC (<= 16 bytes) that divides n_d.
 // HBM-bound (R is read once).  The block has as many threads as there are packs to load (up to 512, in equal shares beyond):
-// with 256 for every size, half of them idled at 32k tokens (128 packs) and a second pass ran at an eighth at 75k (296).  12 x 32760 tokens: 44 -> 28 us, 40 x 32760 (blocks of 128): 125 -> 48 us,
-// 40 x 75600: 600 -> 316 us.  (512, 2): without the second bound the compiler keeps to 40 registers, too few for eight
+// with 256 for every size, half of them idled at 32k tokens (128 packs) and a second pass ran at an eighth at 75k (296).
+// 12 x 32760 tokens: 44 -> 28 us, 40 x 32760 (blocks of 128): 125 -> 48 us, 40 x 75600: 600 -> 316 us.  (512, 2): without the second bound the compiler keeps to 40 registers, too few for eight
 // 16-byte loads in flight, and the last figure is 520 us.
 // SUM: the cells one partial sum takes at a time (the widest VEC <= 8 bytes; the order of the row sum does not follow VEC).
 template <typename T, int VEC, int SUM = VEC>

@@ -197,8 +197,9 @@ class PyramidSparseAttention(nn.Module):
     fuses_rotary = True       # forward() takes rotary=..., so a processor may hand over unrotated q and k
 
     def forward(self, q, k, v, layer_idx, rotary=None):
-        """q, k, v [B, H, S, D].  rotary (ops.RotaryTables, optional): q and k arrive unrotated; on the token-major route
-        the kernels rotate the rows as they read them, on every other route they are rotated here first."""
+        """q, k, v [B, H, S, D].  rotary (ops.RotaryTables, optional): q and k arrive unrotated.  The kernels rotate the rows as
+        they read them, or the copy that lays the operands out does; warm-up steps and tensors that neither takes (fp32, a
+        gradient, a sequence that is not the reordered grid) are rotated here first."""
         is_warmup = self.get_current_time() < self.config.warmup_steps
         if rotary is not None:
             # the in-place routes (token-major views or head-major tensors) rotate inside their loads, the others inside the

@@ -47,9 +47,11 @@ def test_other_calls_take_the_single_entry_points():
     assert not ops.layer_supported(q, q, q, psa_b200.PSAConfig(block_n=32))
     assert not ops.layer_supported(q, q[:, :1], q[:, :1], psa_b200.PSAConfig())
     assert not ops.layer_supported(q, q, q, psa_b200.PSAConfig(attn_impl="old_mask_type", block_n=128))
-    for mode, err in (("mass", ValueError), (None, Exception)):
-        with pytest.raises(err):
-            psa_b200.PSAAttention(psa_b200.PSAConfig(mask_mode=mode))(q, q, q)
+    for mode in ("mass", None):
+        cfg = psa_b200.PSAConfig(mask_mode=mode)
+        assert not ops.layer_supported(q, q, q, cfg)
+        with pytest.raises(ValueError, match=f"Unknown mode: {mode}_newtype"):      # the error of the single entry point
+            psa_b200.PSAAttention(cfg)(q, q, q)
 
 
 def test_an_attention_function_put_in_place_of_the_modules_own_is_called():

@@ -134,3 +134,17 @@ def test_cogvideox_processor_hands_unrotated_head_major_rows_to_the_module(monke
     ops.check_status()
     assert fused_calls == [True, False], fused_calls
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D,first,reorder", [(32, 3, True), (96, 0, False), (256, 40, True)])
+def test_row_copies_of_other_widths_rotate_alike(dtype, D, first, reorder):
+    """16-bit rows of a width that the wide copy kernel is not made for."""
+    from psa_b200 import ops
+    x = C.randn(90, (2, 3, 500, D), dtype, smooth=4).to(DEV)
+    rope = ops.RotaryTables(*_tables(500, first, D, 9), first)
+    perm = torch.randperm(500, generator=torch.Generator().manual_seed(6)).to(torch.int32).to(DEV) if reorder else None
+    want = ops.rotate_rows(x, rope)
+    want = want if perm is None else want[:, :, perm.long()]
+    assert torch.equal(ops.gather_rows(x, perm, rope=rope), want)
+    assert torch.equal(ops.gather_heads(x[0].transpose(0, 1).contiguous(), perm, rope=rope), want[:1])
