@@ -1,6 +1,6 @@
 // Multi-level block-sparse flash-attention forward on tcgen05 tensor cores (f16/bf16, block_m = 128).
 //
-// Persistent CTAs, one per SM (221 KB of shared memory and all 512 TMEM columns each), 12 warps.  A CTA starts with query
+// Persistent CTAs, one per SM (224 KB of shared memory and all 512 TMEM columns each), 12 warps.  A CTA starts with query
 // row R = blockIdx.x (R = batch*head * Mq + query block) and claims further rows from a global counter; its roles run the
 // rows as ONE continuous stream of 128-token tiles: ring stages, score buffers and barrier phases are indexed by the
 // running tile count, so nothing is drained between rows.
@@ -1206,7 +1206,7 @@ static int launch_tc(const FwdArgs& a, cudaStream_t st, int* row_counter, int* g
   cudaError_t e = cudaFuncSetAttribute(psa_fwd_tc_kernel<D, FMT, IMG, CAUSAL, FIXED, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
   PSA_REQUIRE(e == cudaSuccess, PSA_ERR_CUDA, "psa_fwd: shared-memory opt-in (%d B) failed: %s", C::SMEM_BYTES,
               cudaGetErrorString(e));
-  // persistent: one CTA per SM (221 KB of shared memory and all 512 TMEM columns each), rows dealt round-robin so that
+  // persistent: one CTA per SM (224 KB of shared memory and all 512 TMEM columns each), rows dealt round-robin so that
   // the CTAs running at the same time work on neighbouring rows of the same head (K/V stay in L2)
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
