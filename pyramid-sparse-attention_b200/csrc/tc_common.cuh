@@ -36,6 +36,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // the caller then leaves its role loop.  Every try_wait may itself block for a hardware-defined slice, so the
 // limit of 1<<22 polls is of the order of a second.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+#pragma unroll 1
   for (uint32_t it = 0; it < (1u << 22); ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((it & 63) == 63 && *abort_flag) return false;
@@ -193,6 +194,7 @@ __device__ __forceinline__ bool mbar_test_wait_a(uint32_t bar, uint32_t parity) 
   return ok != 0;
 }
 __device__ __forceinline__ bool mbar_wait_a(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+#pragma unroll 1
   for (uint32_t it = 0; it < (1u << 22); ++it) {
     if (mbar_try_wait_a(bar, parity)) return true;
     if ((it & 63) == 63 && *abort_flag) return false;
