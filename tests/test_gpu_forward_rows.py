@@ -1,0 +1,95 @@
+"""GPU: the tcgen05 forward at the ends of its rows - rows of 0 to 6 tiles of 128 columns in every order, so that each softmax group
+finishes rows and starts the next ones early; last tiles of every width; an output that is 16- but not 32-byte aligned; blocks
+that no row selects and that hold values that are not finite; first keys far below the rest of the first tile.  Yardstick: the
+scalar kernel on the same 16-bit inputs."""
+import pytest
+import torch
+
+import cases as C
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _mask(nk, bn, mq, heads, seed, avoid=()):
+    """Rows that select 0 to 6 tiles' worth of blocks, at random levels."""
+    g = torch.Generator().manual_seed(seed)
+    mask = torch.zeros((1, heads, mq, nk + 5), dtype=torch.int32)
+    usable = torch.tensor([b for b in range(nk) if b not in avoid], dtype=torch.int32)
+    for h in range(heads):
+        for r in range(mq):
+            budget = int(torch.randint(0, 7, (1,), generator=g)) * 128 - int(torch.randint(0, 128, (1,), generator=g))
+            blocks = usable[torch.randperm(len(usable), generator=g)].tolist()
+            share = torch.rand(4, generator=g) * (torch.rand(4, generator=g) < 0.7)
+            row, at = [], 0
+            for li in range(4):
+                n = max(0, int(budget * float(share[li]) / max(1e-6, float(share.sum())) / (bn >> li)))
+                n = min(n, len(blocks) - at)
+                row += blocks[at:at + n] + [-1]
+                at += n
+            mask[0, h, r, :len(row)] = torch.tensor(row, dtype=torch.int32)
+    return mask.to(DEV)
+
+
+def _close(a, b):
+    """Probabilities and results rounded to 8 (bf16) or 11 bits by both; a probability relative to another reference rounds anew."""
+    a, b = a.float(), b.float()
+    assert torch.equal(torch.isnan(a), torch.isnan(b))
+    a, b = a.nan_to_num(), b.nan_to_num()
+    assert float((a - b).abs().max()) <= 2e-2 * max(1.0, float(b.abs().max())) and float((a - b).norm()) <= 1e-2 * float(b.norm())
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("D,bn", [(128, 64), (64, 64), (128, 128), (64, 128), (128, 32), (64, 32)])
+def test_short_rows_in_every_order(D, bn, dt):
+    from psa_b200 import ops
+    heads, mq, nk = 6, 70, 1024 // bn + 9
+    S = nk * bn - 3
+    k, v = (C.randn(900 + i, (1, heads, S, D), dt).to(DEV) for i in range(2))
+    q = C.randn(903, (1, heads, mq * 128 - 5, D), dt).to(DEV)
+    mask = _mask(nk, bn, mq, heads, 10 * bn + D)
+    out = torch.full((q.numel() + 8,), 7.0, dtype=dt, device=DEV)[8:].view(q.shape)
+    assert out.data_ptr() % 32 == 16
+    tc = ops.psa_forward(q, k, v, mask, 128, bn, 32, out=out)
+    assert int(tc._psa_status.item()) == 0
+    sc = ops.psa_forward(q, k, v, mask, 128, bn, 32, impl=ops.IMPL_SCALAR)
+    _close(tc, sc)
+    again = ops.psa_forward(q, k, v, mask, 128, bn, 32)
+    assert again.data_ptr() % 32 == 0
+    _close(again, sc)
+
+
+@pytest.mark.parametrize("bn", [32, 64, 128])
+def test_blocks_that_no_row_selects_may_hold_anything(bn):
+    from psa_b200 import ops
+    heads, mq, nk, D = 2, 40, 1024 // bn + 9, 128
+    S = nk * bn
+    bad = (0, 2, 3, 5)      # block 0 and those that narrow levels pair up with (2, 3 at most)
+    k, v = (C.randn(910 + i, (1, heads, S, D), torch.bfloat16).to(DEV) for i in range(2))
+    q = C.randn(913, (1, heads, mq * 128, D), torch.bfloat16).to(DEV)
+    mask = _mask(nk, bn, mq, heads, bn, avoid=bad)
+    clean = ops.psa_forward(q, k, v, mask, 128, bn, 32, compat_quirk=False)
+    for b, x in zip(bad, (float("inf"), float("nan"), float("-inf"), float("inf"))):
+        k[:, :, b * bn:(b + 1) * bn] = x
+        v[:, :, b * bn:(b + 1) * bn] = x
+    dirty = ops.psa_forward(q, k, v, mask, 128, bn, 32, compat_quirk=False)
+    assert torch.equal(torch.nan_to_num(clean.float(), nan=3.0), torch.nan_to_num(dirty.float(), nan=3.0))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_first_keys_far_below_the_rest_of_the_first_tile(D):
+    from psa_b200 import ops
+    nk, bn, heads = 8, 64, 2
+    S = nk * bn
+    q, k, v = (C.randn(920 + i, (1, heads, S, D), torch.bfloat16).to(DEV) for i in range(3))
+    for octaves in (20, 300):      # inside the range that one reference covers, and past it
+        q[..., 0] = 16.0
+        k[..., 0] = 0.0
+        k[:, :, :32, 0] = -octaves * 0.6931 * D ** 0.5 / 16.0
+        mask = torch.zeros((1, heads, S // 128, nk + 5), dtype=torch.int32, device=DEV)
+        mask[..., :nk] = torch.arange(nk, device=DEV, dtype=torch.int32)
+        mask[..., nk:nk + 4] = -1
+        tc = ops.psa_forward(q, k, v, mask, 128, bn, 32)
+        sc = ops.psa_forward(q, k, v, mask, 128, bn, 32, impl=ops.IMPL_SCALAR)
+        assert int(tc._psa_status.item()) == 0
+        _close(tc, sc)
