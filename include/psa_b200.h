@@ -103,6 +103,11 @@ int psa_assign_levels(const void* po, int32_t* mask, int64_t rows, int nk, int d
                       const int32_t* ends, const float* thresholds, const int32_t* aligns, int min_index,
                       int text_blocks, void* stream);
 
+/* Sample offsets.  Replaces the torch.topk of _random_sample_tokens, src/psa_triton/attention.py:132-133: idx[row][0..keep) =
+ * positions of the `keep` largest of the row's `block` (<= 128) random numbers in [0, 1), largest first, equal ones by ascending
+ * position.  random: float32 [rows][block]; idx: int64 [rows][keep]. */
+int psa_draw_samples(const float* random, int64_t* idx, int64_t rows, int block, int keep, void* stream);
+
 /* Mask density.  Replaces calc_density_newtype / calc_density,
  * src/psa_triton/utils/transfer_attn_to_mask.py:510-622.  per_bh: float32 [BH], the mean density of
  * each (batch, head); no host synchronisation. */

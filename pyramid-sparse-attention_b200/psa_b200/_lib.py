@@ -70,6 +70,7 @@ SIGNATURES = {
     "psa_block_scores_static_capacity": (_sz, []),
     "psa_block_scores_static": (_i, [_p] * 5 + [_i64, _i64, _i64, _i, _i, _i, _i, _i, _p]),
     "psa_assign_levels": (_i, [_p, _p, _i64, _i, _i, _i, _i, _i, _p, _p, _p, _p, _p, _i, _i, _p]),
+    "psa_draw_samples": (_i, [_p, _p, _i64, _i, _i, _p]),
     "psa_density": (_i, [_p, _p, _i64, _i64, _i, _i, _p]),
     "psa_ksim": (_i, [_p, _p, _i64, _i64, _i, _i, _f, _f, _f, _i, _p]),
     "psa_ksim_perm": (_i, [_p, _p, _p, _i64, _i64, _i, _i, _f, _f, _f, _i, _p]),

@@ -333,11 +333,17 @@ def psa_forward_tm(q_heads, images: KVImages, mask, out_tm, block_m: int, block_
 
 
 def draw_sample_indices(B: int, H: int, block: int, keep: int, device) -> torch.Tensor:
-    """topk(rand(B,H,1,block), keep).indices: the same two torch calls, in the same order on the same
-    generator, as _random_sample_tokens (src/psa_triton/attention.py:132-133)."""
+    """topk(rand(B,H,1,block), keep).indices, as _random_sample_tokens draws them (src/psa_triton/attention.py:132-133): the
+    numbers come from the same torch call on the same generator, their selection on a GPU is one kernel of the library."""
     rand_vals = torch.rand(B, H, 1, block, device=device)
-    _, idx = torch.topk(rand_vals, keep, dim=3)
-    return idx.view(B, H, keep)
+    if rand_vals.device.type != "cuda" or rand_vals.dtype != torch.float32 or not 0 < keep <= block <= 128 or B * H == 0:
+        _, idx = torch.topk(rand_vals, keep, dim=3)
+        return idx.view(B, H, keep)
+    with _on(rand_vals):
+        idx = torch.empty((B, H, keep), dtype=torch.int64, device=rand_vals.device)
+        rc = lib.psa_draw_samples(_ptr(rand_vals), _ptr(idx), B * H, block, keep, _stream(rand_vals))
+    check(rc, "psa_draw_samples")
+    return idx
 
 
 def block_scores(q, k, idx_q, idx_k, block_m: int, block_n: int, impl: int = IMPL_AUTO, perm_q=None, perm_k=None,
