@@ -103,7 +103,7 @@ struct TcParams {
 // FIXED: the reference exponent of a query row is the maximum of its FIRST tile and is never raised (see the head of the
 // file).  No maximum pass after the first tile, no rescaling of the accumulator, hence ONE accumulator for both softmax
 // groups and room for a third score buffer.
-template <int D, bool FIXED = false> struct Cfg {
+template <int D, bool FIXED = false, bool CAUSAL = false> struct Cfg {
   static constexpr int SLABS = D / 64;
   static constexpr int NK = D == 64 ? 4 : 3;                 // K-tile ring
   static constexpr int NV = D == 64 ? 4 : FIXED ? 3 : 2;     // V-tile ring
@@ -115,6 +115,11 @@ template <int D, bool FIXED = false> struct Cfg {
   // Two score buffers: one thread issues both products, in the order QK0 QK1 PV0 QK2 PV1 ..., so that Q K^T follows the product
   // that frees its buffer at once.  Three: one thread for each, neither of which ever waits behind the other's barriers.
   static constexpr bool ONE_ISSUER = NSB == 2;
+  // A whole tile's MMAs one after the other in the code, or as a loop.  Unrolled, the eight of P V take 718 cycles instead of 880 and those
+  // of Q K^T 717 instead of 815 at head_dim 128 (12x32760x128 629 -> 620 us, fp16 12x16384x128 247 -> 239); where the loops of a tile
+  // fill the instruction cache already they cost more than that (causal 14x32768x128 1779 -> 1930 us), and at head_dim 64 the softmax is the bound
+  // (48x17776x64 694 -> 701 us).
+  static constexpr bool UNROLL_MMA = D == 128 && !CAUSAL;
   // Bias words of tile t are written when the scores of tile t-NK are complete; these were issued behind P V of tile
   // t-NK-NSB, whose softmax is therefore done with its words.
   static constexpr int SLOTS = NK + NSB;
@@ -150,8 +155,8 @@ template <class C> struct Ctrl {
   int abort_flag;
 };
 
-template <int D, bool FIXED> constexpr int smem_bytes() {
-  using C = Cfg<D, FIXED>;
+template <int D, bool FIXED, bool CAUSAL> constexpr int smem_bytes() {
+  using C = Cfg<D, FIXED, CAUSAL>;
   return C::OFF_CTRL + (int)sizeof(Ctrl<C>);
 }
 
@@ -309,7 +314,7 @@ __device__ __forceinline__ float4 column_bias(const float* bias, const unsigned 
 // the tile-image buffers; IMG = false: [slab][128 rows][128 B] filled by tensor-map TMA boxes from row-major tensors.
 template <int D, int FMT, bool IMG, bool CAUSAL, bool FIXED>
 __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_constant__ TmapPack maps, const TcParams p) {
-  using C = Cfg<D, FIXED>;
+  using C = Cfg<D, FIXED, CAUSAL>;
   using Ctl = Ctrl<C>;
   if (p.only_if && *p.only_if == 0) return;
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -506,6 +511,7 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
           planned = true;
           progressed = true;
         }
+        if (!progressed) __nanosleep(40);      // (the ring holds three tiles; a spinning warp takes issue slots and power)
         if (progressed) {
           spins = 0;
         } else if (++spins > (1u << 24) || ((spins & 255) == 255 && *abort_flag)) {
@@ -540,7 +546,7 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
         const int cols = tile_columns(cur, vt, 16);
         const LaneColumns b = lane_columns(cur, vt, cols, lane, bn_shift);
         // fill number f of the stage waits for P V of fill f-1
-        if (ring.fill > 0) ok = spin_wait(v_empty_a + ring.stage * 8, (ring.fill - 1) & 1, abort_flag);
+        if (ring.fill > 0) ok = tc::mbar_wait_a(v_empty_a + ring.stage * 8, (ring.fill - 1) & 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         const uint32_t bar_a = v_full_a + ring.stage * 8;
@@ -580,7 +586,7 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
         uint64_t kdesc = kdesc0 + (uint64_t)(kring.stage * (C::TILE_BYTES >> 4)), qd = qdesc;
         const uint32_t idesc = last ? tc::make_idesc(FMT, 128, (last_cols + 31) & ~31, 0, 0) : idesc_qk;
         const uint32_t tSb = tmem + qk_buf * 128;
-#pragma unroll 1
+#pragma unroll(C::UNROLL_MMA ? C::SLABS : 1)
         for (int sl = 0; sl < C::SLABS; ++sl) {
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks) tc::umma_ss(tSb, qd + ks * 2, kdesc + ks * 2, idesc, (uint32_t)(sl + ks));
@@ -604,13 +610,19 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
         uint32_t tP = tmem + pv_buf * 128;                           // probabilities overwrite the scores they came from
         const uint32_t tO = tmem + C::O_BASE + b * C::O_STRIDE;      // two accumulators: even and odd tiles separately
         uint32_t accumulate = t > (FIXED ? 0 : 1) ? 1u : 0u;
-        const int steps = t == n_tiles - 1 ? (last_cols + 15) >> 4 : 8;      // of 16 keys
-#pragma unroll 1
-        for (int ks = 0; ks < steps; ++ks) {
+        if (C::UNROLL_MMA && t < n_tiles - 1) {
           tc::umma_ts(tO, tP, vdesc, idesc_pv, accumulate);
-          accumulate = 1u;
-          tP += 8;
-          vdesc += (2 * kGroupStride) >> 4;
+#pragma unroll
+          for (int ks = 1; ks < 8; ++ks) tc::umma_ts(tO, tP + ks * 8, vdesc + (uint64_t)(ks * ((2 * kGroupStride) >> 4)), idesc_pv, 1u);
+        } else {
+          const int steps = t == n_tiles - 1 ? (last_cols + 15) >> 4 : 8;      // of 16 keys
+#pragma unroll 1
+          for (int ks = 0; ks < steps; ++ks) {
+            tc::umma_ts(tO, tP, vdesc, idesc_pv, accumulate);
+            accumulate = 1u;
+            tP += 8;
+            vdesc += (2 * kGroupStride) >> 4;
+          }
         }
         tc::umma_commit_a(v_empty_a + vring.stage * 8);   // V tile may be refilled, score buffer may be overwritten
         // "accumulator final", for the last product of the row; with two accumulators for the last one of each.  Three score
@@ -1094,7 +1106,7 @@ static int next_counters(int n, int** out, cudaStream_t st) {
 
 template <int D, int FMT, bool IMG, bool CAUSAL, bool FIXED>
 static int launch_tc(const FwdArgs& a, cudaStream_t st, int* row_counter, int* guard = nullptr, const int* only_if = nullptr) {
-  constexpr int kSmem = smem_bytes<D, FIXED>();
+  constexpr int kSmem = smem_bytes<D, FIXED, CAUSAL>();
   static_assert(kSmem <= 232448, "more than 227 KB of shared memory");
   TmapPack maps;
   const int is_bf16 = FMT == 1;
