@@ -45,7 +45,7 @@ KERNELS_PER_CALL = {
     # forward: the fixed-reference kernel and, right behind it, the exact kernel that returns at once unless the first
     # one raised its guard word
     "psa_assign_levels": 1, "psa_fwd_images": 2, "psa_fwd": 2, "psa_fwd_perm": 2, "psa_layer": 7, "psa_fwd_images_scatter": 2, "psa_push_heads": 1,
-    "psa_push_samples": 1, "psa_pull_heads": 1, "psa_density": 1, "psa_legacy_fwd_images": 3, "psa_legacy_bwd_tc": 3,
+    "psa_push_samples": 1, "psa_pull_heads": 1, "psa_density": 1, "psa_draw_samples": 1, "psa_legacy_fwd_images": 3, "psa_legacy_bwd_tc": 3,
     "psa_legacy_bwd_tcgen05": 4, "psa_ksim": 1, "psa_ksim_perm": 1, "psa_legacy_fwd_images_perm": 3, "psa_gather_rows": 1, "psa_gather_views": 1,
     "psa_pyramid_kv_images_perm": 1, "psa_block_scores_perm": 3, "psa_antidiag_scores_impl": 2, "psa_assign_levels_causal": 1,
 }

@@ -26,7 +26,7 @@
 //               accumulator).  The group that owns a row's last tile finishes the row: it takes the other one's sums from
 //               shared memory, reads the accumulators from TMEM and stores 32 bytes per thread and instruction, while the other
 //               group works on the next row's first tile.
-// What bounds it: ~1750 cycles per tile = a chain of softmax (2000-2500), P V (~870), Q K^T (~800) and their hand-overs over
+// What bounds it: ~1750 cycles per tile = a chain of softmax (2000-2500), P V (~720), Q K^T (~720) and their hand-overs over
 // three score buffers, against 1024 cycles of the tensor pipe and as many of the ex2 unit; and the 1000 W power cap (at 75600
 // tokens the SM clock falls from 1965 to ~1500 MHz).
 // CODE SIZE counts: an SM holds about 32 KB of instructions, and the twelve warps are in five different places of the code.
