@@ -555,6 +555,7 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
         __syncwarp();
         ring.next();
       }
+      __syncwarp();       // every lane has read the row's slot, also of a row without tiles, before it is handed back
       if (ok && lane == 0) tc::mbar_arrive(&ctl->row_done[rs]);
     }
   } else if (warp < 4) {

@@ -93,3 +93,29 @@ def test_first_keys_far_below_the_rest_of_the_first_tile(D):
         sc = ops.psa_forward(q, k, v, mask, 128, bn, 32, impl=ops.IMPL_SCALAR)
         assert int(tc._psa_status.item()) == 0
         _close(tc, sc)
+
+
+@pytest.mark.parametrize("empty", [0.97, 0.6])
+def test_rows_without_tiles_among_others(empty):
+    """Most rows select no block (0/0, as the reference divides) - runs of them hand the four row slots of a CTA round and round,
+    about 22 rows per CTA; the others select one to three tiles."""
+    from psa_b200 import ops
+    heads, mq, nk, bn, D = 48, 70, 25, 64, 64
+    k, v = (C.randn(930 + i, (1, heads, nk * bn, D), torch.bfloat16).to(DEV) for i in range(2))
+    q = C.randn(933, (1, heads, mq * 128, D), torch.bfloat16).to(DEV)
+    g = torch.Generator().manual_seed(int(empty * 100))
+    level = torch.randint(0, 4, (heads, mq), generator=g)
+    count = torch.randint(1, 7, (heads, mq), generator=g) * (torch.rand(heads, mq, generator=g) >= empty)
+    mask = torch.full((1, heads, mq, nk + 5), -1, dtype=torch.int32)
+    for h in range(heads):
+        for r in range(mq):
+            n, at = int(count[h, r]), int(level[h, r])      # `at` empty levels before the one that holds the row's blocks
+            mask[0, h, r, at:at + n] = torch.randperm(nk, generator=g)[:n].to(torch.int32)
+    mask = mask.to(DEV)
+    tc = ops.psa_forward(q, k, v, mask, 128, bn, 32)
+    assert int(tc._psa_status.item()) == 0
+    rows_nan = torch.isnan(tc.float()).view(heads, mq, 128 * D)
+    assert torch.equal(rows_nan.all(-1).cpu(), count == 0) and torch.equal(rows_nan.any(-1).cpu(), count == 0)
+    _close(tc, ops.psa_forward(q, k, v, mask, 128, bn, 32, impl=ops.IMPL_SCALAR))
+    again = ops.psa_forward(q, k, v, mask, 128, bn, 32)
+    assert torch.equal(tc.nan_to_num(), again.nan_to_num())
