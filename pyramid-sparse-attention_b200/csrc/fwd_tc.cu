@@ -222,8 +222,9 @@ struct LaneColumns {
   int li, blk, inside, col;
   bool in, start, extra, pad;      // in: the tile has these columns; extra: block of a narrow level added for reference compatibility
 };
-// The row's last tile is filled up with inert blocks (bias -inf): K to a multiple of 32 columns, the chunk of the softmax, V to a
-// multiple of 16, the step of its product.  They are copies of the row's last block, so a value that is not finite enters no row that did not select it.
+// The row's last tile is filled up: K to a multiple of 32 columns, the chunk of the softmax, with copies of the row's last block (bias
+// -inf: a score that is not finite enters no row that did not select it), V to a multiple of 16, the step of its product, with zeros
+// (a probability of 0 times a copied value that is not finite would be NaN, where the block's own product may be infinite or 0).
 __device__ __forceinline__ int tile_columns(const RowPlan& c, int t, int multiple) {
   return t == c.n_tiles - 1 ? (c.last_cols + multiple - 1) & -multiple : 128;
 }
@@ -543,7 +544,7 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
       const int n_tiles = cur.n_tiles, bh = cur.R / p.mq;
 #pragma unroll 1
       for (int vt = 0; vt < n_tiles; ++vt) {
-        const int cols = tile_columns(cur, vt, 16);
+        const int cols = tile_columns(cur, vt, 1), zero_rows = tile_columns(cur, vt, 16) - cols;
         const LaneColumns b = lane_columns(cur, vt, cols, lane, bn_shift);
         // fill number f of the stage waits for P V of fill f-1
         if (ring.fill > 0) ok = tc::mbar_wait_a(v_empty_a + ring.stage * 8, (ring.fill - 1) & 1, abort_flag);
@@ -551,6 +552,17 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
         if (!ok) break;
         const uint32_t bar_a = v_full_a + ring.stage * 8;
         if (b.start) fetch_block<D, IMG>(p, b, bh, sV_a + ring.stage * C::TILE_BYTES, bar_a, p.vimg, vmap0);
+        if (zero_rows) {       // 4 to 12 rows of 128 bytes per slab (whole rows: the swizzle moves nothing out of them)
+          unsigned char* tile = sV + ring.stage * C::TILE_BYTES;
+#pragma unroll 1
+          for (int i = lane; i < zero_rows * C::SLABS * 8; i += 32) {
+            const int sl = (i >> 3) % C::SLABS, row = cols + (i >> 3) / C::SLABS;
+            const int at = IMG ? (row >> 3) * (C::SLABS * 1024) + sl * 1024 + (row & 7) * 128 : sl * kSlabBytes + row * 128;
+            *reinterpret_cast<uint4*>(tile + at + (i & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+          }
+          tc::fence_proxy_async();      // the tensor pipe reads them
+          __syncwarp();
+        }
         if (lane == 0) tc::mbar_arrive_expect_tx_a(bar_a, (uint32_t)(cols * D * 2));
         __syncwarp();
         ring.next();

@@ -119,3 +119,29 @@ def test_rows_without_tiles_among_others(empty):
     _close(tc, ops.psa_forward(q, k, v, mask, 128, bn, 32, impl=ops.IMPL_SCALAR))
     again = ops.psa_forward(q, k, v, mask, 128, bn, 32)
     assert torch.equal(tc.nan_to_num(), again.nan_to_num())
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("D,bn,images", [(128, 64, True), (64, 64, True), (128, 64, False), (64, 64, False), (128, 32, False), (64, 32, False)])
+def test_infinite_value_in_the_last_selected_block(D, bn, images, dt):
+    """A selected value that is infinite makes its channel infinite, not NaN, however the row's last tile is filled up: rows that end
+    in a block of 4 or 8 columns, one to four tiles long, the last block the one with the infinite value."""
+    from psa_b200 import ops
+    heads, mq, nk = 2, 40, 1024 // bn + 9
+    S = nk * bn
+    k, v = (C.randn(940 + i, (1, heads, S, D), dt).to(DEV) for i in range(2))
+    q = C.randn(943, (1, heads, mq * 128, D), dt).to(DEV)
+    v[0, :, S - bn + 5, 3], v[0, :, S - bn + 5, 7] = float("inf"), float("-inf")
+    mask = torch.full((1, heads, mq, nk + 5), -1, dtype=torch.int32)
+    for r in range(mq):
+        n = 1 + r % (nk - 1)            # blocks of level 1 before the last block of the sequence at level 8
+        mask[:, :, r, :n] = torch.arange(n, dtype=torch.int32)
+        mask[:, :, r, n + 3] = nk - 1
+    mask = mask.to(DEV)
+    tc = ops.psa_forward(q, k, v, mask, 128, bn, 32, pyramid=None if images else ops.pyramid_kv(k, v, bn))
+    assert int(tc._psa_status.item()) == 0
+    assert bool((tc[..., 3] == float("inf")).all()) and bool((tc[..., 7] == float("-inf")).all())
+    sc = ops.psa_forward(q, k, v, mask, 128, bn, 32, impl=ops.IMPL_SCALAR)
+    keep = [c for c in range(D) if c not in (3, 7)]
+    assert bool(torch.isfinite(tc[..., keep]).all())
+    _close(tc[..., keep], sc[..., keep])
