@@ -37,8 +37,8 @@
 // head_dim 64: three score buffers [0,384), O of even tiles [384,448), O of odd tiles [448,512).
 //
 // bf16 calls run the FIXED-REFERENCE variant of the same kernel first: the exponent that the probabilities of a query row
-// are taken relative to is a maximum over columns of the row's FIRST tile (the first chunk of 32 in which every row of the warp sees
-// a key; the group that owns that tile leaves it in shared memory for the other one) and is never raised.  A bf16 probability has the exponent range of fp32, so later scores may exceed the
+// are taken relative to is the maximum of the row's FIRST tile (the group that owns that tile leaves it in shared memory
+// for the other one) and is never raised.  A bf16 probability has the exponent range of fp32, so later scores may exceed the
 // reference by dozens of octaves without losing a bit.  (Not so fp16, which takes the exact kernel: a probability below 2^-14
 // is subnormal, and with one reference for both groups more of them are - error against 64 bits up to 4 % larger.)  The sum
 // stays in fp32.  That removes the maximum pass from every tile but
@@ -759,27 +759,16 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
     mx2 = fmaxf(mx2, fmaf(fmaxf(fmaxf(f[24], f[25]), fmaxf(f[26], f[27])), p.scale_log2, gb.z));                             \
     mx3 = fmaxf(mx3, fmaf(fmaxf(fmaxf(f[28], f[29]), fmaxf(f[30], f[31])), p.scale_log2, gb.w));                             \
   } while (0)
-            if (FIXED) {
-              // any key's score will do as the reference: the chunks up to the first one in which every row of the warp sees one
+            tc::tmem_ld32(tS, va);
 #pragma unroll 1
-              for (int c = 0; c < chunks; ++c) {
-                tc::tmem_ld32(tS + 32 * c, va);
+            for (int c = 0; c < chunks; c += 2) {
+              tc::tmem_wait_ld();
+              if (c + 1 < chunks) tc::tmem_ld32(tS + 32 * c + 32, vb);
+              PSA_MAX_CHUNK(va, c);
+              if (c + 1 < chunks) {
                 tc::tmem_wait_ld();
-                PSA_MAX_CHUNK(va, c);
-                if (__all_sync(0xffffffffu, fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) > -INFINITY)) break;
-              }
-            } else {
-              tc::tmem_ld32(tS, va);
-#pragma unroll 1
-              for (int c = 0; c < chunks; c += 2) {
-                tc::tmem_wait_ld();
-                if (c + 1 < chunks) tc::tmem_ld32(tS + 32 * c + 32, vb);
-                PSA_MAX_CHUNK(va, c);
-                if (c + 1 < chunks) {
-                  tc::tmem_wait_ld();
-                  if (c + 2 < chunks) tc::tmem_ld32(tS + 32 * c + 64, va);
-                  PSA_MAX_CHUNK(vb, c + 1);
-                }
+                if (c + 2 < chunks) tc::tmem_ld32(tS + 32 * c + 64, va);
+                PSA_MAX_CHUNK(vb, c + 1);
               }
             }
 #undef PSA_MAX_CHUNK
@@ -796,7 +785,6 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
                 mx2 = fmaxf(mx2, fmaf(__uint_as_float(va[4 * q4 + 2]), p.scale_log2, ba.z));
                 mx3 = fmaxf(mx3, fmaf(__uint_as_float(va[4 * q4 + 3]), p.scale_log2, ba.w));
               }
-              if (FIXED && __all_sync(0xffffffffu, fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) > -INFINITY)) break;
             }
           }
           const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
