@@ -485,9 +485,10 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
             if (b.extra) bias2 += log2f((float)(pick4(b.li, cur.cnt0, cur.cnt1, cur.cnt2, cur.cnt3) >> 1));
             words[lane] = b.in && !b.pad && nvalid > 0 ? bias2 : -INFINITY;
             const bool diag = CAUSAL && b.in && b.blk == m && !b.pad && !b.extra;
-            // a block that ends inside a group of 4 columns, or the diagonal block of a causal row, makes the tile take the
-            // per-column path of the softmax
-            const unsigned odd_lanes = __ballot_sync(0xffffffffu, b.in && !b.pad && ((nvalid > 0 && nvalid < 4) || diag));
+            // a block that ends inside a group of 4 columns, the diagonal block of a causal row, or the end of the row's tokens
+            // 16 columns or more before the tile's makes the tile take the per-column path of the softmax
+            const unsigned odd_lanes = __ballot_sync(0xffffffffu, (b.in && !b.pad && ((nvalid > 0 && nvalid < 4) || diag)) ||
+                                                                      (kt == n_tiles - 1 && cur.last_cols <= 112));
             if (odd_lanes) reinterpret_cast<unsigned char*>(words + 36)[lane] = (unsigned char)(nvalid > 0 && nvalid < 4 ? (1 << nvalid) - 1 : 15);
             if (lane == 0) reinterpret_cast<int*>(words)[32] = odd_lanes != 0;
             if (CAUSAL) {
@@ -728,7 +729,8 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
           const unsigned char* valid4 = reinterpret_cast<const unsigned char*>(slot_words + 36);   // 4 bits per group of 4 columns
           // Fast path: the bias is uniform inside every aligned group of 4 columns (blocks are at least 4 wide), so the
           // maximum is taken on raw scores per group and the bias enters once per group.  A tile with a block that ends
-          // inside a group, or with the causal diagonal, takes the per-column path.
+          // inside a group, with the causal diagonal, or that ends 16 columns early or more takes the per-column path (which rounds
+          // score times scale before it subtracts the reference, so that the column with the maximum has exactly 1, whatever its size).
           const bool odd = reinterpret_cast<const int*>(slot_words)[32] != 0;
           // causal: of the diagonal block's pooled tokens (level li, columns [c0, c0 + 128 / l)) number i ends at position
           // (i + 1) l - 1, so row r sees the first (r + 1) / l of them

@@ -172,3 +172,25 @@ def test_bf16_reference_is_the_maximum_of_the_whole_first_tile(D, causal):
     assert int(out._psa_status.item()) == 0
     got = out[:, :, 128:].double().cpu()
     assert abs(float((got / want).mean()) - 1.0) <= 1e-3
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("D,bn", [(64, 64), (128, 64), (64, 32), (128, 32)])
+def test_large_equal_scores_in_a_tile_that_ends_early(D, bn, dt):
+    """Equal scores of 2^17 to 2^19 octaves (half of that in fp16) in a tile of 4 or 8 columns: the reference is one of them, so every
+    probability is exactly 1 and the result the common value.  A score that is multiplied by the scale and reduced by the rounded
+    reference in one step leaves what the reference's rounding took, up to half a unit of 2^-5 octaves, in the sum but not in the
+    rounded probabilities."""
+    from psa_b200 import ops
+    unit = 1.0 if dt == torch.bfloat16 else 0.5
+    gains = [129, 131, 133, 137, 139, 143]
+    heads, S = len(gains), 8 * bn
+    q = torch.full((1, heads, 256, D), 128.0 * unit)
+    k = torch.tensor(gains, dtype=torch.float32).view(1, heads, 1, 1).expand(1, heads, S, D).contiguous()
+    v = torch.ones((1, heads, S, D))
+    q, k, v = (x.to(dt).to(DEV) for x in (q, k, v))
+    assert k.float().mean(dim=(2, 3)).cpu().view(-1).tolist() == gains
+    mask = torch.tensor([-1, -1, -1, 3, -1] + [0] * 8, dtype=torch.int32).view(1, 1, 1, 13).expand(1, heads, 2, 13).contiguous().to(DEV)
+    out = ops.psa_forward(q, k, v, mask, 128, bn, 32)
+    assert int(out._psa_status.item()) == 0
+    assert bool((out == 1).all()), out[0, :, 0, 0].tolist()
