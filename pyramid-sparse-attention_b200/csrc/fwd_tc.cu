@@ -120,6 +120,10 @@ template <int D, bool FIXED = false, bool CAUSAL = false> struct Cfg {
   // fill the instruction cache already they cost more than that (causal 14x32768x128 1779 -> 1930 us), and at head_dim 64 the softmax is the bound
   // (48x17776x64 694 -> 701 us).
   static constexpr bool UNROLL_MMA = D == 128 && !CAUSAL;
+  // The second pass of a full tile, two chunks at a time in a loop or all four in the code.  The loop, half the code, is the better one
+  // (exact kernel, 16 x 9973 x 128 168 against 205 us, 6 x 32760 x 128 387 / 438, causal 8 x 16384 x 64 318 / 344) except in the exact kernel at
+  // head_dim 64 without the causal rule, where three score buffers keep both groups in this pass (6 x 32760 365 / 311, 8 x 20011 704 / 610).
+  static constexpr bool UNROLL_EXP = D == 64 && !FIXED && !CAUSAL;
   // Bias words of tile t are written when the scores of tile t-NK are complete; these were issued behind P V of tile
   // t-NK-NSB, whose softmax is therefore done with its words.
   static constexpr int SLOTS = NK + NSB;
@@ -731,6 +735,8 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
           // maximum is taken on raw scores per group and the bias enters once per group.  A tile with a block that ends
           // inside a group, with the causal diagonal, or that ends 16 columns early or more takes the per-column path (which rounds
           // score times scale before it subtracts the reference, so that the column with the maximum has exactly 1, whatever its size).
+          // So the fast path's tiles have four chunks, and its loops no tests of their number: with them the exact kernel at head_dim 128
+          // spilled 12 bytes and took 8 to 14 % longer (fp16 8 x 20011 x 128 878 -> 776 us, bf16 645 -> 630).
           const bool odd = reinterpret_cast<const int*>(slot_words)[32] != 0;
           // causal: of the diagonal block's pooled tokens (level li, columns [c0, c0 + 128 / l)) number i ends at position
           // (i + 1) l - 1, so row r sees the first (r + 1) / l of them
@@ -763,15 +769,13 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
   } while (0)
             tc::tmem_ld32(tS, va);
 #pragma unroll 1
-            for (int c = 0; c < chunks; c += 2) {
+            for (int c = 0; c < 4; c += 2) {
               tc::tmem_wait_ld();
-              if (c + 1 < chunks) tc::tmem_ld32(tS + 32 * c + 32, vb);
+              tc::tmem_ld32(tS + 32 * c + 32, vb);
               PSA_MAX_CHUNK(va, c);
-              if (c + 1 < chunks) {
-                tc::tmem_wait_ld();
-                if (c + 2 < chunks) tc::tmem_ld32(tS + 32 * c + 64, va);
-                PSA_MAX_CHUNK(vb, c + 1);
-              }
+              tc::tmem_wait_ld();
+              if (c == 0) tc::tmem_ld32(tS + 64, va);
+              PSA_MAX_CHUNK(vb, c + 1);
             }
 #undef PSA_MAX_CHUNK
           } else if (ref_tile) {
@@ -866,16 +870,14 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
     tc::tmem_st16(tS + 16 * (c), pk);                                                                                        \
   } while (0)
             tc::tmem_ld32(tS, va);
-#pragma unroll 1
-            for (int c = 0; c < chunks; c += 2) {
+#pragma unroll(C::UNROLL_EXP ? 2 : 1)
+            for (int c = 0; c < 4; c += 2) {
               tc::tmem_wait_ld();
-              if (c + 1 < chunks) tc::tmem_ld32(tS + 32 * c + 32, vb);
+              tc::tmem_ld32(tS + 32 * c + 32, vb);
               PSA_EXP_CHUNK(va, c);
-              if (c + 1 < chunks) {
-                tc::tmem_wait_ld();
-                if (c + 2 < chunks) tc::tmem_ld32(tS + 32 * c + 64, va);
-                PSA_EXP_CHUNK(vb, c + 1);
-              }
+              tc::tmem_wait_ld();
+              if (c == 0) tc::tmem_ld32(tS + 64, va);
+              PSA_EXP_CHUNK(vb, c + 1);
             }
 #undef PSA_EXP_CHUNK
 #undef PSA_EXP_GROUP
