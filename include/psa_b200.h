@@ -31,6 +31,14 @@ extern "C" {
 
 #define PSA_MAX_LEVELS 8
 
+/* Index lists and key blocks that calls of the tcgen05 forward may have; what goes beyond takes the scalar kernel or is refused.  The
+ * kernel holds no table of a list: these are the lengths that it has been run and compared at, and callers choose
+ * their route by them (longer lists than PSA_FWD_LIST_MAX only with row-major K/V). */
+#define PSA_FWD_LIST_MAX 1472
+#define PSA_FWD_BLOCKS_MAX 16384
+#define PSA_FWD_LIST_MAX_ROWS 4096
+#define PSA_FWD_BLOCKS_MAX_ROWS 8192   /* of lists above PSA_FWD_LIST_MAX */
+
 /* Text of the last error raised on the calling thread ("" if none). */
 const char* psa_last_error_string(void);
 
@@ -126,7 +134,7 @@ int psa_ksim(const void* k, int32_t* out, int64_t bh, int64_t seq, int head_dim,
  * level-4, -1, level-8, -1, rest ignored.  compat_quirk != 0 reproduces the reference's handling of levels
  * whose pooled block is narrower than half a tile (:261-278): each merged pair also attends pooled tokens
  * [2P, tile_n) of that level.  impl: 0 = pick, 1 = scalar kernel, 2 = tcgen05 kernel (f16/bf16, block_m 128; lists of up to
- * 1472 entries over up to 16384 key blocks, or of up to 4096 entries over up to 8192 - what 0 picks it for).
+ * PSA_FWD_LIST_MAX entries over up to PSA_FWD_BLOCKS_MAX key blocks, or the longer ones of the _ROWS limits - what 0 picks it for).
  * status: device int32 word, written non-zero if a bounded wait inside the kernel expired (may be NULL).
  * The tcgen05 kernel is persistent: its CTAs claim query blocks from a counter.  The counters are a ring of 256 device
  * words inside the library (one per launch, zeroed on the launching stream right before the kernel); the first
@@ -135,10 +143,10 @@ int psa_ksim(const void* k, int32_t* out, int64_t bh, int64_t seq, int head_dim,
  * its slot for every replay: do not replay such graphs while more than 255 other launches overlap them).  This holds
  * for every psa_fwd* / psa_legacy_fwd_images* entry point.
  * A bf16 call is TWO launches of the tcgen05 kernel (an fp16 one is the second of them alone).  The first takes the probabilities of a query row
- * relative to the maximum of the row's first tile instead of a running maximum (same result: the factor cancels against
- * the row sum; bf16 probabilities and the fp32 sum have the exponent range for it), which saves the maximum pass and
- * the rescaling; a row whose sum leaves the safe range, or whose accumulated values are not finite, sets a guard word
- * (another slot of the counter ring).  The
+ * relative to the maximum of the row's first tile (its first 128 gathered keys) instead of a running maximum (same result: the factor
+ * cancels against the row sum; bf16 probabilities and the fp32 sum have the exponent range for it), which saves the maximum pass and
+ * the rescaling; a row whose sum leaves the safe range (a key about 90 octaves above all of the first tile), or whose accumulated
+ * values are not finite, sets a guard word (another slot of the counter ring) and makes the whole call run again.  The
  * second launch is the running-maximum kernel: it reads the guard word, returns at once if it is zero and recomputes
  * the call otherwise.  Both are ordered on `stream`; nothing is read back by the host.  A bf16 call therefore takes THREE
  * words of the ring (two row counters and the guard word): about 85 such calls may be in flight on one device before words are

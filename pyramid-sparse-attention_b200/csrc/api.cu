@@ -52,8 +52,8 @@ static int fwd_rows(const void* q, const void* k, const void* v, const void* k2,
   a.scatter.row_perm = out_perm;
   const bool tc_ok = fwd_tc_supported(a);
   if (impl == 2) PSA_REQUIRE(tc_ok, PSA_ERR_UNSUPPORTED, 
-                              "psa_fwd: the tcgen05 kernel needs f16/bf16, block_m=128, lists of at most 4096 entries and 8192 key blocks (16384 "
-                              "up to 1472 entries)");
+                              "psa_fwd: the tcgen05 kernel needs f16/bf16, block_m=128, lists of at most %d entries and %d key blocks (%d "
+                              "up to %d entries)", PSA_FWD_LIST_MAX_ROWS, PSA_FWD_BLOCKS_MAX_ROWS, PSA_FWD_BLOCKS_MAX, PSA_FWD_LIST_MAX);
   if (impl == 2 || (impl == 0 && tc_ok)) return fwd_tc_launch(a, st);
   return fwd_simt_dispatch(q, kl, vl, nl, mask, out, bh, seq_q, head_dim, block_m, block_n, tile_n, mask_width, sm_scale,
                            compat_quirk, dtype, st);
@@ -111,7 +111,7 @@ extern "C" int psa_fwd_images(const void* q, const void* kimg, const void* vimg,
   a.bh = bh; a.seq_q = seq_q; a.seq_k = seq_k; a.D = head_dim; a.bm = block_m; a.bn = block_n; a.tn = tile_n;
   a.width = mask_width; a.scale = sm_scale; a.quirk = compat_quirk; a.dtype = dtype;
   PSA_REQUIRE(fwd_tc_supported(a), PSA_ERR_UNSUPPORTED,
-              "psa_fwd_images: needs f16/bf16, block_m=128, tile_n=32, head_dim 64/128, mask width <= 1472");
+              "psa_fwd_images: needs f16/bf16, block_m=128, tile_n=32, head_dim 64/128, mask width <= %d", PSA_FWD_LIST_MAX);
   return fwd_tc_launch(a, (cudaStream_t)stream);
 }
 
@@ -134,7 +134,7 @@ extern "C" int psa_fwd_images_perm(const void* q, const void* kimg, const void* 
   a.width = mask_width; a.scale = sm_scale; a.quirk = compat_quirk; a.dtype = dtype;
   a.scatter.row_perm = out_perm;
   PSA_REQUIRE(fwd_tc_supported(a), PSA_ERR_UNSUPPORTED,
-              "psa_fwd_images_perm: needs f16/bf16, block_m=128, tile_n=32, head_dim 64/128, mask width <= 1472");
+              "psa_fwd_images_perm: needs f16/bf16, block_m=128, tile_n=32, head_dim 64/128, mask width <= %d", PSA_FWD_LIST_MAX);
   return fwd_tc_launch(a, (cudaStream_t)stream);
 }
 
@@ -158,7 +158,7 @@ extern "C" int psa_fwd_images_tm(const void* q, const void* kimg, const void* vi
   a.scatter.n_peers = 1; a.scatter.heads_total = heads; a.scatter.head0 = 0; a.scatter.tokens_per_rank = seq;
   a.scatter.row_perm = out_perm;
   PSA_REQUIRE(fwd_tc_supported(a), PSA_ERR_UNSUPPORTED,
-              "psa_fwd_images_tm: needs f16/bf16, block_m=128, tile_n=32, head_dim 64/128, mask width <= 1472");
+              "psa_fwd_images_tm: needs f16/bf16, block_m=128, tile_n=32, head_dim 64/128, mask width <= %d", PSA_FWD_LIST_MAX);
   return fwd_tc_launch(a, (cudaStream_t)stream);
 }
 
@@ -191,6 +191,6 @@ extern "C" int psa_fwd_images_scatter(const void* q, const void* kimg, const voi
   a.scatter.n_peers = n_peers; a.scatter.heads_total = heads_total; a.scatter.head0 = head0;
   a.scatter.tokens_per_rank = tokens_per_rank;
   PSA_REQUIRE(fwd_tc_supported(a), PSA_ERR_UNSUPPORTED,
-              "psa_fwd_images_scatter: needs f16/bf16, block_m=128, tile_n=32, head_dim 64/128, mask width <= 1472");
+              "psa_fwd_images_scatter: needs f16/bf16, block_m=128, tile_n=32, head_dim 64/128, mask width <= %d", PSA_FWD_LIST_MAX);
   return fwd_tc_launch(a, (cudaStream_t)stream);
 }

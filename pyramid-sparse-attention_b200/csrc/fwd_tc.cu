@@ -64,9 +64,6 @@ namespace psa {
 
 namespace {
 
-// Longest index lists and largest block counts that this kernel takes; callers size and route by them.
-constexpr int kMaxWidth = 1472, kMaxBlocks = 16384;             // common lists, and everything on tile images
-constexpr int kMaxWidthLong = 4096, kMaxBlocksLong = 8192;      // longer lists, row-major K/V
 constexpr int kSlabBytes = 128 * 128;  // 128 rows x 128 B (64 16-bit channels)
 constexpr int kSoftmaxThreads = 256;
 constexpr int kThreads = 4 * 32 + kSoftmaxThreads;   // 384
@@ -375,9 +372,9 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
   const uint32_t tmem = ctl->tmem_base;
 
   // A CTA is persistent: it starts with query row R = blockIdx.x (R = bh * mq + m) and claims further rows from a global
-  // counter (SMs do not all run at the same speed, so a fixed split would leave the fast ones idle at the end); its three
-  // roles run the rows as one continuous stream of tiles.  Ring stages, score buffers and barrier phases are indexed by
-  // the running tile count g0 + t, so the producers decode and prefetch the next row while the MMAs and the softmax of
+  // counter (SMs do not all run at the same speed, so a fixed split would leave the fast ones idle at the end); its
+  // roles run the rows as one continuous stream of tiles.  Ring stages, score buffers and barrier phases follow
+  // the running tile count, so the producers plan and prefetch the next row while the MMAs and the softmax of
   // the current row are still in flight, and the first scores of the next row are computed under the epilogue.
   if (warp == 0) {
     // ============================================================ K producer, query tiles, planning of the rows
@@ -517,7 +514,7 @@ __global__ void __launch_bounds__(kThreads, 1) psa_fwd_tc_kernel(const __grid_co
           planned = true;
           progressed = true;
         }
-        if (!progressed) __nanosleep(40);      // (the ring holds three tiles; a spinning warp takes issue slots and power)
+        if (!progressed) __nanosleep(40);      // (the ring holds three or four tiles; a spinning warp takes issue slots and power)
         if (progressed) {
           spins = 0;
         } else if (++spins > (1u << 24) || ((spins & 255) == 255 && *abort_flag)) {
@@ -1067,8 +1064,9 @@ bool fwd_tc_supported(const FwdArgs& a) {
   if (a.dtype != PSA_F16 && a.dtype != PSA_BF16) return false;
   if (a.bm != 128 || a.tn != 32) return false;
   if (a.D != 64 && a.D != 128) return false;
-  if (a.width > (a.kimg || a.causal ? kMaxWidth : kMaxWidthLong)) return false;
-  if (cdiv64(a.seq_k, a.bn) > (a.width > kMaxWidth ? kMaxBlocksLong : kMaxBlocks)) return false;
+  // (no table in the kernel bounds these: what its lists have been tested at, and what callers route by)
+  if (a.width > (a.kimg || a.causal ? PSA_FWD_LIST_MAX : PSA_FWD_LIST_MAX_ROWS)) return false;
+  if (cdiv64(a.seq_k, a.bn) > (a.width > PSA_FWD_LIST_MAX ? PSA_FWD_BLOCKS_MAX_ROWS : PSA_FWD_BLOCKS_MAX)) return false;
   if (a.bh > 65535) return false;
   if (!(a.scale > 0.f)) return false;
   const void* ptrs[] = {a.q, a.out, a.k[0], a.k[1], a.k[2], a.k[3], a.v[0], a.v[1], a.v[2], a.v[3]};
@@ -1138,8 +1136,8 @@ static int launch_tc(const FwdArgs& a, cudaStream_t st, int* row_counter, int* g
   cudaError_t e = cudaFuncSetAttribute(psa_fwd_tc_kernel<D, FMT, IMG, CAUSAL, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   PSA_REQUIRE(e == cudaSuccess, PSA_ERR_CUDA, "psa_fwd: shared-memory opt-in (%d B) failed: %s", kSmem,
               cudaGetErrorString(e));
-  // persistent: one CTA per SM (224 KB of shared memory and all 512 TMEM columns each), rows dealt round-robin so that
-  // the CTAs running at the same time work on neighbouring rows of the same head (K/V stay in L2)
+  // persistent: one CTA per SM (up to 227 KB of shared memory and all 512 TMEM columns each); rows are claimed from a counter in
+  // ascending order, so the CTAs running at the same time work on neighbouring rows of the same head (K/V stay in L2)
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

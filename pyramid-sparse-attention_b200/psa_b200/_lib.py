@@ -13,6 +13,8 @@ LIB_PATH = os.path.join(_HERE, "libpsa_b200.so")
 
 PSA_OK, PSA_ERR_ARG, PSA_ERR_UNSUPPORTED, PSA_ERR_CUDA, PSA_ERR_TIMEOUT = 0, 1, 2, 3, 4
 PSA_F32, PSA_F16, PSA_BF16 = 0, 1, 2
+# index lists and key blocks that calls of the tcgen05 forward may have (see the header)
+PSA_FWD_LIST_MAX, PSA_FWD_BLOCKS_MAX, PSA_FWD_LIST_MAX_ROWS, PSA_FWD_BLOCKS_MAX_ROWS = 1472, 16384, 4096, 8192
 
 if not os.path.exists(LIB_PATH):
     raise ImportError(

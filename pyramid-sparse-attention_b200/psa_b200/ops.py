@@ -10,7 +10,7 @@ from typing import Dict, List, Optional, Sequence, Tuple
 import torch
 
 from . import _lib
-from ._lib import check, lib
+from ._lib import PSA_FWD_BLOCKS_MAX, PSA_FWD_LIST_MAX, check, lib
 
 _DT = {torch.float32: _lib.PSA_F32, torch.float16: _lib.PSA_F16, torch.bfloat16: _lib.PSA_BF16}
 
@@ -583,8 +583,8 @@ def psa_forward(q, k, v, mask, block_m: int, block_n: int, tile_n: int, sm_scale
     Sk = k.shape[2]
     if sm_scale is None:
         sm_scale = D ** -0.5
-    use_images = isinstance(pyramid, KVImages) or (pyramid is None and impl == IMPL_AUTO and mask.shape[-1] <= 1472
-                                                   and -(-Sk // block_n) <= 16384    # block numbers of the tcgen05 kernel
+    use_images = isinstance(pyramid, KVImages) or (pyramid is None and impl == IMPL_AUTO and mask.shape[-1] <= PSA_FWD_LIST_MAX
+                                                   and -(-Sk // block_n) <= PSA_FWD_BLOCKS_MAX
                                                    and images_supported(k, block_m, block_n, tile_n) and sm_scale > 0)
     if use_images:
         if pyramid is None:
@@ -646,7 +646,7 @@ def layer_supported(q, k, v, config) -> bool:
     n = len(config.mask_ratios) if config.mask_ratios else 0
     return (config.attn_impl == "new_mask_type" and not config.use_sim_mask and config.mask_mode in ("topk", "thresholdbound")
             and images_supported(k, config.block_m, config.block_n, config.tile_n) and 0 < n <= 8
-            and -(-k.shape[2] // config.block_n) + n <= 1472 and q.shape[0] * q.shape[1] < 65536)
+            and -(-k.shape[2] // config.block_n) + n <= PSA_FWD_LIST_MAX and q.shape[0] * q.shape[1] < 65536)
 
 
 def psa_layer(q, k, v, idx_q, idx_k, config) -> torch.Tensor:
@@ -699,7 +699,7 @@ IMPL_WARP_MMA = 3      # legacy backward only: the warp-level mma.sync kernels
 
 
 def _legacy_tc_ok(q: torch.Tensor, sm_scale: float) -> bool:
-    return q.dtype in (torch.float16, torch.bfloat16) and -(-q.shape[2] // 128) + 5 <= 1472 and sm_scale > 0
+    return q.dtype in (torch.float16, torch.bfloat16) and -(-q.shape[2] // 128) + 5 <= PSA_FWD_LIST_MAX and sm_scale > 0
 
 
 def legacy_forward(q, k, v, mask, causal: bool = False, sm_scale: Optional[float] = None, need_lse: bool = False,

@@ -14,6 +14,7 @@ import torch
 import torch.nn as nn
 
 from . import ops
+from ._lib import PSA_FWD_LIST_MAX, PSA_FWD_LIST_MAX_ROWS
 from .attention import compute_block_mask, psa_attention_token_major, token_major_view
 from .kernels import legacy_sparse_attention_factory, sparse_attention_factory
 from .rearrange import GilbertRearranger
@@ -148,7 +149,7 @@ class PyramidSparseAttention(nn.Module):
         return (self.use_rearrange and c.attn_impl == "new_mask_type" and not c.use_sim_mask and q.is_cuda
                 and q.shape[2] == k.shape[2] == self.gilbert_rearranger.total_elements + self.gilbert_rearranger.text_length
                 and ops.images_supported(k, c.block_m, c.block_n, c.tile_n)
-                and -(-k.shape[2] // c.block_n) + 5 <= 1472)
+                and -(-k.shape[2] // c.block_n) + 5 <= PSA_FWD_LIST_MAX)
 
     def _rows_in_place_old_format(self, q, k) -> bool:
         """The same for the old mask format (with or without the similarity cap; block 128): inference only, the
@@ -157,7 +158,7 @@ class PyramidSparseAttention(nn.Module):
         return (self.use_rearrange and c.attn_impl == "old_mask_type" and q.is_cuda
                 and not (torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or self._v_requires_grad))
                 and q.dtype in (torch.float16, torch.bfloat16) and c.block_m == 128 and c.block_n == 128 and c.tile_n == 32
-                and q.shape[-1] in (64, 128) and -(-q.shape[2] // 128) + 5 <= 1472
+                and q.shape[-1] in (64, 128) and -(-q.shape[2] // 128) + 5 <= PSA_FWD_LIST_MAX
                 and q.shape[2] == k.shape[2] == self.gilbert_rearranger.total_elements + self.gilbert_rearranger.text_length)
 
     _v_requires_grad = False      # set per call by forward()
@@ -233,7 +234,7 @@ class PyramidSparseAttention(nn.Module):
             q_r, k_r, v_r = ops.gather_views(q, k, v, perm, rotary)
             c = self.config
             if (perm is not None and self.sparse_attention_fn is self._own_attention_fn and c.attn_impl == "new_mask_type"
-                    and c.block_m == 128 and c.block_n == 32 and c.tile_n == 32 and -(-k.shape[2] // c.block_n) + len(c.mask_ratios) <= 4096):
+                    and c.block_m == 128 and c.block_n == 32 and c.tile_n == 32 and -(-k.shape[2] // c.block_n) + len(c.mask_ratios) <= PSA_FWD_LIST_MAX_ROWS):
                 # ... and the way back is where the forward stores its rows
                 with torch.no_grad():
                     mask, _, _ = compute_block_mask(q_r, k_r, c, text_length=c.text_length)

@@ -1,6 +1,6 @@
-"""GPU: index lists longer than the common forward kernel's tables (row-major K/V) on the tcgen05 kernel, against the scalar
-kernel on the same inputs and mask: just past the common limit, at the variant's limit, both head sizes and element types, rows
-that are nearly dense, empty, or hold one narrow block."""
+"""GPU: index lists of more than PSA_FWD_LIST_MAX entries (row-major K/V) on the tcgen05 kernel, against the scalar kernel on the same
+inputs and mask: just past that limit, at PSA_FWD_LIST_MAX_ROWS, both head sizes and element types, rows that are nearly dense,
+empty, or hold one narrow block."""
 import pytest
 import torch
 
@@ -44,11 +44,11 @@ def test_wide_rows_equal_the_scalar_kernel(D, nk, bn, dt):
     (128, 2400, 128, 2405, torch.bfloat16),     # 307200 gathered tokens in a row: more than 2048 tiles
     (64, 4091, 128, 4096, torch.float16),       # ... and the most a list can hold
     (128, 5000, 32, 1500, torch.bfloat16),      # block numbers above 4095 in lists past the common limit
-    (64, 8192, 32, 4096, torch.bfloat16),       # ... up to the largest the wide tables hold
+    (64, 8192, 32, 4096, torch.bfloat16),       # ... up to PSA_FWD_BLOCKS_MAX_ROWS
     (128, 8193, 32, 1500, torch.bfloat16),      # one block more: the scalar kernel takes the call
-    (128, 5000, 32, 1472, torch.float16),       # the same in the common kernel, row-major ...
+    (128, 5000, 32, 1472, torch.float16),       # the same in lists up to PSA_FWD_LIST_MAX, row-major ...
     (64, 5000, 64, 700, torch.bfloat16),        # ... and from tile images
-    (64, 16384, 32, 1472, torch.bfloat16),      # the largest number the common tables hold
+    (64, 16384, 32, 1472, torch.bfloat16),      # PSA_FWD_BLOCKS_MAX blocks
     (64, 16385, 64, 300, torch.bfloat16),       # one block more
 ])
 def test_rows_of_very_long_sequences_equal_the_scalar_kernel(D, nk, bn, width, dt):

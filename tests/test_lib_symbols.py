@@ -27,6 +27,13 @@ def test_library_exports_every_declared_symbol():
     assert b"sm_100a" in _lib.lib.psa_build_info()
 
 
+def test_list_limits_of_the_header():
+    from psa_b200 import _lib
+    src = open(os.path.join(ROOT, "include", "psa_b200.h")).read()
+    limits = dict(re.findall(r"#define (PSA_FWD_[A-Z_]+) (\d+)", src))
+    assert len(limits) == 4 and all(getattr(_lib, name) == int(value) for name, value in limits.items())
+
+
 def test_argument_errors_need_no_gpu():
     from psa_b200 import _lib
     rc = _lib.lib.psa_pyramid_kv(None, None, None, None, None, None, None, None, 1, 1, 64, 64, 0, None)
