@@ -1,7 +1,8 @@
-"""GPU: the tcgen05 forward at the ends of its rows - rows of 0 to 6 tiles of 128 columns in every order, so that each softmax group
-finishes rows and starts the next ones early; last tiles of every width; an output that is 16- but not 32-byte aligned; blocks
-that no row selects and that hold values that are not finite; first keys far below the rest of the first tile.  Yardstick: the
-scalar kernel on the same 16-bit inputs."""
+"""GPU: the tcgen05 forward at the ends of its rows - rows of 0 to 6 tiles of 128 columns in many orders, so that each softmax group
+finishes rows and starts the next ones early, 13 to 22 rows to a CTA (one runs on each of 148 SMs), so that row slots and barriers
+go round several times; last tiles of every width; an output that is 16- but not 32-byte aligned, or in the buffers of several
+owners; the causal rule, log-sum-exp rows and rows without a visible key; blocks that no row selects and that hold values that are
+not finite; first keys far below the rest of the first tile.  Yardstick: the scalar kernel on the same 16-bit inputs."""
 import pytest
 import torch
 
@@ -41,9 +42,9 @@ def _close(a, b):
 
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
 @pytest.mark.parametrize("D,bn", [(128, 64), (64, 64), (128, 128), (64, 128), (128, 32), (64, 32)])
-def test_short_rows_in_every_order(D, bn, dt):
+def test_short_rows_in_many_orders(D, bn, dt):
     from psa_b200 import ops
-    heads, mq, nk = 6, 70, 1024 // bn + 9
+    heads, mq, nk = 48, 70, 1024 // bn + 9
     S = nk * bn - 3
     k, v = (C.randn(900 + i, (1, heads, S, D), dt).to(DEV) for i in range(2))
     q = C.randn(903, (1, heads, mq * 128 - 5, D), dt).to(DEV)
@@ -56,13 +57,14 @@ def test_short_rows_in_every_order(D, bn, dt):
     _close(tc, sc)
     again = ops.psa_forward(q, k, v, mask, 128, bn, 32)
     assert again.data_ptr() % 32 == 0
+    assert torch.equal(again.nan_to_num(), tc.nan_to_num())
     _close(again, sc)
 
 
 @pytest.mark.parametrize("bn", [32, 64, 128])
 def test_blocks_that_no_row_selects_may_hold_anything(bn):
     from psa_b200 import ops
-    heads, mq, nk, D = 2, 40, 1024 // bn + 9, 128
+    heads, mq, nk, D = 48, 40, 1024 // bn + 9, 128
     S = nk * bn
     bad = (0, 2, 3, 5)      # block 0 and those that narrow levels pair up with (2, 3 at most)
     k, v = (C.randn(910 + i, (1, heads, S, D), torch.bfloat16).to(DEV) for i in range(2))
@@ -194,3 +196,66 @@ def test_large_equal_scores_in_a_tile_that_ends_early(D, bn, dt):
     out = ops.psa_forward(q, k, v, mask, 128, bn, 32)
     assert int(out._psa_status.item()) == 0
     assert bool((out == 1).all()), out[0, :, 0, 0].tolist()
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [False, True], ids=["full", "causal"])
+def test_short_rows_of_the_old_format(D, causal, dt):
+    """Rows of 0 to 6 tiles from level masks, with log-sum-exp: rows without a block or (causal, diagonal block of a pooled level alone)
+    without a visible key give 0 and -inf; a last block that ends inside a group of four columns."""
+    from psa_b200 import ops
+    heads, nb = 48, 70
+    S = nb * 128 - 5
+    q, k, v = (C.randn(950 + i, (1, heads, S, D), dt).to(DEV) for i in range(3))
+    g = torch.Generator().manual_seed(D + causal)
+    mask = torch.zeros((1, heads, nb, nb), dtype=torch.int32)
+    levels = torch.tensor([1, 2, 4, 8], dtype=torch.int32)
+    for h in range(heads):
+        for m in range(nb):
+            seen = m + 1 if causal else nb
+            n = min(int(torch.randint(0, 7, (1,), generator=g)), seen)
+            picks = torch.randperm(seen, generator=g)[:n]
+            if n and int(torch.randint(0, 2, (1,), generator=g)):
+                picks[0] = seen - 1                       # the diagonal block, or the sequence's last one
+            mask[0, h, m, picks] = levels[torch.randint(0, 4, (n,), generator=g)]
+    mask = mask.to(DEV)
+    out, lse, _ = ops.legacy_forward(q, k, v, mask, causal, need_lse=True)
+    assert int(out._psa_status.item()) == 0
+    ref, ref_lse, _ = ops.legacy_forward(q, k, v, mask, causal, need_lse=True, impl=ops.IMPL_SCALAR)
+    _close(out, ref)
+    dead = torch.isinf(ref_lse)
+    assert bool(dead.any()) and torch.equal(dead, torch.isinf(lse)) and bool((lse[dead] < 0).all()) and bool((out[dead] == 0).all())
+    # fp32 sums of at most 768 terms in another order, and an exp2 that is right to 2^-22
+    assert float((lse[~dead] - ref_lse[~dead]).abs().max()) <= 1e-4
+    again, lse2, _ = ops.legacy_forward(q, k, v, mask, causal, need_lse=True)
+    assert torch.equal(out, again) and torch.equal(lse, lse2)
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("D,bn,owners", [(128, 64, 2), (64, 128, 3)])
+def test_rows_scattered_to_several_owners(D, bn, owners, dt):
+    """Output rows that go to the buffer of the rank that owns the token, all of them in this GPU's memory here: the bits of the plain
+    forward at the places of the address contract, nothing anywhere else."""
+    import ctypes
+    from psa_b200 import ops
+    from psa_b200._lib import check, lib
+    heads, head0, total, mq, nk = 6, 3, 11, 70, 1024 // bn + 9
+    S, Sq = nk * bn - 3, mq * 128 - 5
+    per = -(-Sq // owners)
+    k, v = (C.randn(960 + i, (1, heads, S, D), dt).to(DEV) for i in range(2))
+    q = C.randn(963, (1, heads, Sq, D), dt).to(DEV)
+    mask = _mask(nk, bn, mq, heads, 7 * bn)
+    images = ops.pyramid_kv_images(k, v, bn)
+    want = ops.psa_forward(q, k, v, mask, 128, bn, 32, pyramid=images)
+    bufs = [torch.full((per, total, D), 7.0, dtype=dt, device=DEV) for _ in range(owners)]
+    peers = (ctypes.c_void_p * owners)(*[b.data_ptr() for b in bufs])
+    status = ops.status_word(q.device)
+    check(lib.psa_fwd_images_scatter(q.data_ptr(), images.kimg.data_ptr(), images.vimg.data_ptr(), mask.data_ptr(), peers, owners, per, total,
+                                     head0, heads, Sq, S, D, 128, bn, 32, mask.shape[-1], D ** -0.5, 1, ops._dt(q), status.data_ptr(),
+                                     ops._stream(q)), "psa_fwd_images_scatter")
+    assert int(status.item()) == 0
+    got = torch.cat(bufs)
+    assert torch.equal(got[:Sq, head0:head0 + heads].transpose(0, 1).nan_to_num(), want[0].nan_to_num())
+    got[:Sq, head0:head0 + heads] = 7.0
+    assert bool((got == 7.0).all())
