@@ -75,8 +75,8 @@ class LaunchCounter:
 # shape with a reduced head count (profiles/); the figure is about the unique bytes of Q, O and the K/V images, so it
 # scales with heads x tokens.
 FWD_TRAFFIC_PER_HEAD_TOKEN = {
-    "wan2.1-1.3b-attn-layer": (1514.0, "profiles/psa_fwd_tc_kernel__wan2.1-1.3b-shape_6heads.md"),
-    "wan2.1-14b-attn-layer": (2837.0, "profiles/psa_fwd_tc_kernel__wan2.1-14b-shape_5heads_dram.md"),
+    "wan2.1-1.3b-attn-layer": (1502.0, "profiles/psa_fwd_tc_kernel__wan2.1-1.3b-shape_6heads.md"),
+    "wan2.1-14b-attn-layer": (2848.0, "profiles/psa_fwd_tc_kernel__wan2.1-14b-shape_5heads_dram.md"),
 }
 
 

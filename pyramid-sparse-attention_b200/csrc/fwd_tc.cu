@@ -28,7 +28,8 @@
 //               group works on the next row's first tile.
 // What bounds it: ~1750 cycles per tile = a chain of softmax (2000-2500), P V (~720), Q K^T (~720) and their hand-overs over
 // three score buffers, against 1024 cycles of the tensor pipe and as many of the ex2 unit; and the 1000 W power cap (at 75600
-// tokens the SM clock falls from 1965 to ~1500 MHz).
+// tokens the SM clock falls from 1965 to 1500-1700 MHz).  A copy takes its warp ~90 cycles: a tile of 32 blocks of 4 columns (row-major,
+// head_dim 128: 64 boxes per operand) takes 5600.
 // CODE SIZE counts: an SM holds about 32 KB of instructions, and the twelve warps are in five different places of the code.
 // What does not fit is fetched through a cache that up to six SMs share (with 143 KB of unrolled code the softmax of a tile took
 // 2120 cycles on an SM with that cache for two, 2990 on one with six).  Hence loops that are not unrolled, waits that are not,
@@ -117,7 +118,7 @@ template <int D, bool FIXED = false, bool CAUSAL = false> struct Cfg {
   // fill the instruction cache already they cost more than that (causal 14x32768x128 1779 -> 1930 us), and at head_dim 64 the softmax is the bound
   // (48x17776x64 694 -> 701 us).
   static constexpr bool UNROLL_MMA = D == 128 && !CAUSAL;
-  // The second pass of a full tile, two chunks at a time in a loop or all four in the code.  The loop, half the code, is the better one
+  // The second pass of a full tile, two chunks at a time in a loop or all four in the code.  The loop is the better one
   // (exact kernel, 16 x 9973 x 128 168 against 205 us, 6 x 32760 x 128 387 / 438, causal 8 x 16384 x 64 318 / 344) except in the exact kernel at
   // head_dim 64 without the causal rule, where three score buffers keep both groups in this pass (6 x 32760 365 / 311, 8 x 20011 704 / 610).
   static constexpr bool UNROLL_EXP = D == 64 && !FIXED && !CAUSAL;

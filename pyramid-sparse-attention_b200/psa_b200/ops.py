@@ -334,7 +334,9 @@ def psa_forward_tm(q_heads, images: KVImages, mask, out_tm, block_m: int, block_
 
 def draw_sample_indices(B: int, H: int, block: int, keep: int, device) -> torch.Tensor:
     """topk(rand(B,H,1,block), keep).indices, as _random_sample_tokens draws them (src/psa_triton/attention.py:132-133): the
-    numbers come from the same torch call on the same generator, their selection on a GPU is one kernel of the library."""
+    numbers come from the same torch call on the same generator, their selection on a GPU is one kernel of the library.  Equal
+    numbers (a pair in one row of 2000 of 128) stand by ascending position; torch selects the same ones and leaves their order
+    open.  A block's score is a maximum over its samples, so the order does not enter it."""
     rand_vals = torch.rand(B, H, 1, block, device=device)
     if rand_vals.device.type != "cuda" or rand_vals.dtype != torch.float32 or not 0 < keep <= block <= 128 or B * H == 0:
         _, idx = torch.topk(rand_vals, keep, dim=3)
