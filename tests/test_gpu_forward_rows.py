@@ -42,7 +42,7 @@ def _close(a, b):
 
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
 @pytest.mark.parametrize("D,bn", [(128, 64), (64, 64), (128, 128), (64, 128), (128, 32), (64, 32)])
-def test_short_rows_in_many_orders(D, bn, dt):
+def test_short_rows_in_every_order(D, bn, dt):
     from psa_b200 import ops
     heads, mq, nk = 48, 70, 1024 // bn + 9
     S = nk * bn - 3
